@@ -2,14 +2,18 @@
 //
 // This is the product of the true 32-bit engine (float inputs, float FMA, no
 // reduced-precision matrix mode) and the fallback of the bfloat16 engine for
-// shapes the tensor-core kernel refuses.  Every output element is accumulated
-// by one thread, in one fixed order: the products of each run of 16 values of k
-// are summed from zero and the runs' sums are added up in order (two short
-// chains of roundings instead of one of length K), so a row's result does not
+// shapes the tensor-core kernel refuses.  The order of additions is that of
+// rows_product.cuh: one order for every shape, so a row's result does not
 // depend on how many other rows are in the call.
-#include "common.cuh"
+#include "rows_product.cuh"
 
 namespace mdma {
+
+// The blocks that stream W are the faster ones as long as (rows of the matrices) x (passes of 8 rows of A) is small, since
+// every pass reads W again (from the second-level cache); both give the same bits.  Measured, few against tile, us (the
+// tile with one run on its way): 1,024 x 1,024 with 32 rows 10.5 / 14.9, 64 rows 20.2 / 21.1, 128 rows 35.8 / 25.1; 4,096 x
+// 1,024 with 16 rows 19.8 / 23.5, 24 rows 28.5 / 24.1; gated, 4,096 x 1,024, 8 rows 19.2 / 23.8, 12 rows 29.8 / 24.1.
+constexpr long kFewPasses = 8192;
 
 enum GemmMode : int {
     kStore = 0,        // out = acc
@@ -18,109 +22,62 @@ enum GemmMode : int {
     kStoreAct = 3,     // out = act(acc): a feed-forward without a gate
 };
 
-constexpr int TM = 64, TN = 64, TK = 16, PAD = 4;
-
-template <typename TA, typename TW, typename TO, int MODE>
-__global__ void __launch_bounds__(256)
+// FEW: blocks of up to 8 rows that stream W; else tiles of 32 rows.
+template <typename TA, typename TW, typename TO, int MODE, bool FEW>
+__global__ void __launch_bounds__(kRowsThreads)
 gemm_nt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, const TW* __restrict__ W2,
                TO* __restrict__ out, int ldo, int M, int N, int K, const Ending e,
                long batch_a, long batch_w, long batch_o) {
+    constexpr bool kDual = MODE == kSwiGLU;
+    extern __shared__ __align__(16) float smem[];
+    chain_release();
     // blockIdx.z: one of several products of the same sizes (a head each), operands `batch_*` elements apart
     A += (size_t)blockIdx.z * batch_a;
     W += (size_t)blockIdx.z * batch_w;
-    if (MODE == kSwiGLU) W2 += (size_t)blockIdx.z * batch_w;
+    if (kDual) W2 += (size_t)blockIdx.z * batch_w;
     out += (size_t)blockIdx.z * batch_o;
-    __shared__ float As[TK][TM + PAD];
-    __shared__ float Ws[TK][TN + PAD];
-    __shared__ float Ws2[MODE == kSwiGLU ? TK : 1][TN + PAD];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int ty = tid / 16, tx = tid % 16;
-    const int lrow = tid / 4, lk = (tid % 4) * 4;
-
-    float acc[4][4] = {};
-    float acc2[MODE == kSwiGLU ? 4 : 1][4] = {};
-
-    for (int k0 = 0; k0 < K; k0 += TK) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int k = k0 + lk + i;
-            const int m = m0 + lrow, n = n0 + lrow;
-            As[lk + i][lrow] = (m < M && k < K) ? to_float(A[(size_t)m * lda + k]) : 0.f;
-            Ws[lk + i][lrow] = (n < N && k < K) ? to_float(W[(size_t)n * K + k]) : 0.f;
-            if (MODE == kSwiGLU)
-                Ws2[lk + i][lrow] = (n < N && k < K) ? to_float(W2[(size_t)n * K + k]) : 0.f;
-        }
-        __syncthreads();
-        float part[4][4] = {};
-        float part2[MODE == kSwiGLU ? 4 : 1][4] = {};
-#pragma unroll
-        for (int k = 0; k < TK; ++k) {
-            float a[4], w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = fmaf(a[i], w[j], part[i][j]);
-            if (MODE == kSwiGLU) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) w[j] = Ws2[k][tx * 4 + j];
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) part2[i][j] = fmaf(a[i], w[j], part2[i][j]);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[i][j] += part[i][j];
-                if (MODE == kSwiGLU) acc2[i][j] += part2[i][j];
-            }
+    constexpr int kRows = FEW ? kFewRows : kTileRows;
+    const bool vec_a = rows_of_four(A, lda, K), vec_w = rows_of_four(W, K, K) && (!kDual || rows_of_four(W2, K, K));
+    if (!FEW) chain_wait();
+    for (int m0 = blockIdx.y * kRows; m0 < M; m0 += gridDim.y * kRows) {
+        const int rows = min(kRows, M - m0);
+        auto row_of = [&](int m) { return A + (size_t)(m0 + m) * lda; };
+        auto store = [&](int m, int n, float acc, float acc2) {
+            TO* o = out + (size_t)(m0 + m) * ldo + n;
+            const float r = acc + ending_bias(e.bias, e.bias_dtype, n);
+            if (MODE == kStore) *o = from_float<TO>(r);
+            else if (MODE == kAccumulate) *o = from_float<TO>(to_float(*o) + r);
+            else if (MODE == kStoreAct) *o = from_float<TO>(gate_activation(r, e.act));
+            else *o = from_float<TO>(gated_pair(r, acc2 + ending_bias(e.bias2, e.bias_dtype, n), e.act, e.act_limit, e.act_alpha));
+        };
+        if (FEW) few_rows_product<TA, TW, kDual>(rows, row_of, W, W2, blockIdx.x * few_rows_features(K, kDual), N, K, vec_a, vec_w,
+                                                 smem, [] { chain_wait(); }, store);
+        else tile_product<TA, TW, kDual>(rows, row_of, W, W2, blockIdx.x * (kDual ? kTileFeats / 2 : kTileFeats), N, K, vec_a, vec_w, smem, store);
         __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            TO* o = out + (size_t)m * ldo + n;
-            const float r = acc[i][j] + ending_bias(e.bias, e.bias_dtype, n);
-            if (MODE == kStore) {
-                *o = from_float<TO>(r);
-            } else if (MODE == kAccumulate) {
-                *o = from_float<TO>(to_float(*o) + r);
-            } else if (MODE == kStoreAct) {
-                *o = from_float<TO>(gate_activation(r, e.act));
-            } else {
-                *o = from_float<TO>(gated_pair(r, acc2[i][j] + ending_bias(e.bias2, e.bias_dtype, n), e.act, e.act_limit, e.act_alpha));
-            }
-        }
-    }
+}
+
+template <typename TA, typename TW, typename TO, int MODE>
+static void launch_mode(const void* A, int lda, const void* W, const void* W2, void* out, int ldo, int M, int N, int K,
+                        const Ending& e, cudaStream_t stream, int batch, long batch_a, long batch_w, long batch_o) {
+    constexpr bool kDual = MODE == kSwiGLU;
+    const bool few = (long)N * (kDual ? 2 : 1) * ((M + kFewRows - 1) / kFewRows) <= kFewPasses;
+    const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats, rows = few ? kFewRows : kTileRows;
+    const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, true> : gemm_nt_kernel<TA, TW, TO, MODE, false>;
+    launch_chained(kernel, dim3((N + feats - 1) / feats, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads),
+                   rows_product_smem(kernel, few), stream, (const TA*)A, lda,
+                   (const TW*)W, (const TW*)W2, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o);
 }
 
 template <typename TA, typename TW, typename TO>
 static int launch_gemm(int mode, const void* A, int lda, const void* W, const void* W2, void* out, int ldo,
                        int M, int N, int K, const Ending& e, cudaStream_t stream,
                        int batch = 1, long batch_a = 0, long batch_w = 0, long batch_o = 0) {
-    dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, batch);
-    if (mode == kStore)
-        gemm_nt_kernel<TA, TW, TO, kStore><<<grid, 256, 0, stream>>>((const TA*)A, lda, (const TW*)W, nullptr, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o);
-    else if (mode == kAccumulate)
-        gemm_nt_kernel<TA, TW, TO, kAccumulate><<<grid, 256, 0, stream>>>((const TA*)A, lda, (const TW*)W, nullptr, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o);
-    else if (mode == kSwiGLU)
-        gemm_nt_kernel<TA, TW, TO, kSwiGLU><<<grid, 256, 0, stream>>>((const TA*)A, lda, (const TW*)W, (const TW*)W2, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o);
-    else if (mode == kStoreAct)
-        gemm_nt_kernel<TA, TW, TO, kStoreAct><<<grid, 256, 0, stream>>>((const TA*)A, lda, (const TW*)W, nullptr, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o);
-    else
-        return fail("gemm_simt: unknown mode %d", mode);
+    if (mode == kStore) launch_mode<TA, TW, TO, kStore>(A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+    else if (mode == kAccumulate) launch_mode<TA, TW, TO, kAccumulate>(A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+    else if (mode == kSwiGLU) launch_mode<TA, TW, TO, kSwiGLU>(A, lda, W, W2, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+    else if (mode == kStoreAct) launch_mode<TA, TW, TO, kStoreAct>(A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+    else return fail("gemm_simt: unknown mode %d", mode);
     MDMA_LAUNCH_OK("gemm_simt");
     return 0;
 }
@@ -128,7 +85,6 @@ static int launch_gemm(int mode, const void* A, int lda, const void* W, const vo
 }  // namespace mdma
 
 using namespace mdma;
-
 extern "C" int mdma_gemm_simt(int mode, const void* A, int a_dtype, int lda, const void* W, const void* W2,
                               int w_dtype, void* out, int out_dtype, int ldo, int M, int N, int K,
                               const void* bias, const void* bias2, int bias_dtype, int act, float act_limit, float act_alpha,
@@ -136,7 +92,7 @@ extern "C" int mdma_gemm_simt(int mode, const void* A, int a_dtype, int lda, con
     MDMA_REQUIRE(M >= 0 && N > 0 && K > 0 && lda >= K && ldo >= N, "gemm_simt: bad sizes M=%d N=%d K=%d lda=%d ldo=%d", M, N, K, lda, ldo);
     MDMA_REQUIRE(mode != kSwiGLU || W2 != nullptr, "gemm_simt: SwiGLU needs two weights");
     MDMA_REQUIRE(mode != kAccumulate || out_dtype == kF32, "gemm_simt: the residual stream is float");
-    MDMA_REQUIRE((size_t)((M + TM - 1) / TM) <= 65535, "gemm_simt: too many rows (%d)", M);
+    MDMA_REQUIRE((M + 63) / 64 <= 65535, "gemm_simt: too many rows (%d)", M);
     MDMA_REQUIRE(act >= kActSilu && act <= kActReluSquared, "gemm_simt: unknown activation %d", act);
     MDMA_REQUIRE(act != kActSwishLimit || mode == kSwiGLU, "gemm_simt: the limited activation belongs to a gated product");
     MDMA_REQUIRE(bias_dtype == kF32 || bias_dtype == kBF16, "gemm_simt: unknown bias dtype %d", bias_dtype);
@@ -158,7 +114,7 @@ extern "C" int mdma_gemm_simt_batched(const void* A, int a_dtype, int lda, long 
                                       long batch_w, void* out, int out_dtype, int ldo, long batch_o, int batch,
                                       int M, int N, int K, cudaStream_t stream) {
     MDMA_REQUIRE(M >= 0 && N > 0 && K > 0 && batch > 0 && batch <= 65535, "gemm_simt_batched: bad sizes M=%d N=%d K=%d batch=%d", M, N, K, batch);
-    MDMA_REQUIRE((size_t)((M + TM - 1) / TM) <= 65535, "gemm_simt_batched: too many rows (%d)", M);
+    MDMA_REQUIRE((M + 63) / 64 <= 65535, "gemm_simt_batched: too many rows (%d)", M);
     if (M == 0) return 0;
     const Ending e{nullptr, nullptr, kF32, kActSilu};
     if (a_dtype == kF32 && w_dtype == kF32 && out_dtype == kF32)

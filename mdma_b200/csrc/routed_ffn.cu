@@ -21,9 +21,15 @@
 // by expert (steps of many tokens): the (token, choice) pairs are counted and sorted by expert on the
 // device, and a block computes a tile of pairs x features of ONE expert with the expert's matrix tile
 // staged in shared memory once for all its pairs.  No step of either way reads anything on the host.
-#include "common.cuh"
+#include "rows_product.cuh"
 
 namespace mdma {
+
+// Pairs per expert up to which the blocks that stream an expert's matrices are the faster ones.  Measured, 14 experts of 512
+// on rows of 1,024 floats, four a token, the whole feed-forward: 16 tokens (4.6 pairs an expert) 45 us against 75 with
+// tiles, 32 tokens (9.1) 70 against 76, 64 tokens (18) 117 against 78; 4 tokens 29 (385 with tiles that had nothing on
+// their way and four launches to sort the pairs).
+constexpr int kFewPairsPerExpert = 10;
 
 constexpr int kMaxRouted = 1024, kMaxTop = 32, kMaxGroupTop = 8;
 
@@ -61,6 +67,21 @@ __device__ __forceinline__ float warp_dot(const TA* __restrict__ a, const TW* __
     return warp_sum(acc);
 }
 
+// The place of the largest of n values above minus infinity (ties: the lower place), -1 without one; a whole warp calls it.
+__device__ __forceinline__ int warp_largest(const float* v, int n, int lane) {
+    int at = -1;
+    float best = -INFINITY;
+    for (int i = lane; i < n; i += 32)
+        if (v[i] > best) { best = v[i]; at = i; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, best, o);
+        const int place = __shfl_xor_sync(0xffffffffu, at, o);
+        if (place >= 0 && (at < 0 || other > best || (other == best && place < at))) { best = other; at = place; }
+    }
+    return at;
+}
+
 // ---------------------------------------------------------------- router
 template <typename TA, typename TW, typename TC>
 __global__ void __launch_bounds__(256)
@@ -72,77 +93,95 @@ route_kernel(const TA* __restrict__ h, int h_stride, const TW* __restrict__ rout
     chain_wait();
     __shared__ float z[kMaxRouted];
     __shared__ float c[kMaxRouted];
+    __shared__ float group_score[kMaxRouted];
+    __shared__ unsigned kept[kMaxRouted / 32];
     const int t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
     const TA* row = h + (size_t)t * h_stride;
+    const bool vec_row = width % 8 == 0 && ((uintptr_t)row & 15) == 0;
+    const bool vec = vec_row && ((uintptr_t)router & 15) == 0, vec_gate = vec_row && ((uintptr_t)shared_gate & 15) == 0;
     for (int e = warp; e < n_routed; e += n_warps) {
-        const float v = warp_dot(row, router + (size_t)e * width, width, lane);
+        const float v = warp_dot(row, router + (size_t)e * width, width, lane, vec);
         if (lane == 0) z[e] = v + (logit_bias ? to_float(correction[e]) : 0.f);
     }
     if (shared_gate != nullptr && warp == n_warps - 1) {
-        const float v = warp_dot(row, shared_gate, width, lane);
+        const float v = warp_dot(row, shared_gate, width, lane, vec_gate);
         if (lane == 0) shared_scale[t] = 1.0f / (1.0f + expf(-v));
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    // the rest is a few hundred operations: one thread, one order
+    // the rest is a few hundred operations of one warp: exponentials, group scores and the search for a largest score side
+    // by side, every sum by one lane in one order
+    if (warp != 0) return;
     if (scoring == 1) {
-        for (int e = 0; e < n_routed; ++e) z[e] = 1.0f / (1.0f + expf(-z[e]));
+        for (int e = lane; e < n_routed; e += 32) z[e] = 1.0f / (1.0f + expf(-z[e]));
     } else {
         float m = -INFINITY;
-        for (int e = 0; e < n_routed; ++e) m = fmaxf(m, z[e]);
+        for (int e = lane; e < n_routed; e += 32) m = fmaxf(m, z[e]);
+        m = warp_max(m);
+        for (int e = lane; e < n_routed; e += 32) z[e] = expf(z[e] - m);
+        __syncwarp();
         float sum = 0.f;
-        for (int e = 0; e < n_routed; ++e) { z[e] = expf(z[e] - m); sum += z[e]; }
-        for (int e = 0; e < n_routed; ++e) z[e] = z[e] / sum;
+        for (int e = 0; e < n_routed; ++e) sum += z[e];
+        __syncwarp();
+        for (int e = lane; e < n_routed; e += 32) z[e] = z[e] / sum;
     }
-    for (int e = 0; e < n_routed; ++e) c[e] = z[e] + (correction && !logit_bias ? to_float(correction[e]) : 0.f);   // z: s; c: choice score
+    for (int e = lane; e < n_routed; e += 32) c[e] = z[e] + (correction && !logit_bias ? to_float(correction[e]) : 0.f);   // z: s; c: choice score
+    __syncwarp();
     if (n_groups > 1 && keep_groups < n_groups) {
         const int per = n_routed / n_groups;
+        for (int g = lane; g < n_groups; g += 32) {
+            float gs = -INFINITY;
+            if (group_top <= 1) {
+                for (int e = g * per; e < (g + 1) * per; ++e) gs = fmaxf(gs, c[e]);
+            } else {
+                // the group's largest scores, largest first, are added up (a group of fewer members: all of them)
+                float best_of[kMaxGroupTop];
+#pragma unroll
+                for (int i = 0; i < kMaxGroupTop; ++i) best_of[i] = -INFINITY;
+                for (int e = g * per; e < (g + 1) * per; ++e) {
+                    float v = c[e];
+#pragma unroll
+                    for (int i = 0; i < kMaxGroupTop; ++i)
+                        if (v > best_of[i]) { const float tmp = best_of[i]; best_of[i] = v; v = tmp; }
+                }
+                gs = 0.f;
+#pragma unroll
+                for (int i = 0; i < kMaxGroupTop; ++i) if (i < group_top && i < per) gs += best_of[i];
+            }
+            group_score[g] = gs;
+        }
+        __syncwarp();
+        for (int w = lane; w < (n_groups + 31) / 32; w += 32) kept[w] = 0u;
+        __syncwarp();
         // the best group not yet kept is looked for keep_groups times (ties: the lower number); a bit per group
-        unsigned kept[kMaxRouted / 32];
-        for (int g = 0; g < (n_groups + 31) / 32; ++g) kept[g] = 0u;
-        for (int k = 0; k < keep_groups; ++k) {
+        for (int k = 0; lane == 0 && k < keep_groups; ++k) {
             int best = -1;
             float best_score = -INFINITY;
             for (int g = 0; g < n_groups; ++g) {
                 if (kept[g >> 5] >> (g & 31) & 1u) continue;
-                float gs = -INFINITY;
-                if (group_top <= 1) {
-                    for (int e = g * per; e < (g + 1) * per; ++e) gs = fmaxf(gs, c[e]);
-                } else {
-                    // the group's largest scores, largest first, are added up (a group of fewer members: all of them)
-                    float best_of[kMaxGroupTop];
-                    const int n_best = min(group_top, per);
-                    for (int i = 0; i < n_best; ++i) best_of[i] = -INFINITY;
-                    for (int e = g * per; e < (g + 1) * per; ++e) {
-                        float v = c[e];
-                        for (int i = 0; i < n_best; ++i)
-                            if (v > best_of[i]) { const float tmp = best_of[i]; best_of[i] = v; v = tmp; }
-                    }
-                    gs = 0.f;
-                    for (int i = 0; i < n_best; ++i) gs += best_of[i];
-                }
+                const float gs = group_score[g];
                 if (best < 0 || gs > best_score) { best = g; best_score = gs; }
             }
             if (best >= 0) kept[best >> 5] |= 1u << (best & 31);
         }
-        for (int g = 0; g < n_groups; ++g)
-            if (!(kept[g >> 5] >> (g & 31) & 1u))
-                for (int e = g * per; e < (g + 1) * per; ++e) c[e] = -INFINITY;
+        __syncwarp();
+        for (int e = lane; e < n_routed; e += 32) {
+            const int g = e / per;
+            if (!(kept[g >> 5] >> (g & 31) & 1u)) c[e] = -INFINITY;
+        }
+        __syncwarp();
     }
-    int pick[kMaxTop];
+    int mine = -1;                                        // lane k keeps the k-th choice
     float total = 0.f;
     for (int k = 0; k < top; ++k) {
-        int best = -1;
-        float best_score = -INFINITY;
-        for (int e = 0; e < n_routed; ++e)
-            if (c[e] > best_score) { best = e; best_score = c[e]; }
-        pick[k] = best;
-        if (best >= 0) { c[best] = -INFINITY; total += z[best]; }
+        const int best = warp_largest(c, n_routed, lane);
+        if (lane == k) mine = best;
+        if (best >= 0) { total += z[best]; if (lane == 0) c[best] = -INFINITY; }
+        __syncwarp();
     }
-    for (int k = 0; k < top; ++k) {
-        chosen[(size_t)t * top + k] = pick[k];
-        weights[(size_t)t * top + k] = pick[k] < 0 ? 0.f : weight_scale * (renormalize ? z[pick[k]] / (total + 1e-20f) : z[pick[k]]);
+    if (lane < top) {
+        chosen[(size_t)t * top + lane] = mine;
+        weights[(size_t)t * top + lane] = mine < 0 ? 0.f : weight_scale * (renormalize ? z[mine] / (total + 1e-20f) : z[mine]);
     }
 }
 
@@ -261,8 +300,51 @@ expert_place_kernel(const int* __restrict__ chosen, int n_pairs, int n_experts, 
     if (where) where[p] = at;
 }
 
+// The same three in one block, for steps of up to kSortPairs pairs: one launch instead of a memset and three.
+constexpr int kSortPairs = 8192, kSortThreads = 512;
+__global__ void __launch_bounds__(kSortThreads)
+expert_sort_kernel(const int* __restrict__ chosen, int n_pairs, int n_experts, int* __restrict__ first,
+                   int* __restrict__ order, int* __restrict__ where) {
+    chain_release();
+    chain_wait();
+    __shared__ int place[kMaxRouted];
+    for (int e = threadIdx.x; e < n_experts; e += kSortThreads) place[e] = 0;
+    __syncthreads();
+    for (int p = threadIdx.x; p < n_pairs; p += kSortThreads) {
+        const int e = chosen[p];
+        if (e >= 0 && e < n_experts) atomicAdd(&place[e], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int run = 0;
+        for (int e0 = 0; e0 < n_experts; e0 += 32) {
+            const int n = e0 + lane < n_experts ? place[e0 + lane] : 0;
+            int upto = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += v; }
+            if (e0 + lane < n_experts) { place[e0 + lane] = run + upto - n; first[e0 + lane] = run + upto - n; }
+            run += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (lane == 0) first[n_experts] = run;
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < n_pairs; p += kSortThreads) {
+        const int e = chosen[p];
+        if (e < 0 || e >= n_experts) continue;
+        const int at = atomicAdd(&place[e], 1);
+        order[at] = p;
+        if (where) where[p] = at;
+    }
+}
+
 // `first` holds 2 * (n_experts + 1) ints: the starts, then the counters
 static int sort_pairs(const int* chosen, int n_pairs, int n_experts, int* first, int* order, int* where, cudaStream_t stream) {
+    if (n_pairs <= kSortPairs && n_experts <= kMaxRouted) {
+        launch_chained(expert_sort_kernel, dim3(1), dim3(kSortThreads), 0, stream, chosen, n_pairs, n_experts, first, order, where);
+        MDMA_LAUNCH_OK("expert sort");
+        return 0;
+    }
     int* counters = first + n_experts + 1;
     if (cudaMemsetAsync(counters, 0, sizeof(int) * (size_t)(n_experts + 1), stream) != cudaSuccess) return fail("experts: memset failed");
     const int blocks = (n_pairs + 255) / 256;
@@ -288,134 +370,59 @@ expert_gather_kernel(const TA* __restrict__ h, int h_stride, const int* __restri
     for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < width; e += gridDim.y * blockDim.x) dst[e] = src[e];
 }
 
-// Tile sizes of the expert-by-expert products: kPairTile pairs x kFeatTile features per block, K walked kKTile at a time.
-constexpr int kPairTile = 32, kFeatTile = 64, kKTile = 16;
-
-// act[pair, f] = silu(G_e h) * (U_e h) for the pairs of expert blockIdx.z, tile blockIdx.y of its pairs
-template <typename TA, typename TW>
-__global__ void __launch_bounds__(256)
+// The products of expert blockIdx.z with its run of pairs, in the shapes and with the order of additions of
+// rows_product.cuh: FEW blocks stream the expert's matrices over up to 8 pairs, else tiles of 32 pairs.
+// act[pair, f] = pair_act(G_e h, U_e h), or act(G_e h) without U
+template <typename TA, typename TW, bool DUAL, bool FEW>
+__global__ void __launch_bounds__(kRowsThreads)
 expert_gate_up_sorted_kernel(const TA* __restrict__ h, int h_stride, const TW* __restrict__ G, const TW* __restrict__ U,
                              const int* __restrict__ first, const int* __restrict__ order, int top, int width, int ff,
                              TA* __restrict__ act, int pair_act, float act_limit, float act_alpha) {
     chain_release();
     chain_wait();
-    const int e = blockIdx.z;
-    const int begin = first[e] + blockIdx.y * kPairTile, end = first[e + 1];
-    if (begin >= end) return;
-    const int n = min(kPairTile, end - begin);
-    const int f0 = blockIdx.x * kFeatTile;
-    __shared__ float hs[kKTile][kPairTile + 1];
-    __shared__ float gs[kKTile][kFeatTile + 1];
-    __shared__ float us[kKTile][kFeatTile + 1];
-    __shared__ int pair_of[kPairTile];
-    if (threadIdx.x < kPairTile) pair_of[threadIdx.x] = threadIdx.x < n ? order[begin + threadIdx.x] : -1;
-    __syncthreads();
-    // thread (py, fx): pairs py*2 .. py*2+1, features fx*4 .. fx*4+3   (16 x 16 threads)
-    const int py = threadIdx.x / 16, fx = threadIdx.x % 16;
-    float ag[2][4] = {}, au[2][4] = {};
-    for (int k0 = 0; k0 < width; k0 += kKTile) {
-        for (int i = threadIdx.x; i < kKTile * kPairTile; i += 256) {
-            const int p = i / kKTile, k = i % kKTile;
-            const int pr = pair_of[p];
-            hs[k][p] = (pr >= 0 && k0 + k < width) ? to_float(h[(size_t)(pr / top) * h_stride + k0 + k]) : 0.f;
-        }
-        for (int i = threadIdx.x; i < kKTile * kFeatTile; i += 256) {
-            const int f = i / kKTile, k = i % kKTile;
-            const bool ok = f0 + f < ff && k0 + k < width;
-            const size_t at = ((size_t)e * ff + f0 + f) * width + k0 + k;
-            gs[k][f] = ok ? to_float(G[at]) : 0.f;
-            us[k][f] = ok && U != nullptr ? to_float(U[at]) : 0.f;
-        }
+    constexpr int kRows = FEW ? kFewRows : kTileRows;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int pair_of[kRows];
+    const int e = blockIdx.z, stop = first[e + 1];
+    G += (size_t)e * ff * width;
+    if (DUAL) U += (size_t)e * ff * width;
+    const bool vec_h = rows_of_four(h, h_stride, width), vec_w = rows_of_four(G, width, width) && (!DUAL || rows_of_four(U, width, width));
+    for (int begin = first[e] + blockIdx.y * kRows; begin < stop; begin += gridDim.y * kRows) {
+        const int n = min(kRows, stop - begin);
+        if (threadIdx.x < n) pair_of[threadIdx.x] = order[begin + threadIdx.x];
         __syncthreads();
-        float pg[2][4] = {}, pu[2][4] = {};
-#pragma unroll
-        for (int k = 0; k < kKTile; ++k) {
-            float a[2], g[4], u[4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) a[i] = hs[k][py * 2 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { g[j] = gs[k][fx * 4 + j]; u[j] = us[k][fx * 4 + j]; }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) { pg[i][j] = fmaf(a[i], g[j], pg[i][j]); pu[i][j] = fmaf(a[i], u[j], pu[i][j]); }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { ag[i][j] += pg[i][j]; au[i][j] += pu[i][j]; }
+        auto row_of = [&](int m) { return h + (size_t)(pair_of[m] / top) * h_stride; };
+        auto store = [&](int m, int f, float g, float u) {
+            act[(size_t)pair_of[m] * ff + f] = from_float<TA>(DUAL ? gated_pair(g, u, pair_act, act_limit, act_alpha) : gate_activation(g, pair_act));
+        };
+        if (FEW) few_rows_product<TA, TW, DUAL>(n, row_of, G, U, blockIdx.x * few_rows_features(width, DUAL), ff, width, vec_h, vec_w, smem, [] {}, store);
+        else tile_product<TA, TW, DUAL>(n, row_of, G, U, blockIdx.x * (DUAL ? kTileFeats / 2 : kTileFeats), ff, width, vec_h, vec_w, smem, store);
         __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int pr = pair_of[py * 2 + i];
-        if (pr < 0) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int f = f0 + fx * 4 + j;
-            if (f < ff) act[(size_t)pr * ff + f] = from_float<TA>(U == nullptr ? gate_activation(ag[i][j], pair_act) : gated_pair(ag[i][j], au[i][j], pair_act, act_limit, act_alpha));
-        }
     }
 }
 
 // y[pair, f] = D_e[f] . act[pair] for the pairs of expert blockIdx.z (float rows, one per pair)
-template <typename TA, typename TW>
-__global__ void __launch_bounds__(256)
+template <typename TA, typename TW, bool FEW>
+__global__ void __launch_bounds__(kRowsThreads)
 expert_down_sorted_kernel(const TA* __restrict__ act, const TW* __restrict__ D, const int* __restrict__ first,
                           const int* __restrict__ order, int width, int ff, float* __restrict__ y) {
     chain_release();
     chain_wait();
-    const int e = blockIdx.z;
-    const int begin = first[e] + blockIdx.y * kPairTile, end = first[e + 1];
-    if (begin >= end) return;
-    const int n = min(kPairTile, end - begin);
-    const int f0 = blockIdx.x * kFeatTile;
-    __shared__ float as[kKTile][kPairTile + 1];
-    __shared__ float ds[kKTile][kFeatTile + 1];
-    __shared__ int pair_of[kPairTile];
-    if (threadIdx.x < kPairTile) pair_of[threadIdx.x] = threadIdx.x < n ? order[begin + threadIdx.x] : -1;
-    __syncthreads();
-    const int py = threadIdx.x / 16, fx = threadIdx.x % 16;
-    float acc[2][4] = {};
-    for (int k0 = 0; k0 < ff; k0 += kKTile) {
-        for (int i = threadIdx.x; i < kKTile * kPairTile; i += 256) {
-            const int p = i / kKTile, k = i % kKTile;
-            const int pr = pair_of[p];
-            as[k][p] = (pr >= 0 && k0 + k < ff) ? to_float(act[(size_t)pr * ff + k0 + k]) : 0.f;
-        }
-        for (int i = threadIdx.x; i < kKTile * kFeatTile; i += 256) {
-            const int f = i / kKTile, k = i % kKTile;
-            ds[k][f] = (f0 + f < width && k0 + k < ff) ? to_float(D[((size_t)e * width + f0 + f) * ff + k0 + k]) : 0.f;
-        }
+    constexpr int kRows = FEW ? kFewRows : kTileRows;
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int pair_of[kRows];
+    const int e = blockIdx.z, stop = first[e + 1];
+    D += (size_t)e * width * ff;
+    const bool vec_a = rows_of_four(act, ff, ff), vec_w = rows_of_four(D, ff, ff);
+    for (int begin = first[e] + blockIdx.y * kRows; begin < stop; begin += gridDim.y * kRows) {
+        const int n = min(kRows, stop - begin);
+        if (threadIdx.x < n) pair_of[threadIdx.x] = order[begin + threadIdx.x];
         __syncthreads();
-        float part[2][4] = {};
-#pragma unroll
-        for (int k = 0; k < kKTile; ++k) {
-            float a[2], d[4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) a[i] = as[k][py * 2 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) d[j] = ds[k][fx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = fmaf(a[i], d[j], part[i][j]);
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+        auto row_of = [&](int m) { return act + (size_t)pair_of[m] * ff; };
+        auto store = [&](int m, int f, float v, float) { y[(size_t)pair_of[m] * width + f] = v; };
+        if (FEW) few_rows_product<TA, TW, false>(n, row_of, D, D, blockIdx.x * few_rows_features(ff, false), width, ff, vec_a, vec_w, smem, [] {}, store);
+        else tile_product<TA, TW, false>(n, row_of, D, D, blockIdx.x * kTileFeats, width, ff, vec_a, vec_w, smem, store);
         __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int pr = pair_of[py * 2 + i];
-        if (pr < 0) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int f = f0 + fx * 4 + j;
-            if (f < width) y[(size_t)pr * width + f] = acc[i][j];
-        }
     }
 }
 
@@ -511,17 +518,25 @@ int mdma_experts_sorted(const void* h, int h_dtype, int h_stride, const void* G,
     MDMA_REQUIRE(n_tokens >= 0 && width > 0 && ff > 0 && top > 0 && n_experts >= 0 && n_experts <= kMaxRouted, "experts: bad sizes");
     if (n_tokens == 0) return 0;
     const int n_pairs = n_tokens * top;
-    const int pair_tiles = (n_pairs + kPairTile - 1) / kPairTile;
-    MDMA_REQUIRE(pair_tiles <= 65535 && n_experts <= 65535, "experts: too many pairs (%d)", n_pairs);
+    MDMA_REQUIRE((n_pairs + 31) / 32 <= 65535, "experts: too many pairs (%d)", n_pairs);
+    // by the pairs an expert has on average: the blocks take more tiles each where one has more
+    const bool few = n_pairs <= kFewPairsPerExpert * n_experts;
+    const int rows = few ? kFewRows : kTileRows;
+    const int pair_tiles = n_experts > 0 ? (n_pairs / n_experts + rows) / rows + 1 : 1;
     const int wparts = (width + 255) / 256 > 64 ? 64 : (width + 255) / 256;
     MDMA_DISPATCH_2(h_dtype, TA, w_dtype, TW, {
         if (n_experts > 0) {
             if (int rc = sort_pairs(chosen, n_pairs, n_experts, first, order, nullptr, stream)) return rc;
-            launch_chained(expert_gate_up_sorted_kernel<TA, TW>, dim3((ff + kFeatTile - 1) / kFeatTile, pair_tiles, n_experts),
-                           dim3(256), 0, stream, (const TA*)h, h_stride, (const TW*)G, (const TW*)U, first, order, top, width,
-                           ff, (TA*)act, pair_act, act_limit, act_alpha);
-            launch_chained(expert_down_sorted_kernel<TA, TW>, dim3((width + kFeatTile - 1) / kFeatTile, pair_tiles, n_experts),
-                           dim3(256), 0, stream, (const TA*)act, (const TW*)D, first, order, width, ff, y);
+            const bool dual = U != nullptr;
+            const int gf = few ? few_rows_features(width, dual) : dual ? kTileFeats / 2 : kTileFeats;
+            const int df = few ? few_rows_features(ff, false) : kTileFeats;
+            auto up = dual ? (few ? expert_gate_up_sorted_kernel<TA, TW, true, true> : expert_gate_up_sorted_kernel<TA, TW, true, false>)
+                           : (few ? expert_gate_up_sorted_kernel<TA, TW, false, true> : expert_gate_up_sorted_kernel<TA, TW, false, false>);
+            launch_chained(up, dim3((ff + gf - 1) / gf, pair_tiles, n_experts), dim3(kRowsThreads), rows_product_smem(up, few), stream, (const TA*)h, h_stride,
+                           (const TW*)G, (const TW*)U, first, order, top, width, ff, (TA*)act, pair_act, act_limit, act_alpha);
+            auto down = few ? expert_down_sorted_kernel<TA, TW, true> : expert_down_sorted_kernel<TA, TW, false>;
+            launch_chained(down, dim3((width + df - 1) / df, pair_tiles, n_experts), dim3(kRowsThreads), rows_product_smem(down, few), stream, (const TA*)act,
+                           (const TW*)D, first, order, width, ff, y);
         }
         launch_chained(expert_combine_kernel<TA>, dim3(n_tokens, wparts), dim3(256), 0, stream, y, (const TA*)h, h_stride,
                        chosen, weights, (const int*)nullptr, n_experts, top, width, x);
