@@ -75,14 +75,15 @@ int mdma_attention_decode_rotary(const void* qkv, int q_stride, const float* pro
                                  void* k_cache, void* v_cache, int n_pages, const int* seq_start, const int* seq_pos0,
                                  const int* seq_slot, const int* page_table, int max_pages, int page_size, void* out,
                                  int n_seqs, int n_heads, int n_kv_heads, int head_dim, int window, float scale,
-                                 int splits, float* scratch, long scratch_floats, int* status, cudaStream_t stream) {
+                                 int splits, int chunk_keys, float* scratch, long scratch_floats, int* status,
+                                 cudaStream_t stream) {
     FusedRotary fz;
     fz.inv_freq = inv_freq; fz.rotary_dim = rotary_dim; fz.interleaved = interleaved;
     fz.partial = proj_splits > 0 ? proj_partial : nullptr; fz.splits = proj_splits; fz.split_stride = proj_split_stride;
     fz.width = (n_heads + 2 * n_kv_heads) * head_dim;
     return launch_attention_mma(qkv, q_stride, k_cache, v_cache, seq_start, seq_pos0, seq_slot, page_table, max_pages,
                                 page_size, out, n_seqs, n_seqs, 1, n_heads, n_kv_heads, head_dim, window, scale, splits,
-                                scratch, scratch_floats, stream, n_pages, status, &fz);
+                                scratch, scratch_floats, stream, n_pages, status, &fz, nullptr, nullptr, chunk_keys);
 }
 
 // Everything the EXT forms take; see launch_attention_mma_general.

@@ -64,6 +64,7 @@ struct AttnParams {
     __nv_bfloat16* out;                             // [tokens, heads * head_dim]
     float* part_o; float* part_ml;                  // split partials: [tokens, heads, splits, head_dim], [.., 2]
     int n_heads, n_kv_heads, head_dim, group, tile_tokens, window, splits;
+    int chunk_keys;                                 // > 0 (decode by tile loads): a split is that many keys, however many a sequence has
     float scale_log2;                               // scale * log2(e)
     int* status;                                    // optional device word, set non-zero if a wait ran out
     // A softmax with a sink: 2^(sink_log2[head] - m) is added to every row's denominator once (a term with
@@ -570,8 +571,16 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const int keep = EXT ? p.rule.keep_first : 0, kb = EXT ? min((keep + KB - 1) / KB, blk_lo) : 0;
     auto tile_of = [&](int i) { return EXT && i < blk_lo ? i - (blk_lo - kb) : i; };
     const int list_lo = blk_lo - kb;
-    const int per = (blk_hi - list_lo + p.splits - 1) / p.splits;
+    const int per = p.chunk_keys > 0 ? p.chunk_keys / KB : (blk_hi - list_lo + p.splits - 1) / p.splits;
     const int b0 = list_lo + split * per, b1 = min(blk_hi, b0 + per);
+    if (p.chunk_keys > 0 && b0 >= blk_hi) {              // the sequence is shorter: an empty part for the merge
+        chain_wait();
+        if ((int)threadIdx.x < G) {
+            const size_t slot = ((size_t)token * p.n_heads + kvh * G + threadIdx.x) * p.splits + split;
+            p.part_ml[slot * 2] = -INFINITY; p.part_ml[slot * 2 + 1] = 0.f;
+        }
+        return;
+    }
     const int k_halves = (D + 63) / 64, v_halves = (DV + 63) / 64;
 
     auto load_tile = [&](const CUtensorMap* tmap, bool is_v, uint32_t dst, uint32_t bar, int at) {      // one lane
@@ -911,7 +920,7 @@ static int launch_attention_mma(const void* q, int q_stride, const void* k_cache
                        int n_heads, int n_kv_heads, int head_dim, int window, float scale, int splits,
                        float* scratch, long scratch_floats, cudaStream_t stream, int n_pages = 0,
                        int* status = nullptr, const FusedRotary* fz = nullptr, const float* sink_log2 = nullptr,
-                       const float* slope_log2 = nullptr) {
+                       const float* slope_log2 = nullptr, int chunk_keys = 0) {
     // (launch_attention_mma_general below is the launcher of the EXT forms)
     MDMA_REQUIRE(attention_mma_supported(n_heads, n_kv_heads, head_dim),
                  "attention_mma: heads %d / kv heads %d / head_dim %d is outside its limits (head_dim a multiple of 16 up to 128, group up to 64)",
@@ -934,6 +943,8 @@ static int launch_attention_mma(const void* q, int q_stride, const void* k_cache
     p.rot_inv_freq = nullptr; p.rotary_dim = 0; p.rot_interleaved = 0;
     p.proj_partial = nullptr; p.proj_splits = 0; p.proj_split_stride = 0; p.proj_width = 0;
     p.k_cache_w = nullptr; p.v_cache_w = nullptr;
+    p.chunk_keys = splits > 1 ? chunk_keys : 0;
+    MDMA_REQUIRE(chunk_keys >= 0 && chunk_keys % 64 == 0 && (chunk_keys == 0 || fz != nullptr), "attention: keys in chunks of %d", chunk_keys);
     p.v_dim = head_dim; p.maps = 1; p.rule = {window, 0, 0}; p.cap_log2 = p.cap_rate = 0.f; p.out_f32 = nullptr;
     if (fz != nullptr) {
         MDMA_REQUIRE(max_new == 1 && n_pages > 0 && attention_fused_rotary_supported(n_heads, n_kv_heads, head_dim, page_size, fz->rotary_dim),
@@ -976,7 +987,7 @@ static int launch_attention_mma(const void* q, int q_stride, const void* k_cache
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         // the most warps per block with which every block of the grid is resident at once
-        const long blocks = (long)n_seqs * n_kv_heads * splits;
+        const long blocks = (long)n_seqs * n_kv_heads * (p.chunk_keys > 0 ? 1 : splits);
         // (up to ten blocks per SM: one warp each.  128 sequences x 8 kv heads at context 580, with the rotary kernel
         // before it: 64.0 us against 77.8 us in two and a bit rounds of four-warp blocks; 184 sequences 88.0 against
         // 98.8 us.  Beyond that, rounds of four-warp blocks: 192 sequences 99.0 us against 110.7 us with one warp)

@@ -284,6 +284,22 @@ def attention_splits(n_seqs: int, max_new: int, max_len: int, n_heads: int, n_kv
     return max(1, min(-(-2 * sms // blocks), key_blocks, 32))
 
 
+CHUNK_KEYS = 1024        # (512 measures the same)
+
+
+def decode_chunks(n_seqs: int, max_len: int, n_kv_heads: int, sms: int) -> tuple[int, int]:
+    """(splits, keys per split) of a single-token step whose blocks, one per (sequence, kv head), already cover the
+    device (`attention_splits` gives 1): contexts beyond 1,024 are cut into pieces of the same number of keys for
+    every sequence, so that the device does not wait for the longest one's blocks.  No more than 5 x SMs blocks (the
+    scratch that engines reserve); (1, 0): whole contexts.  Measured, 8 sequences of 255 to 2,040 tokens, 32 kv heads of 128:
+    a whole decode step of 32 layers 4.26 -> 3.77 ms with the merge that the pieces need."""
+    longest = -(-max_len // 1024) * 1024           # as the replayed decode graphs see it
+    splits = min(longest // CHUNK_KEYS, 5 * sms // (n_seqs * n_kv_heads))
+    if longest <= 1024 or n_seqs * n_kv_heads < sms or splits < 2:
+        return 1, 0
+    return splits, -(-longest // splits // 64) * 64
+
+
 def attention_tc_supported(n_heads: int, n_kv_heads: int, head_dim: int, page_size: int) -> bool:
     return (attention_supported(n_heads, n_kv_heads, head_dim) and n_heads // n_kv_heads <= 128
             and page_size % 64 == 0)
@@ -365,7 +381,8 @@ def fused_rotary_supported(n_heads: int, n_kv_heads: int, head_dim: int, page_si
 
 def attention_decode_rotary(ctx, qkv: torch.Tensor, view, out: torch.Tensor, n_heads: int, n_kv_heads: int,
                             head_dim: int, window: int, scale: float, inv_freq: torch.Tensor, rotary_dim: int,
-                            interleaved: bool, splits: Optional[int] = None, st: Optional[TensorState] = None) -> None:
+                            interleaved: bool, splits: Optional[int] = None, st: Optional[TensorState] = None,
+                            chunk_keys: int = 0) -> None:
     """A step of one token per sequence: the projection rows `qkv` (or the K-split partial sums a
     deferred product left for them) are rotated, the keys and values written to the cache and the
     attention computed by ONE kernel; it asks for all its key and value tiles before it waits for
@@ -385,6 +402,9 @@ def attention_decode_rotary(ctx, qkv: torch.Tensor, view, out: torch.Tensor, n_h
         flush_pending(qkv.device, st)
     if splits is None:
         splits = attention_splits(ctx.n_seqs, 1, ctx.max_len, n_heads, n_kv_heads, st.sms, getattr(ctx, "most_seqs", None))
+        if splits == 1 and not window:
+            splits, chunk_keys = decode_chunks(ctx.n_seqs, ctx.max_len, n_kv_heads, st.sms)
+    assert chunk_keys == 0 or chunk_keys * splits >= ctx.max_len
     # the attention's own partials (keys split over blocks) lie behind the projection's
     used = -(-proj_splits * stride // 64) * 64
     need = ctx.n_tokens * n_heads * splits * (head_dim + 2) if splits > 1 else 0
@@ -394,7 +414,7 @@ def attention_decode_rotary(ctx, qkv: torch.Tensor, view, out: torch.Tensor, n_h
           ctypes.c_long(stride), _ptr(inv_freq), _i(rotary_dim), _i(int(interleaved)), _ptr(view.k), _ptr(view.v),
           _i(view.k.shape[0]), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(ctx.seq_slot), _ptr(view.page_table),
           _i(view.max_pages), _i(view.page_size), _ptr(out), _i(ctx.n_seqs), _i(n_heads), _i(n_kv_heads), _i(head_dim),
-          _i(window), _f(scale), _i(splits), _ptr(own), ctypes.c_long(own.numel()), _ptr(st.status), _stream(),
+          _i(window), _f(scale), _i(splits), _i(chunk_keys), _ptr(own), ctypes.c_long(own.numel()), _ptr(st.status), _stream(),
           launches=2 if splits > 1 else 1)
 
 

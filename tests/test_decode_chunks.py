@@ -1,0 +1,65 @@
+"""Single-token steps whose sequences' keys are cut into pieces of one size (`decode_chunks`)."""
+import math
+
+import pytest
+import torch
+
+
+@pytest.mark.parametrize("sms", [148, 78])
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(32, 8, 128), (32, 32, 128), (16, 8, 16), (64, 64, 64), (40, 2, 64)])
+def test_pieces_cover_the_context_and_fit_the_scratch(heads, kv_heads, head_dim, sms):
+    from mdma_b200 import ops_tensor
+    reserved = (ops_tensor.scratch_floats_bound(sms, 8192, 1, [(heads, kv_heads, head_dim)])
+                - ops_tensor.scratch_floats_bound(sms, 8192, 1, ()))
+    seen = 0
+    for n_seqs in range(1, 200):
+        for max_len in (1, 1024, 1025, 2048, 3000, 9000, 40000):
+            splits, keys = ops_tensor.decode_chunks(n_seqs, max_len, kv_heads, sms)
+            if splits == 1:
+                assert keys == 0
+                continue
+            seen += 1
+            assert keys % 64 == 0 and splits * keys >= max_len and n_seqs * kv_heads >= sms
+            assert n_seqs * heads * splits * (head_dim + 2) <= reserved
+    assert seen
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,K,hd", [(4, 4, 128), (8, 2, 64), (6, 6, 48)])
+@pytest.mark.parametrize("splits,keys", [(2, 64), (5, 128), (16, 64), (2, 1024)])
+def test_decode_in_pieces(H, K, hd, splits, keys):
+    """Against float64 at lengths around the pieces' edges; a piece that a sequence does not reach leaves nothing behind."""
+    from mdma_b200 import ops_tensor
+    from mdma_b200.parts.rotary import inverse_frequencies
+    from test_kernels import DEV, StepMeta, close, fill_cache, ops_mod, reference_attention
+    ops = ops_mod()
+    torch.manual_seed(H + hd + keys)
+    page, most = 64, splits * keys
+    cached = [min(c, most - 1) for c in (0, keys - 2, keys - 1, keys, 2 * keys - 1, most - 1, 31)]
+    B = len(cached)
+    lens = [c + 1 for c in cached]
+    kc, vc, table, max_pages, dense = fill_cache(lens, K, hd, page, torch.bfloat16, seed=hd, poison=True)
+    inv_freq = inverse_frequencies(hd, 10000.0).to(DEV)
+    qkv = torch.randn(B, (H + 2 * K) * hd).bfloat16().to(DEV)
+    meta = StepMeta(cached, [1] * B)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    kc2, vc2, qkv2 = kc.clone(), vc.clone(), qkv.clone()
+    ops.rope_cache_write(qkv2, B, i32(list(range(B))), i32(cached), meta.seq_slot, inv_freq, kc2, vc2, table, max_pages, page, H, K, hd,
+                         hd, False, True, None, 0, 0)
+
+    class View:
+        pass
+    view = View()
+    view.k, view.v, view.page_table, view.max_pages, view.page_size = kc, vc, table, max_pages, page
+    out = torch.full((B + 1, H * hd), 9.0, device=DEV, dtype=torch.bfloat16)
+    ops_tensor._device_state(torch.device(DEV)).scratch.fill_(float("nan"))
+    scale = 1.0 / math.sqrt(hd)
+    ops_tensor.attention_decode_rotary(meta, qkv, view, out, H, K, hd, 0, scale, inv_freq, hd, False, splits=splits, chunk_keys=keys)
+    ops_tensor.check_status(torch.device(DEV))
+    assert torch.equal(kc.view(torch.int16), kc2.view(torch.int16)) and torch.equal(vc.view(torch.int16), vc2.view(torch.int16))
+    for s, n in enumerate(lens):
+        pg = int(table[s, (n - 1) // page])
+        dense[s][0][n - 1], dense[s][1][n - 1] = kc2[pg, (n - 1) % page].cpu(), vc2[pg, (n - 1) % page].cpu()
+    want = reference_attention(qkv2[:, :H * hd].double().cpu().reshape(B, H, hd), dense, list(range(B)), cached, scale, 0)
+    close(out[:B], want, 2e-2, 2e-2)
+    assert bool((out[B:] == 9.0).all())
