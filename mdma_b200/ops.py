@@ -8,6 +8,7 @@ is no fallback: without the compiled library, or off the GPU, these raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -401,6 +402,12 @@ def mamba2_scan(conv, proj, dt_col: int, dt_bias, a_log, d, seq_start, seq_slot,
     assert conv.dtype == proj.dtype == y.dtype == torch.float32 and conv.stride(1) == 1 and proj.stride(1) == 1
     assert y.is_contiguous() and y.shape[1] == heads * vdim and conv.shape[1] == heads * vdim + 2 * groups * n_state
     sp, ss = _state(state)
+    if chunk_rows > 0 and chunk_rows == chunk_scan_rows(n_state, vdim) and not wide_state and scratch.data_ptr() % 16 == 0:
+        _call("core", "mdma_mamba2_chunks", _ptr(conv), _i(conv.stride(0)), _ptr(proj), _i(proj.stride(0)), _i(dt_col),
+              _ptr(dt_bias), _ptr(a_log), _ptr(d), _i(dtype_code(d.dtype)), _ptr(seq_start), _ptr(seq_slot), sp, ss, _ptr(y),
+              _i(n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(max_chunks), _ptr(scratch),
+              ctypes.c_long(scratch.numel()), _stream(), launches=3)
+        return
     _call("core", "mdma_mamba2_scan", _ptr(conv), _i(conv.stride(0)), _ptr(proj), _i(proj.stride(0)), _i(dt_col),
           _ptr(dt_bias), _ptr(a_log), _ptr(d), _i(_same_dtype(dt_bias, a_log, d)), _ptr(seq_start), _ptr(seq_slot),
           sp, ss, _ptr(y), _i(n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(chunk_rows), _i(max_chunks),
@@ -686,6 +693,14 @@ def add_scaled(y: torch.Tensor, z: torch.Tensor, a: float, n_rows: int) -> None:
     _call("core", "mdma_add_scaled", _ptr(y), _ptr(z), _f(a), ctypes.c_long(n_rows * y.shape[1]), _stream())
 
 
+# ---- prompts through recurrences linear in their state, chunks of rows side by side (csrc/chunk_scan.cu) ----------------
+@functools.lru_cache(maxsize=None)
+def chunk_scan_rows(n: int, vdim: int) -> int:
+    """Rows of a chunk: `linear_attention` and `mamba2_scan` asked for runs of that many rows take the kernels whose chunks
+    all start from a state that one launch in between has made; 0 where heads of n x vdim do not fit them."""
+    return int((_build._loaded.get("core") or _build.load("core")).mdma_chunk_scan_rows(_i(n), _i(vdim)))
+
+
 # ---- linear attention with a decay per head (csrc/linear_attention.cu) -----------------------------------------------------
 def linear_attention_fits(dim: int, vdim: int, chunked: bool = False) -> bool:
     """Whether heads of dim x vdim fit a block's shared memory in the walk row by row, or a chunk of rows at a time."""
@@ -714,6 +729,12 @@ def linear_attention(proj, q_col: int, k_col: int, v_col: int, decay, seq_start,
     assert rotary_dim == 0 or (inv_freq.dtype == torch.float32 and inv_freq.numel() >= rotary_dim // 2 and tok_pos is not None)
     sp, ss = _state(state)
     assert state.shape[1] >= heads * dim * vdim
+    if run_rows > 0 and run_rows == chunk_scan_rows(dim, vdim) and scratch.data_ptr() % 16 == 0:
+        _call("core", "mdma_linear_attention_chunks", _ptr(proj), _i(dtype_code(proj.dtype)), _i(proj.stride(0)), _i(q_col),
+              _i(k_col), _i(v_col), _ptr(decay), _ptr(seq_start), _ptr(seq_slot), sp, ss, _ptr(out), _i(n_seqs), _i(heads),
+              _i(dim), _i(vdim), _i(max_runs), _ptr(scratch), ctypes.c_long(scratch.numel()), _i(int(silu)), _i(rotary_dim),
+              _i(int(interleaved)), _ptr(inv_freq), _ptr(tok_pos), _f(k_scale), _stream(), launches=3)
+        return
     _call("core", "mdma_linear_attention", _ptr(proj), _i(dtype_code(proj.dtype)), _i(proj.stride(0)), _i(q_col), _i(k_col),
           _i(v_col), _ptr(decay), _ptr(seq_start), _ptr(seq_slot), sp, ss, _ptr(out), _i(n_seqs), _i(heads), _i(dim),
           _i(vdim), _i(2 if single else int(chunked)), _i(run_rows), _i(max_runs), _ptr(scratch),

@@ -41,7 +41,10 @@ class LinearAttention(Part):
     graph_safe = True
     takes_out_scale = True
     CHUNKS_FROM = 16          # rows of a sequence in a step from which the serving engine walks chunk by chunk
-    RUN_ROWS = 128            # rows of a run; sequences of two runs and more are walked as runs side by side
+    # rows of a sequence in a step from which its chunks are worked on side by side (16 heads of 128 x 128, the walk chunk by
+    # chunk against that: 64 rows 39 / 57 us, 100 rows 59 / 58, 200 rows 96 / 59)
+    SIDE_BY_SIDE_FROM = 100
+    RUN_ROWS = 128            # rows of a run, where heads or scratch do not suit the chunk kernels
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -132,11 +135,13 @@ class LinearAttention(Part):
         # the 32-bit engine, row by row
         chunked = self.chunks_fit and proj.dtype != torch.float32 and ctx.max_new >= self.CHUNKS_FROM
         run_rows, max_runs, scratch = 0, 1, None
-        if chunked and ctx.max_new >= 2 * self.RUN_ROWS:
+        if chunked and ctx.max_new >= min(self.SIDE_BY_SIDE_FROM, 2 * self.RUN_ROWS):
             runs = ctx.buf(f"lin_runs_{tag}_{self.dim}", self._run_columns(), torch.float32).view(-1)
-            most = -(-ctx.max_new // self.RUN_ROWS)
-            if ctx.n_seqs * most * self.heads * self.dim * self.v_dim <= runs.numel():
-                run_rows, max_runs, scratch = self.RUN_ROWS, most, runs
+            for rows, least in ((ops.chunk_scan_rows(self.dim, self.v_dim), self.SIDE_BY_SIDE_FROM), (self.RUN_ROWS, 2 * self.RUN_ROWS)):
+                most = -(-ctx.max_new // rows) if rows else 0
+                if rows and ctx.max_new >= least and ctx.n_seqs * most * self.heads * self.dim * self.v_dim <= runs.numel():
+                    run_rows, max_runs, scratch = rows, most, runs
+                    break
         inv_freq, rotary_dim, interleaved = self.position.rotary_table() if self.position is not None else (None, 0, False)
         ops.linear_attention(proj, 0, self.k_col, self.v_col, self.decay_dev, ctx.seq_start, ctx.seq_slot, view.state, sums,
                              ctx.n_seqs, self.heads, self.dim, self.v_dim, chunked, run_rows, max_runs, scratch,

@@ -105,7 +105,10 @@ class MinGRU(_StatefulMixer):
 @MIXERS.register("mamba2")
 class Mamba2(_StatefulMixer):
     MAX_STATE, MAX_TAPS = 256, 16          # the scan kernel's and the convolution kernel's limits
-    CHUNK_ROWS = 256                       # the serving engine walks prompts as runs of this many rows side by side
+    # rows of a sequence in a step from which its chunks are worked on side by side (64 heads, the walk row by row against
+    # that: 64 rows 46 / 35 us, 200 rows 132 / 47)
+    SIDE_BY_SIDE_FROM = 64
+    CHUNK_ROWS = 256                       # rows of a run, where the state or the scratch does not suit the chunk kernels
 
     def __init__(self, spec):
         super().__init__(spec)
@@ -156,8 +159,8 @@ class Mamba2(_StatefulMixer):
         return f"mamba_proj_{tag}", f"mamba_conv_{tag}", f"mamba_y_{tag}", f"mamba_g_{tag}", f"mamba_runs_{tag}"
 
     def _run_columns(self) -> int:
-        # scratch for the side-by-side runs: room for two runs' states (and decays) per CHUNK_ROWS rows of a step
-        return -(-2 * (self.state_elements + self.heads) // self.CHUNK_ROWS)
+        # scratch for what is worked on side by side: room for a state (and its decays) per 64 rows of a step
+        return -(-(self.state_elements + self.heads) // 64)
 
     def workspace(self):
         proj, conv, y, g, runs = self._names()
@@ -183,15 +186,17 @@ class Mamba2(_StatefulMixer):
         self.w_in.store(h, proj, n)
         ops.causal_conv_silu(proj, self.inner, self.conv_w, self.conv_b, self.taps, self.channels, ctx.tok_seq,
                              ctx.seq_start, ctx.seq_slot, conv_state, conv, n, ctx.n_seqs)
-        # steps of long prompts in the serving engine: runs of CHUNK_ROWS rows side by side, if the scratch holds
+        # steps of long prompts in the serving engine: chunks, or runs of CHUNK_ROWS rows, side by side, if the scratch holds
         # them (it does unless one long prompt comes with many short ones); else, and always in the 32-bit engine,
         # row by row
         chunk_rows, max_chunks, scratch = 0, 1, None
-        if g.dtype != torch.float32 and ctx.max_new >= 2 * self.CHUNK_ROWS:
+        if g.dtype != torch.float32 and ctx.max_new >= min(self.SIDE_BY_SIDE_FROM, 2 * self.CHUNK_ROWS):
             runs = ctx.buf(names[4], self._run_columns(), torch.float32).view(-1)
-            most = -(-ctx.max_new // self.CHUNK_ROWS)
-            if ctx.n_seqs * most * (self.state_elements + self.heads) <= runs.numel():
-                chunk_rows, max_chunks, scratch = self.CHUNK_ROWS, most, runs
+            for rows, least in ((ops.chunk_scan_rows(self.n_state, self.vdim), self.SIDE_BY_SIDE_FROM), (self.CHUNK_ROWS, 2 * self.CHUNK_ROWS)):
+                most = -(-ctx.max_new // rows) if rows else 0
+                if rows and ctx.max_new >= least and ctx.n_seqs * most * (self.state_elements + self.heads) <= runs.numel():
+                    chunk_rows, max_chunks, scratch = rows, most, runs
+                    break
         ops.mamba2_scan(conv, proj, self.proj_width - self.heads, self.dt_bias, self.a_log, self.d, ctx.seq_start,
                         ctx.seq_slot, ssm_state, y, ctx.n_seqs, self.heads, self.vdim, self.n_state, self.groups,
                         chunk_rows, max_chunks, scratch, self.wide_state)
