@@ -340,7 +340,7 @@ __device__ inline PairWork pair_work(int pair, int n_pairs, int n_tiles, int n_k
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(tc2_threads<MODE>())
+__global__ void __launch_bounds__(tc2_threads<MODE>(), 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                 const __grid_constant__ CUtensorMap map_x, const TcParams p) {
     // Persistent: the grid holds at most one pair per two SMs and every pair walks over its segments.
@@ -481,6 +481,41 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 if (!ok) { *abort_flag = 1; break; }
             }
             const uint32_t lane_addr = tmem_base + buf * kBufCols + ((uint32_t)(quad * 32) << 16);
+            // this warp has read its part of the buffer: tell the leading block's MMA thread
+            auto release = [&] {
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive_cluster(lead_empty[buf]);
+            };
+            if (kDual && sg.kind == kSegFull && p.ending.act == kActSilu && !p.out_f32) {
+                // The gated product's only buffer keeps the tensor cores waiting until it has been read out: once a
+                // warp has its last 16 columns in registers it gives the buffer back, and their activation and stores run under
+                // the next tile's MMAs.
+                auto finish = [&](int c, const float* v, const float* u) {
+                    if (f >= p.n_features) return;
+                    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)(t0 + c) * p.ldo + f;
+                    const int valid = p.n_tokens - (t0 + c);
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) {
+                        const float g = v[q] + b1;
+                        const __nv_bfloat16 r = __float2bfloat16_rn(__fdividef(g * (u[q] + b2), 1.0f + __expf(-g)));
+                        if (q < valid) *o = r;
+                        o += p.ldo;
+                    }
+                };
+                const int c_stop = min(c_end, c_begin + max(0, (p.n_tokens - t0 - c_begin + 15) / 16 * 16));     // columns with tokens
+                float v[16], u[16];
+                int c = c_begin;
+#pragma unroll 1
+                for (; c + 16 < c_stop; c += 16) {
+                    ptx::tmem_load_16_twice(lane_addr + c, lane_addr + BN + c, v, u);
+                    finish(c, v, u);
+                }
+                if (c < c_stop) ptx::tmem_load_16_twice(lane_addr + c, lane_addr + BN + c, v, u);
+                release();
+                if (c < c_stop) finish(c, v, u);
+                continue;
+            }
             // the other pair's partial sums of the next 16 columns are fetched while these 16 are finished
             float pv[16], pu[16];
             auto fetch_partial = [&](int c) {
@@ -537,10 +572,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                 }
             }
-            // this warp has read its part of the buffer: tell the leading block's MMA thread
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive_cluster(lead_empty[buf]);
+            release();
             if (sg.kind == kSegHead || sg.kind == kSegTail) {
                 // the eight epilogue warps of this block: all partial rows written (read) before the flag moves
                 // (an mbarrier, not bar.sync: a warp that gave up elsewhere must not leave the others waiting for ever)
