@@ -782,9 +782,12 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // The even split of K blocks pays when the tiles do not fill whole rounds of pairs, and only with
-    // two weight matrices: with one, the product runs at the power limit of the device either way
-    // (measured: 2048 tokens, gate+up 455 -> 425 us; QKV 79 -> 83 us, down 180 -> 192 us).
+    // The even split of K blocks saves the empty part of the last round and costs about 25 us (partial tiles through
+    // global memory, and pairs that no longer share operands): it pays from about 56 K blocks of saved work per pair on.
+    // Measured, split against whole tiles: gated, 3,000 x 14,336, K 4,096 (9.08 rounds) 520 against 558 us, 1,000 tokens
+    // (3.03 rounds) 190 against 194, 2,048 (6.05 rounds) 344 against 343, 700 (2.27 rounds) 154 against 144; K 2,048, 2,385 x
+    // 8,192 (4.32 rounds) 150 against 131; accumulated, 2,385 x 2,048 (1.08 rounds) with K 8,192 89 against 112 us, with K
+    // 2,048 43 against 40.
     // A pair that finishes a shared tile waits for the pair before it (a lower block index, so it has
     // been started no later), with a limit.  The split is only used when the device can hold all pairs
     // at once (asked once); the launch is an ordinary cluster launch, which profilers take.
@@ -794,7 +797,8 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
         if (cudaOccupancyMaxActiveClusters(&n, gemm_tc2_kernel<MODE>, &cfg) != cudaSuccess) { n = 0; (void)cudaGetLastError(); }
         max_pairs = n;
     }
-    const bool uneven = MODE == kTcSwiGLU && tiles > pairs && tiles % pairs != 0;
+    const long rounds = (tiles + pairs - 1) / pairs;
+    const bool uneven = tiles > pairs && (rounds * pairs - tiles) * p.k_blocks >= 56l * pairs;
     if (!(uneven && pairs <= max_pairs)) { p.sk_partial = nullptr; p.sk_flags = nullptr; }
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<MODE>, mw, mw2, mx, p);
     if (e != cudaSuccess) return fail("gemm_tc2: launch failed: %s", cudaGetErrorString(e));

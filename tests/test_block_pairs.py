@@ -1,0 +1,31 @@
+"""The block-pair product at the edges of its token tiles (a gated tile's last columns are finished after its buffer is given
+back) and where the K blocks of the last rounds are divided among all pairs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("M,N,K,mode", [(1, 512, 64, 2), (15, 300, 128, 2), (16, 256, 128, 2), (17, 256, 128, 2), (33, 256, 192, 2),
+                                        (65, 512, 64, 2), (193, 256, 128, 2), (255, 256, 128, 2), (257, 19000, 128, 2), (500, 19100, 192, 2),
+                                        (512, 9728, 3712, 0), (500, 9700, 3720, 1), (512, 9728, 4096, 2), (300, 9728, 3648, 1)])
+def test_edges(M, N, K, mode):
+    from mdma_b200 import ops, ops_tensor
+    torch.manual_seed(M + N)
+    a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    w, w2 = ((torch.randn(N, K, device=DEV) * K ** -0.5).bfloat16() for _ in range(2))
+    x0 = torch.randn(M + 1, N, device=DEV)
+    for _ in range(2):                          # a second call finds the scratch and its flags as the first left them
+        out = x0.clone() if mode == 1 else torch.full((M + 1, N), 9.0, device=DEV, dtype=torch.bfloat16)
+        keep = out[M:].clone()
+        ops_tensor.gemm(a, w, out, mode, w2 if mode == 2 else None, M, bn=512, splits=1)
+        ops_tensor.check_status(torch.device(DEV))
+        assert torch.equal(out[M:], keep)
+        ref = a.double() @ w.double().t()
+        if mode == 1:                           # sums of K products of order 0.5 / sqrt(K) in float
+            assert bool(((out[:M] - x0[:M].double() - ref).abs() <= 1e-5 * (1 + ref.abs())).all())
+            continue
+        if mode == 2:
+            ref = ref / (1 + torch.exp(-ref)) * (a.double() @ w2.double().t())
+        assert bool(((out[:M].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all())       # one rounding to bfloat16
