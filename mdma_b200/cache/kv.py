@@ -129,8 +129,14 @@ class CacheGroup:
         """Copy the page-table rows that changed to the device."""
         if self.table_dev is None or not self.dirty:
             return
-        for row in sorted(self.dirty):      # straight into the table: no device memory is taken for the copy
-            self.table_dev[row].copy_(torch.from_numpy(self.table_host[row]))
+        # straight into the table: no device memory is taken for the copy; several rows that lie near one another go up
+        # as one piece (the rows between them are the same on the device, or of free slots)
+        first, last = min(self.dirty), max(self.dirty)
+        if len(self.dirty) > 1 and (last - first + 1) * self.max_pages * 4 <= 65536:
+            self.table_dev[first:last + 1].copy_(torch.from_numpy(self.table_host[first:last + 1]))
+        else:
+            for row in sorted(self.dirty):
+                self.table_dev[row].copy_(torch.from_numpy(self.table_host[row]))
         self.dirty.clear()
 
 
@@ -202,41 +208,54 @@ class SequenceCache:
 
     def can_extend(self, extensions: dict[int, int]) -> Optional[str]:
         """None if every slot in {slot: new tokens} can grow, else the reason."""
-        for g in self.groups:
+        for slot, n_new in extensions.items():
+            reach = self.lengths[slot] + n_new
+            if reach > self.max_context:
+                return (f"sequence in slot {slot} would reach {reach} tokens, "
+                        f"beyond the context of {self.max_context}")
+        growing = self._growing(extensions)
+        for g in self.groups if growing else ():
             want = 0
-            for slot, n_new in extensions.items():
-                old = self.lengths[slot]
-                if old + n_new > self.max_context:
-                    return (f"sequence in slot {slot} would reach {old + n_new} tokens, "
-                            f"beyond the context of {self.max_context}")
+            for slot, old, reach in growing:
                 have = g.seq_pages.get(slot, {})
                 first = g.need.first_key(old) // self.page_size
                 if old > 0:                    # pages up to the one that holds position old - 1 are held
                     first = max(first, (old - 1) // self.page_size)
-                last = (old + n_new - 1) // self.page_size
+                last = (reach - 1) // self.page_size
                 want += sum(1 for p in range(first, last + 1) if p not in have)
             if want > g.pages.free_count:
                 return (f"the step needs {want} more cache pages of {self.page_size} tokens, "
                         f"{g.pages.free_count} of {g.n_pages} are free")
         return None
 
-    def extend(self, extensions: dict[int, int]) -> None:
-        """Reserve pages so that each slot can take its new tokens; all or nothing."""
-        why = self.can_extend(extensions)
-        if why:
-            raise CacheFull(why)
+    def _growing(self, extensions: dict[int, int]) -> list[tuple[int, int, int]]:
+        """(slot, tokens it has, tokens it will have) of the sequences whose new tokens go beyond the page of their last
+        one (that page is held): of single tokens, one in `page_size`."""
+        out = []
         for slot, n_new in extensions.items():
             old = self.lengths[slot]
+            if old == 0 or (old - 1) // self.page_size != (old + n_new - 1) // self.page_size:
+                out.append((slot, old, old + n_new))
+        return out
+
+    def extend(self, extensions: dict[int, int], checked: bool = False) -> None:
+        """Reserve pages so that each slot can take its new tokens; all or nothing.  `checked`: `can_extend` has just said
+        that they can."""
+        why = None if checked else self.can_extend(extensions)
+        if why:
+            raise CacheFull(why)
+        for slot, old, reach in self._growing(extensions):
             for g in self.groups:
-                g.grow(slot, old, old + n_new)
+                g.grow(slot, old, reach)
         for g in self.groups:
             g.sync_tables()
 
     def commit(self, extensions: dict[int, int]) -> None:
         """The step ran: the new tokens are part of the sequences."""
+        bounded = [g for g in self.groups if g.need.bounded]
         for slot, n_new in extensions.items():
             self.lengths[slot] += n_new
-            for g in self.groups:
+            for g in bounded:
                 g.trim(slot, self.lengths[slot])
 
     def truncate(self, slot: int, length: int) -> None:

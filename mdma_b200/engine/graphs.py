@@ -22,12 +22,10 @@ from __future__ import annotations
 import gc
 from typing import Optional, Sequence
 
-import numpy as np
 import torch
 
 from .. import ops
 from ..sampling.params import SamplingParams
-from ..cache.slots import CacheFull
 from .step import StepContext, StepError
 
 BUCKET = 1024          # graphs are captured per this many positions of the longest sequence
@@ -46,7 +44,8 @@ class DecodeSession:
             b["ids"], b["tok_pos"], b["seq_slot"], b["seq_pos0"], b["arange"])
         self.ring, self.ring_counter = engine.token_ring, engine.ring_counter
         self.logits = engine.logits
-        self._host = torch.empty(3 * cap, dtype=torch.int32).pin_memory()
+        self._rows = b["rows"]                        # ids, tok_pos, seq_slot, seq_pos0: one upload
+        self._host = torch.zeros(4, cap, dtype=torch.int32).pin_memory()
         self._host_np = self._host.numpy()            # the same pinned words, written without a tensor in between
         self._ring_host = torch.empty(tuple(self.ring.shape), dtype=torch.int32).pin_memory()
         self.ctx = StepContext(engine.rt, engine.workspace)
@@ -80,17 +79,11 @@ class DecodeSession:
         self.requests = list(requests) if requests is not None else list(range(B))
         self.steps_done = list(steps) if steps is not None else [0] * B
         pos = [self.engine.cache.length(s) for s in slots]
-        cap = self.engine.max_slots
         h = self._host_np
         torch.cuda.current_stream().synchronize()       # earlier copies out of the staging words are done
-        h[:B] = np.asarray(list(tokens), dtype=np.int32)
-        h[cap:cap + B] = np.asarray(pos, dtype=np.int32)
-        h[2 * cap:2 * cap + B] = np.asarray(self.slots, dtype=np.int32)
-        self.ids[:B].copy_(self._host[:B], non_blocking=True)
-        self.tok_pos[:B].copy_(self._host[cap:cap + B], non_blocking=True)
-        self.seq_pos0[:B].copy_(self._host[cap:cap + B], non_blocking=True)
-        self.seq_slot[:B].copy_(self._host[2 * cap:2 * cap + B], non_blocking=True)
-        self.engine.h2d_bytes += 16 * B
+        h[0, :B], h[1, :B], h[2, :B], h[3, :B] = list(tokens), pos, self.slots, pos
+        self._rows.copy_(self._host, non_blocking=True)
+        self.engine.h2d_bytes += 4 * self._host.numel()
 
     # ---- one step ----------------------------------------------------------
     @property
@@ -141,10 +134,7 @@ class DecodeSession:
             if n == 1:
                 raise StepError(why)
             n = max(1, n // 2)
-        try:
-            cache.extend(ext)
-        except CacheFull as e:
-            raise StepError(str(e)) from None
+        cache.extend(ext, checked=True)
         p = self.params
         if self._state_stale and self._draws:
             # once per batch: options, requests, step counts and recent tokens go up; from then on the

@@ -103,8 +103,11 @@ def lay_out(model: DecoderModel, carver: Carver, *, dtype, device, sms: int, max
     lay.meta_cap = 6 * chunk_tokens + 4 * max_slots + logit_rows + 16
     lay.meta_dev = carver.take("metadata", (lay.meta_cap,), torch.int32)
     # the replayed decode step reads its inputs from here: ids, positions (twice), slots, 0..cap
-    lay.decode = {name: carver.take("metadata", (max_slots + (1 if name == "arange" else 0),), torch.int32)
-                  for name in ("ids", "tok_pos", "seq_slot", "seq_pos0", "arange")}
+    # (the first four side by side: one copy brings them)
+    rows = carver.take("metadata", (4, max_slots), torch.int32)
+    lay.decode = {name: rows[i] if rows is not None else None for i, name in enumerate(("ids", "tok_pos", "seq_slot", "seq_pos0"))}
+    lay.decode["rows"] = rows
+    lay.decode["arange"] = carver.take("metadata", (max_slots + 1,), torch.int32)
     lay.sampler = DeviceSampler(model.spec.vocab_size, max_slots, device, history_cap, alloc=carver.taker("sampler"))
     # the result words (tokens, flags, status) of the last `run_ahead` replayed decode steps
     lay.token_ring = carver.take("sampler", (max(1, run_ahead), 2 * max_slots + 4), torch.int32)
