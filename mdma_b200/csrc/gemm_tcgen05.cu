@@ -374,30 +374,33 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const PairWork work = pair_work(pair, n_pairs, f_tiles * t_tiles, p.k_blocks, p.sk_flags != nullptr);
     const int n_seg = work.count();
 
-    // This kernel takes no part in programmatic dependent launch: launched early next to the tail of
-    // another kernel it stalled now and then; it is used for many tokens, where a launch gap is
-    // nothing against its run time.
+    // Launched early, the kernel sets up its barriers and waits for the kernel before it BEFORE it takes tensor memory: a
+    // block that held all 512 columns while it waited could keep a block of that kernel, started but not yet at its own
+    // allocation, from ever getting any.  The kernel after it is let in once the columns are taken, for the same reason.
+    // (An early launch takes 3 to 5 us off every product of a prompt: see the launch below.)
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { ptx::mbar_init(full_bar(s), 1); ptx::mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { ptx::mbar_init(acc_full(b), 1); ptx::mbar_init(acc_empty(b), 2 * tc2_epi_warps<MODE>()); }   // epilogue warps x 2 blocks
         ptx::mbar_init(ep_bar, 32 * tc2_epi_warps<MODE>());
         *abort_flag = 0;
         ptx::fence_mbar_init();
+        ptx::prefetch_tensormap(&map_w);
+        ptx::prefetch_tensormap(&map_x);
+        if (kDual) ptx::prefetch_tensormap(&map_w2);
     }
+    chain_wait();
     if (warp == 1) {
         ptx::tmem_alloc_pair(ptx::smem_addr((const void*)tmem_slot), 512);
         ptx::tmem_relinquish_pair();
     }
     ptx::tc_fence_before_sync();
     ptx::cluster_sync();                   // both blocks' barriers exist before either signals the other
+    chain_release();
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0 && lane == 0) {
         // ---- producer: this block's halves; bytes are counted on the leading block's barrier ----
-        ptx::prefetch_tensormap(&map_w);
-        ptx::prefetch_tensormap(&map_x);
-        if (kDual) ptx::prefetch_tensormap(&map_w2);
         int it = 0;                        // stage uses so far, across segments
         bool ok = true;
         for (int si = 0; si < n_seg && ok; ++si) {
@@ -777,9 +780,11 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     const int pairs = (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
     cfg.gridDim = dim3(pairs * 2, 1, 1);
     cfg.blockDim = dim3(tc2_threads<MODE>()); cfg.dynamicSmemBytes = S::kBytes; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // The even split of K blocks saves the empty part of the last round and costs about 25 us (partial tiles through
@@ -800,6 +805,7 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     const long rounds = (tiles + pairs - 1) / pairs;
     const bool uneven = tiles > pairs && (rounds * pairs - tiles) * p.k_blocks >= 56l * pairs;
     if (!(uneven && pairs <= max_pairs)) { p.sk_partial = nullptr; p.sk_flags = nullptr; }
+    cfg.numAttrs = chaining_enabled() ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<MODE>, mw, mw2, mx, p);
     if (e != cudaSuccess) return fail("gemm_tc2: launch failed: %s", cudaGetErrorString(e));
     return 0;

@@ -115,6 +115,12 @@ __device__ __forceinline__ unsigned long long cluster_load_u64(uint32_t remote) 
 __device__ __forceinline__ void cluster_store_u64(uint32_t remote, unsigned long long v) {
     asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v) : "memory");
 }
+// Adds to a word of a block's shared memory; returns what it held.
+__device__ __forceinline__ uint32_t cluster_add_u32(uint32_t remote, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(remote), "r"(v) : "memory");
+    return old;
+}
 __device__ __forceinline__ void cluster_store_f32(uint32_t remote, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }

@@ -719,6 +719,160 @@ __device__ ClusterCrossing find_crossing_cluster(const float* slice, int n, int 
     return c;
 }
 
+// ---- many candidates: the bin that holds the crossing, then a sort of that bin -----------
+// The candidates' bit patterns lie between the min-p threshold's and the leader's.  One pass sums the masses of 2,048
+// equal parts of that range over the cluster (both searches, the top-p cut and the draw, start from the same sums); the
+// part in which the running mass crosses the target is divided again while it may hold more than 1,024 candidates (no
+// candidate's mass is below that of the part's lowest pattern), and its candidates are sorted by the first block.  The
+// draw's target is at most the kept mass, so it crosses at or before the cut and needs no limit.  A part that cannot be
+// divided further (many equal probabilities) is left to the radix descent above.
+constexpr int kBinCount = 2048, kBinCopies = 2;
+struct BinSpace {                 // in the shared memory of the warps' histograms
+    unsigned* limbs;              // [kBinCopies][kBinCount * 3]; the sorted part's keys and running sums afterwards
+    unsigned long long* own;      // [kBinCount] this block's masses, read by the others
+    unsigned long long* all;      // [kBinCount] the cluster's
+    unsigned long long* part;     // [kBinCount] the same of a part that is divided
+};
+
+__device__ void bin_masses(const float* slice, int n, unsigned base, int shift, const BinSpace& b, unsigned long long* all) {
+    const int tid = threadIdx.x;
+    for (int i = tid; i < kBinCopies * kBinCount * 3; i += kSampleThreads) b.limbs[i] = 0u;
+    __syncthreads();
+    unsigned* mine = b.limbs + (tid / (kSampleThreads / kBinCopies)) * kBinCount * 3;
+    DigitPair pair;
+    for (int i = tid; i < n; i += kSampleThreads) {
+        const float p = slice[i];
+        const unsigned at = (__float_as_uint(p) - base) >> shift;
+        if (p > 0.f && __float_as_uint(p) >= base && at < (unsigned)kBinCount) pair.add(mine, (int)at, mass_of(p));
+    }
+    pair.flush(mine);
+    __syncthreads();
+    for (int i = tid; i < kBinCount; i += kSampleThreads) {
+        unsigned long long m = 0ull;
+#pragma unroll
+        for (int c = 0; c < kBinCopies; ++c) m += limb_value(b.limbs + c * kBinCount * 3, i);
+        b.own[i] = m;
+    }
+    ptx::cluster_sync();
+    const uint32_t own = ptx::smem_addr(b.own);
+    for (int i = tid; i < kBinCount; i += kSampleThreads) {
+        unsigned long long m = 0ull;
+#pragma unroll
+        for (int k = 0; k < kSampleCluster; ++k) m += ptx::cluster_load_u64(ptx::cluster_map(own + 8u * i, k));
+        all[i] = m;
+    }
+    ptx::cluster_sync();          // everyone has read this block's masses
+}
+
+// The bin, counted from the top, at which the running mass from `above` reaches `target` (which the bins' masses do
+// reach), and the mass above it; the whole block calls it.
+__device__ int bin_crossing(const unsigned long long* all, unsigned long long above, unsigned long long target, int* misc,
+                            unsigned long long* warp_totals /*32*/, unsigned long long* out_above) {
+    constexpr int kPer = kBinCount / kSampleThreads;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned long long own = 0ull;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) own += all[kBinCount - 1 - (t * kPer + e)];
+    unsigned long long upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += v; }
+    if (lane == 31) warp_totals[warp] = upto;
+    if (t == 0) misc[0] = 0;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) upto += warp_totals[w];
+    unsigned long long run = above + upto - own;
+    if (run < target && run + own >= target) {
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) {
+            const int bin = kBinCount - 1 - (t * kPer + e);
+            const unsigned long long m = all[bin];
+            if (run < target && run + m >= target) { misc[0] = bin; *out_above = run; }
+            run += m;
+        }
+    }
+    __syncthreads();
+    return misc[0];
+}
+
+struct BinAnswer { bool ok; int index; unsigned long long mass; };
+// `all`: the masses of the bins of 2^shift patterns from `base` on; their sum reaches `target`.
+__device__ BinAnswer find_in_bins(const float* slice, int n, int lo, unsigned base, int shift, unsigned long long target,
+                                  const BinSpace& b, SampleExchange* xch, int* misc, unsigned long long* words /*64*/) {
+    const int rank = (int)ptx::cluster_rank(), t = threadIdx.x;
+    const unsigned long long* sums = b.all;
+    unsigned long long above = 0ull;
+    for (;;) {
+        const int bin = bin_crossing(sums, above, target, misc, words, words + 32);
+        above = words[32];
+        const unsigned long long inside = sums[bin];
+        // (the barrier below: everyone has read both before they are written again)
+        base += (unsigned)bin << shift;
+        const unsigned long long least = mass_of(__uint_as_float(base));
+        __syncthreads();
+        if (least > 0ull && inside <= least * (unsigned long long)kSmallMax) break;
+        if (shift == 0) return BinAnswer{false, -1, 0ull};
+        const int finer = shift > 11 ? shift - 11 : 0;
+        bin_masses(slice, n, base, finer, b, b.part);
+        // (a finer division of fewer than 2,048 bins runs on into the next part: those bins lie above the crossing's)
+        for (int i = t; i < kBinCount; i += kSampleThreads) if ((unsigned)i >> (shift - finer)) b.part[i] = 0ull;
+        __syncthreads();
+        sums = b.part;
+        shift = finer;
+    }
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(b.limbs);
+    unsigned long long* cum = keys + kSmallMax;
+    keys[t] = 0ull;
+    if (t == 0) xch->count = 0;
+    ptx::cluster_sync();                              // the first block's list is empty
+    const uint32_t keys0 = ptx::cluster_map(ptx::smem_addr(keys), 0);
+    const uint32_t count0 = ptx::cluster_map(ptx::smem_addr(xch) + (uint32_t)offsetof(SampleExchange, count), 0);
+    for (int i = t; i < n; i += kSampleThreads) {
+        const unsigned bits = __float_as_uint(slice[i]);
+        if (slice[i] > 0.f && bits >= base && (bits - base) >> shift == 0u) {
+            const unsigned at = ptx::cluster_add_u32(count0, 1u);
+            if (at < (unsigned)kSmallMax) ptx::cluster_store_u64(keys0 + at * 8u, small_key(slice[i], lo + i));
+        }
+    }
+    ptx::cluster_sync();                              // the list is complete
+    if (rank == 0) {
+        const int have = min(xch->count, kSmallMax);
+        int size = 32;
+        while (size < have) size <<= 1;
+        for (int k = 2; k <= size; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const int partner = t ^ j;
+                if (t < size && partner > t) {
+                    const unsigned long long x = keys[t], y = keys[partner];
+                    const bool descending = (t & k) == 0;
+                    if (descending ? x < y : x > y) { keys[t] = y; keys[partner] = x; }
+                }
+                __syncthreads();
+            }
+        const unsigned long long key = keys[t];
+        unsigned long long v = t < have ? mass_of(__uint_as_float((unsigned)(key >> 32))) : 0ull;
+        const int lane = t & 31, warp = t >> 5;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const unsigned long long up = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += up; }
+        if (lane == 31) words[warp] = v;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) v += words[w];
+        cum[t] = above + v;
+        __syncthreads();
+        if (t < have && cum[t] >= target && (t == 0 || cum[t - 1] < target)) {
+            xch->answer = (int)(0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull));
+            xch->mass = cum[t];
+        }
+    }
+    ptx::cluster_sync();                              // the first block has its answer
+    const uint32_t xch0 = ptx::smem_addr(xch);
+    BinAnswer a;
+    a.ok = true;
+    a.index = (int)ptx::cluster_load_u32(ptx::cluster_map(xch0 + (uint32_t)offsetof(SampleExchange, answer), 0));
+    a.mass = ptx::cluster_load_u64(ptx::cluster_map(xch0 + (uint32_t)offsetof(SampleExchange, mass), 0));
+    ptx::cluster_sync();                              // and everyone has read it
+    return a;
+}
+
 __global__ void __launch_bounds__(kSampleThreads)
 sample_cluster_kernel(const float* __restrict__ logits, int vocab, int per, const SampleState st,
                       float temperature, float top_p, float min_p, float penalty, int penalty_window,
@@ -825,14 +979,14 @@ sample_cluster_kernel(const float* __restrict__ logits, int vocab, int per, cons
     // 5. probabilities; min-p: keep p >= p_max * min_p (p_max = 1 / sum: the leader's exponential is 1)
     const float thr = min_p > 0.f ? (1.0f / denom) * min_p : 0.f;
     unsigned long long mine = 0ull;
+    int survivors = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         float p = slice[i] / denom;
         if (p < thr) p = 0.f;
         slice[i] = p;
         mine += mass_of(p);
+        survivors += p > 0.f ? 1 : 0;
     }
-    int survivors = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) survivors += slice[i] > 0.f ? 1 : 0;
     const unsigned long long block_mass = block_sum_u64(mine, &total[0]);
     const int block_count = (int)block_sum_u64((unsigned long long)survivors, &total[1]);
     if (threadIdx.x == 0) { xch.mass = block_mass; xch.count = block_count; }
@@ -879,7 +1033,30 @@ sample_cluster_kernel(const float* __restrict__ logits, int vocab, int per, cons
     __syncthreads();
     unsigned long long kept = total[0];
     __syncthreads();
-    // 6. top-p: the smallest descending prefix whose mass reaches top_p
+    // 6. top-p and the draw by bins
+    if (kept > 0ull) {
+        const unsigned first = thr > 0.f ? __float_as_uint(thr) : 1u;
+        const unsigned range = max(__float_as_uint(1.0f / denom), first) - first;
+        const int shift = max(0, 32 - __clz((int)range) - 11);
+        BinSpace b;
+        b.own = small_keys; b.all = b.own + kBinCount; b.part = b.all + kBinCount;
+        b.limbs = reinterpret_cast<unsigned*>(b.part + kBinCount);
+        bin_masses(slice, n, first, shift, b, b.all);
+        BinAnswer cut{true, -1, kept};
+        const unsigned long long goal = mass_of(top_p);
+        if (top_p < 1.0f && goal <= kept) cut = find_in_bins(slice, n, lo, first, shift, goal > 0ull ? goal : 1ull, b, &xch, misc, total);
+        if (cut.ok) {
+            unsigned long long target = (unsigned long long)((double)row_uniform(st, r) * (double)cut.mass);
+            if (target < 1ull) target = 1ull;
+            const BinAnswer drawn = find_in_bins(slice, n, lo, first, shift, target, b, &xch, misc, total);
+            if (drawn.ok) {
+                if (rank == 0 && threadIdx.x == 0) finish_row(st, r, drawn.index, 0, tokens, flags);
+                return;
+            }
+        }
+    }
+    // or, where a bin holds too many equal probabilities, by digits.  Top-p: the smallest descending prefix whose mass
+    // reaches top_p
     int turn = 0;
     unsigned limit_bits = 0;
     int limit_index = -1;
