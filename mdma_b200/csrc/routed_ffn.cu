@@ -54,6 +54,7 @@ template <typename TA, typename TW>
 __device__ __forceinline__ float warp_dot(const TA* __restrict__ a, const TW* __restrict__ w, int n, int lane, bool vec = false) {
     float acc = 0.f;
     if (vec) {
+#pragma unroll 4                                          // four loads of either row in flight
         for (int k = lane * 8; k < n; k += 256) {
             float x[8], y[8];
             load8(a + k, x);
@@ -90,6 +91,11 @@ route_kernel(const TA* __restrict__ h, int h_stride, const TW* __restrict__ rout
              int scoring, int group_top, int renormalize, int logit_bias, float weight_scale,
              int* __restrict__ chosen, float* __restrict__ weights, float* __restrict__ shared_scale) {
     chain_release();
+    // the router's rows come from memory: on their way while the kernel before this one ends (4 tokens, 16 outputs of 1,024
+    // floats: 22 us with a warp waiting for every 256 numbers of every row)
+    const size_t router_bytes = (size_t)n_routed * width * sizeof(TW);
+    for (size_t at = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 128; at < router_bytes; at += (size_t)gridDim.x * blockDim.x * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(router) + at));
     chain_wait();
     __shared__ float z[kMaxRouted];
     __shared__ float c[kMaxRouted];
