@@ -186,7 +186,7 @@ class Attention(Part):
             self._fast_ok = ops_tensor.attention_supported(self.n_heads, self.n_kv_heads, self.head_dim)
         self._tiled_ok = ops.attention_distance_tiled_fits(self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim)
 
-    def _forward_extended(self, ctx, h, x, view, owns_cache):
+    def _forward_extended(self, ctx, h, x, view, owns_cache, stores=False, defer=False):
         """One product for q, k, v and the gate numbers; one kernel rotates and norms q and k and writes the cache;
         attention on the tensor-core kernels where keys and values have one size they take (the sink is theirs, the
         gate a small kernel), else on the CUDA-core kernels, which take the sink, the gate and the scale themselves."""
@@ -212,7 +212,18 @@ class Attention(Part):
             ops.attention_distance(row, view.k, view.v, ctx, view.page_table, view.max_pages, view.page_size, None, gate,
                                    out, self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim, self.window, self.scale,
                                    tiled, sinks=self.sink_f32, gate_heads=True, out_scale=self.out_scale)
-        self.o_proj.accumulate(out, x, n, defer=False)
+        (self.o_proj.store if stores else self.o_proj.accumulate)(out, x, n, defer=defer)
+
+    def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
+        """The result as float rows; `defer`: the last product may leave K-split partial sums of `out` for the caller's next
+        kernel."""
+        if self.extended:
+            return self._forward_extended(ctx, h, out, view, owns_cache, True, defer)
+        out[:ctx.n_tokens].zero_()
+        self.forward(ctx, h, out, view, owns_cache)
+        if self.rt.gemm == "tensor":
+            from .. import ops_tensor
+            ops_tensor.flush_pending(out.device, self.rt.tc)
 
     def forward(self, ctx, h, x, view, owns_cache=True):
         if self.extended:

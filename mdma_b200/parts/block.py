@@ -178,8 +178,8 @@ class SandwichBlock:
         x += post1(mixer(norm1(x)));   x += post2(feed_forward(norm2(x)))       (if the layer has one)
 
     The two norms on the results come from `LayerSpec.extras`: "mixer_post_norm" and "ffn_post_norm"; they must offer
-    `add_normed(ctx, y, x)` (x += norm(y) over float rows).  A sublayer adds its result into a zeroed float buffer
-    through its ordinary `forward`, so any mixer and feed-forward of the registries fits."""
+    `add_normed(ctx, y, x)` (x += norm(y) over float rows).  A sublayer that offers `produce` stores its result, any other
+    adds it into a zeroed float buffer through its ordinary `forward`."""
 
     def __init__(self, spec: LayerSpec):
         self.spec = spec
@@ -204,19 +204,25 @@ class SandwichBlock:
         return {"normed": (self.width, "act"), "sublayer": (self.width, "f32")}
 
     def forward(self, ctx, x, view, owns_cache=True):
-        n = ctx.n_tokens
         h = ctx.buf("normed", self.width)
         y = ctx.buf("sublayer", self.width, torch.float32)
         self.mixer_norm.forward(ctx, x, h)
-        y[:n].zero_()
-        self.mixer.forward(ctx, h, y, view, owns_cache)
-        self.mixer_post.add_normed(ctx, y, x)
+        self._sublayer(ctx, self.mixer, self.mixer_post, h, x, y, view, owns_cache)
         if self.ffn is None:
             return
         self.ffn_norm.forward(ctx, x, h)
-        y[:n].zero_()
-        self.ffn.forward(ctx, h, y)
-        self.ffn_post.add_normed(ctx, y, x)
+        self._sublayer(ctx, self.ffn, self.ffn_post, h, x, y)
+
+    @staticmethod
+    def _sublayer(ctx, part, norm, h, x, y, *more):
+        # (a norm in groups takes partial sums of an added result only)
+        if hasattr(part, "produce") and norm.groups == 1:
+            part.produce(ctx, h, y, *more, defer=True)
+            norm.add_normed(ctx, y, x, stored=True)
+        else:
+            y[:ctx.n_tokens].zero_()
+            part.forward(ctx, h, y, *more)
+            norm.add_normed(ctx, y, x)
 
 
 @BLOCKS.register("postnorm")

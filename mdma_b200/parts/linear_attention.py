@@ -229,14 +229,25 @@ class SideBySide(Part):
         total = sum(self._floats(m) for m, _, _ in self.members)
         return StateNeed((total,), torch.float32) if total else None
 
-    def forward(self, ctx, h, x, view, owns_cache=True):
+    def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
+        """The results' sum as float rows, complete: the first child stores its own where it can."""
+        first, _, folded = self.members[0]
+        stores = folded and hasattr(first, "produce")
+        if not stores:
+            out[:ctx.n_tokens].zero_()
+        self.forward(ctx, h, out, view, owns_cache, stores)
+        if ctx.rt.gemm == "tensor":
+            from .. import ops_tensor
+            ops_tensor.flush_pending(out.device, ctx.rt.tc)
+
+    def forward(self, ctx, h, x, view, owns_cache=True, first_stores=False):
         at = 0
-        for m, scale, folded in self.members:
+        for i, (m, scale, folded) in enumerate(self.members):
             floats = self._floats(m)
             own = dataclasses.replace(view, state=view.state[:, at:at + floats] if floats else None)
             at += floats
             if folded:
-                m.forward(ctx, h, x, own, owns_cache)
+                (m.produce if first_stores and i == 0 else m.forward)(ctx, h, x, own, owns_cache)
                 continue
             tmp = ctx.buf("side_scratch", self.hidden, torch.float32)
             tmp[:ctx.n_tokens].zero_()
