@@ -520,10 +520,11 @@ attention_decode_kernel(const AttnParams p) {
 // arithmetic was two thirds of the instructions.  Needs page_size to be a multiple of KB.  A tile is
 // stored as halves of 64 head elements: [KB keys x 128 bytes] with the 128-byte swizzle.
 // NW warps per block.  All blocks should run at once (a second, short round of blocks costs as
-// much as the first): eight warps and one block per SM while the blocks are no more than the SMs, else
+// much as the first): twelve warps and one block per SM (what its shared memory
+// holds tiles for) while the blocks are no more than the SMs, else
 // four, three or two warps with three, four or five blocks per SM, or one warp with ten.
 template <int DMAX, int KB, int NW, bool EXT = false>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : NW == 4 ? 3 : NW == 3 ? 4 : NW == 2 ? 5 : 10)
+__global__ void __launch_bounds__(NW * 32, NW >= 8 ? 1 : NW == 4 ? 3 : NW == 3 ? 4 : NW == 2 ? 5 : 10)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                             const AttnParams p) {
     constexpr int kChunks = DMAX / 8;
@@ -614,29 +615,43 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         const int half = p.rotary_dim / 2, tail = D - p.rotary_dim;
         const __nv_bfloat16* row = p.q + (size_t)token * p.q_stride;
         const float* prow = p.proj_partial + (size_t)token * p.proj_width;
-        auto load = [&](int col) -> float {              // the projection's value: as stored, or its partial sums in split order
-            if (p.proj_splits == 0) return __bfloat162float(row[col]);
-            float a = 0.f;
+        // two of the projection's values: as stored, or their partial sums in split order (eight loads in flight)
+        auto load = [&](int c0, int c1, float& x0, float& x1) {
+            if (p.proj_splits == 0) { x0 = __bfloat162float(row[c0]); x1 = __bfloat162float(row[c1]); return; }
+            x0 = x1 = 0.f;
             int sidx = 0;
-            for (; sidx + 4 <= p.proj_splits; sidx += 4) {       // four loads in flight, added in order
-                const float* src = prow + (size_t)sidx * p.proj_split_stride + col;
-                const float v0 = __ldcg(src), v1 = __ldcg(src + p.proj_split_stride),
-                            v2 = __ldcg(src + 2 * p.proj_split_stride), v3 = __ldcg(src + 3 * p.proj_split_stride);
-                a += v0; a += v1; a += v2; a += v3;
+            for (; sidx + 4 <= p.proj_splits; sidx += 4) {
+                const float* src = prow + (size_t)sidx * p.proj_split_stride;
+                float a[4], b[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) { a[u] = __ldcg(src + u * p.proj_split_stride + c0); b[u] = __ldcg(src + u * p.proj_split_stride + c1); }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) { x0 += a[u]; x1 += b[u]; }
             }
-            for (; sidx < p.proj_splits; ++sidx) a += __ldcg(prow + (size_t)sidx * p.proj_split_stride + col);
-            return a;
+            for (; sidx < p.proj_splits; ++sidx) {
+                const float* src = prow + (size_t)sidx * p.proj_split_stride;
+                x0 += __ldcg(src + c0); x1 += __ldcg(src + c1);
+            }
         };
         uint8_t* q_tile = smem + NW * 2 * kTile;
         auto q_elem = [&](int r, int d) -> __nv_bfloat16* {
             return reinterpret_cast<__nv_bfloat16*>(q_tile + tile_offset<DMAX>(r, d >> 3) + (d & 7) * 2);
         };
         const int q_col0 = kvh * G * D, k_col0 = (p.n_heads + kvh) * D, v_col0 = (p.n_heads + p.n_kv_heads + kvh) * D;
-        for (int i = threadIdx.x; i < (G + 1) * half; i += NW * 32) {        // the G query heads, then the key head
-            const int r = i / half, pr = i % half;
-            const int d0 = p.rot_interleaved ? 2 * pr : pr, d1 = p.rot_interleaved ? 2 * pr + 1 : pr + half;
-            const int col = r < G ? q_col0 + r * D : k_col0;
-            const float x0 = load(col + d0), x1 = load(col + d1);
+        // the pairs of the G query heads, of the key head, then the value's neighbours: one pass for 4 query heads of 128
+        // with twelve warps (q and k in one loop and v in another, x0 and x1 one after the other, took 3.5 us)
+        const int turned = (G + 1) * half, pairs = turned + D / 2;
+        for (int i = threadIdx.x; i < pairs; i += NW * 32) {
+            const bool value = i >= turned;
+            const int r = value ? G + 1 : i / half, pr = value ? i - turned : i - r * half;
+            const int d0 = value || p.rot_interleaved ? 2 * pr : pr, d1 = value || p.rot_interleaved ? 2 * pr + 1 : pr + half;
+            const int col = value ? v_col0 : r < G ? q_col0 + r * D : k_col0;
+            float x0, x1;
+            load(col + d0, col + d1, x0, x1);
+            if (value) {
+                fresh_v[d0] = __float2bfloat16_rn(x0); fresh_v[d1] = __float2bfloat16_rn(x1);
+                continue;
+            }
             const float sn = sincos[pr], cs = sincos[half + pr];
             const __nv_bfloat16 y0 = __float2bfloat16_rn(x0 * cs - x1 * sn), y1 = __float2bfloat16_rn(x0 * sn + x1 * cs);
             if (r < G) { *q_elem(r, d0) = y0; *q_elem(r, d1) = y1; }
@@ -644,10 +659,11 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         }
         for (int i = threadIdx.x; i < (G + 1) * tail; i += NW * 32) {        // beyond the rotated width: as it is
             const int r = i / tail, d = p.rotary_dim + i % tail;
-            const __nv_bfloat16 y = __float2bfloat16_rn(load((r < G ? q_col0 + r * D : k_col0) + d));
+            float x, again;
+            load((r < G ? q_col0 + r * D : k_col0) + d, (r < G ? q_col0 + r * D : k_col0) + d, x, again);
+            const __nv_bfloat16 y = __float2bfloat16_rn(x);
             if (r < G) *q_elem(r, d) = y; else fresh_k[d] = y;
         }
-        for (int i = threadIdx.x; i < D; i += NW * 32) fresh_v[i] = __float2bfloat16_rn(load(v_col0 + i));
         __syncthreads();
         // the block that holds the last tile keeps the token's key and value for later steps
         if (b1 == blk_hi && b0 < b1 && threadIdx.x < 2 * d_chunks) {
@@ -788,50 +804,75 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1); l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
     l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1); l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
 
-    // ---- combine the four warps' states in warp order ---------------------------
-    // layout in shared memory (reusing the tiles): per warp [16 rows][DMAX + 2] floats
+    // ---- combine the warps' states in warp order --------------------------------
+    // (8 sequences of 512 tokens, 8 kv heads of 128 under 4 query heads each, in the layer chain: 14.1 us with eight warps, every
+    // warp's share worked out for every number and sixteen rows left behind where there are four; 11.4 so)
+    // layout in shared memory (reusing the tiles): per warp [G rows][DMAX + 8] floats (the eight lanes that write a column
+    // pair of eight rows meet no bank twice), then every row's and warp's maximum, sum and share of the row
     __syncthreads();
     float* comb = reinterpret_cast<float*>(smem);
-    constexpr int kRowF = DMAX + 2;
+    constexpr int kRowF = DMAX + 8;
+    float* top = comb + NW * 16 * kRowF;                    // [NW][16] maxima, then as many sums and shares
     {
         float* mine = comb + (size_t)warp * 16 * kRowF;
         const int r_lo = lane >> 2, r_hi = r_lo + 8;
 #pragma unroll
         for (int n = 0; n < DMAX / 8; ++n) {
             const int d = n * 8 + (lane & 3) * 2;
-            mine[r_lo * kRowF + d] = o[n][0]; mine[r_lo * kRowF + d + 1] = o[n][1];
-            mine[r_hi * kRowF + d] = o[n][2]; mine[r_hi * kRowF + d + 1] = o[n][3];
+            if (r_lo < G) *reinterpret_cast<float2*>(mine + r_lo * kRowF + d) = make_float2(o[n][0], o[n][1]);
+            if (r_hi < G) *reinterpret_cast<float2*>(mine + r_hi * kRowF + d) = make_float2(o[n][2], o[n][3]);
         }
         if ((lane & 3) == 0) {
-            mine[r_lo * kRowF + DMAX] = m_lo; mine[r_lo * kRowF + DMAX + 1] = l_lo;
-            mine[r_hi * kRowF + DMAX] = m_hi; mine[r_hi * kRowF + DMAX + 1] = l_hi;
+            top[warp * 16 + r_lo] = m_lo; top[(NW + warp) * 16 + r_lo] = l_lo;
+            top[warp * 16 + r_hi] = m_hi; top[(NW + warp) * 16 + r_hi] = l_hi;
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < G * DV; i += NW * 32) {
-        const int r = i / DV, d = i % DV;
-        float m = -INFINITY;
+    if ((int)threadIdx.x < G) {                             // a row a thread: its maximum, its sum, the warps' shares
+        const int r = threadIdx.x;
+        float m = -INFINITY, l = 0.f;
 #pragma unroll
-        for (int w = 0; w < NW; ++w) m = fmaxf(m, comb[((size_t)w * 16 + r) * kRowF + DMAX]);
-        float l = 0.f, acc = 0.f;
+        for (int w = 0; w < NW; ++w) m = fmaxf(m, top[w * 16 + r]);
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
-            const float mw = comb[((size_t)w * 16 + r) * kRowF + DMAX];
-            if (mw != -INFINITY) {
-                const float f = exp2f(mw - m);
-                l += f * comb[((size_t)w * 16 + r) * kRowF + DMAX + 1];
-                acc += f * comb[((size_t)w * 16 + r) * kRowF + d];
+            const float mw = top[w * 16 + r], f = mw != -INFINITY ? exp2f(mw - m) : 0.f;
+            l += f * top[(NW + w) * 16 + r];
+            top[(2 * NW + w) * 16 + r] = f;
+        }
+        top[r] = m; top[NW * 16 + r] = l;
+    }
+    __syncthreads();
+    const bool even = (((uintptr_t)p.out & 3) | ((uintptr_t)p.out_f32 & 7)) == 0;
+    for (int i = threadIdx.x; i < G * (DV / 2); i += NW * 32) {
+        const int r = i / (DV / 2), d = 2 * (i - r * (DV / 2));
+        const float m = top[r];
+        float l = top[NW * 16 + r];
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const float f = top[(2 * NW + w) * 16 + r];
+            if (f != 0.f) {                                 // (a warp without keys has nothing but zeros)
+                const float2 x = *reinterpret_cast<const float2*>(comb + ((size_t)w * 16 + r) * kRowF + d);
+                acc.x = fmaf(f, x.x, acc.x); acc.y = fmaf(f, x.y, acc.y);
             }
         }
         const int head = kvh * G + r;
         const size_t out_row = EXT ? ((size_t)token * p.n_heads + head) * maps + map : (size_t)token * p.n_heads + head;
         if (p.splits == 1) {
             if (p.sink_log2) l += exp2f(p.sink_log2[head] - m);
-            if (EXT && p.out_f32) p.out_f32[out_row * DV + d] = acc / l;
-            else p.out[out_row * DV + d] = __float2bfloat16_rn(acc / l);
+            const __nv_bfloat162 y = __floats2bfloat162_rn(acc.x / l, acc.y / l);
+            if (EXT && p.out_f32) {
+                float* to = p.out_f32 + out_row * DV + d;
+                if (even) *reinterpret_cast<float2*>(to) = make_float2(acc.x / l, acc.y / l);
+                else { to[0] = acc.x / l; to[1] = acc.y / l; }
+            } else if (even) {
+                *reinterpret_cast<__nv_bfloat162*>(p.out + out_row * DV + d) = y;
+            } else {
+                p.out[out_row * DV + d] = y.x; p.out[out_row * DV + d + 1] = y.y;
+            }
         } else {
             const size_t slot = out_row * p.splits + split;
-            p.part_o[slot * DV + d] = acc;
+            *reinterpret_cast<float2*>(p.part_o + slot * DV + d) = acc;
             if (d == 0) { p.part_ml[slot * 2] = m; p.part_ml[slot * 2 + 1] = l; }
         }
     }
@@ -982,7 +1023,7 @@ static int launch_attention_mma(const void* q, int q_stride, const void* k_cache
             return 0;
         };
         int rc;
-        // few blocks: eight warps each (one block per SM); many: four warps and three blocks per SM
+        // few blocks: twelve warps each (one block per SM); many: four warps and three blocks per SM
         int sm_count = 0, dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
@@ -991,22 +1032,22 @@ static int launch_attention_mma(const void* q, int q_stride, const void* k_cache
         // (up to ten blocks per SM: one warp each.  128 sequences x 8 kv heads at context 580, with the rotary kernel
         // before it: 64.0 us against 77.8 us in two and a bit rounds of four-warp blocks; 184 sequences 88.0 against
         // 98.8 us.  Beyond that, rounds of four-warp blocks: 192 sequences 99.0 us against 110.7 us with one warp)
-        const int nw = blocks <= sm_count ? 8 : blocks <= 3l * sm_count ? 4 : blocks <= 4l * sm_count ? 3 :
+        const int nw = blocks <= sm_count ? 12 : blocks <= 3l * sm_count ? 4 : blocks <= 4l * sm_count ? 3 :
                        blocks <= 5l * sm_count ? 2 : blocks <= 10l * sm_count ? 1 : 4;
         if (kb == 64) {
-            rc = nw == 8 ? launch(attention_decode_tma_kernel<64, 64, 8>, 8, 64)
+            rc = nw == 12 ? launch(attention_decode_tma_kernel<64, 64, 12>, 12, 64)
                : nw == 4 ? launch(attention_decode_tma_kernel<64, 64, 4>, 4, 64)
                : nw == 3 ? launch(attention_decode_tma_kernel<64, 64, 3>, 3, 64)
                : nw == 2 ? launch(attention_decode_tma_kernel<64, 64, 2>, 2, 64)
                          : launch(attention_decode_tma_kernel<64, 64, 1>, 1, 64);
         } else if (head_dim <= 64) {
-            rc = nw == 8 ? launch(attention_decode_tma_kernel<64, kDecodeKeys, 8>, 8, 64)
+            rc = nw == 12 ? launch(attention_decode_tma_kernel<64, kDecodeKeys, 12>, 12, 64)
                : nw == 4 ? launch(attention_decode_tma_kernel<64, kDecodeKeys, 4>, 4, 64)
                : nw == 3 ? launch(attention_decode_tma_kernel<64, kDecodeKeys, 3>, 3, 64)
                : nw == 2 ? launch(attention_decode_tma_kernel<64, kDecodeKeys, 2>, 2, 64)
                          : launch(attention_decode_tma_kernel<64, kDecodeKeys, 1>, 1, 64);
         } else {
-            rc = nw == 8 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 8>, 8, 128)
+            rc = nw == 12 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 12>, 12, 128)
                : nw == 4 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 4>, 4, 128)
                : nw == 3 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 3>, 3, 128)
                : nw == 2 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 2>, 2, 128)
@@ -1098,15 +1139,15 @@ static int launch_attention_mma_general(const void* q, int q_stride, const void*
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         const long blocks = (long)n_seqs * n_kv_heads * maps * splits;
-        const int nw = blocks <= sm_count ? 8 : blocks <= 3l * sm_count ? 4 : blocks <= 5l * sm_count ? 2 : blocks <= 10l * sm_count ? 1 : 4;
+        const int nw = blocks <= sm_count ? 12 : blocks <= 3l * sm_count ? 4 : blocks <= 5l * sm_count ? 2 : blocks <= 10l * sm_count ? 1 : 4;
         int rc;
         if (kb == 64)
-            rc = nw == 8 ? launch(attention_decode_tma_kernel<64, 64, 8, true>, 8, 64)
+            rc = nw == 12 ? launch(attention_decode_tma_kernel<64, 64, 12, true>, 12, 64)
                : nw == 4 ? launch(attention_decode_tma_kernel<64, 64, 4, true>, 4, 64)
                : nw == 2 ? launch(attention_decode_tma_kernel<64, 64, 2, true>, 2, 64)
                          : launch(attention_decode_tma_kernel<64, 64, 1, true>, 1, 64);
         else                     // (narrow heads on pages of 32 use the wide tiles too: the second half is not loaded)
-            rc = nw == 8 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 8, true>, 8, 128)
+            rc = nw == 12 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 12, true>, 12, 128)
                : nw == 4 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 4, true>, 4, 128)
                : nw == 2 ? launch(attention_decode_tma_kernel<128, kDecodeKeys, 2, true>, 2, 128)
                          : launch(attention_decode_tma_kernel<128, kDecodeKeys, 1, true>, 1, 128);
