@@ -48,6 +48,8 @@ struct TcParams {
     int cluster;               // > 1: that many blocks of a cluster split K and reduce through shared memory
     Ending ending;             // bias vectors over the features and the gate's activation
     int pair_tokens;           // block-pair kernel: width of a token tile (a multiple of 32 up to 256)
+    int heads;                 // one-block kernel: that many products side by side (blockIdx.z), the columns of x and of out and the
+                               // rows of the weights in as many equal parts; 0: one product
     float* sk_partial;         // block-pair kernel: one partial tile per pair and block, for tiles shared by two pairs
     int* sk_flags;             // [pairs * 2] zero between launches; non-null switches the even K-block split on
 };
@@ -89,7 +91,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int rank = p.cluster > 1 ? (int)ptx::cluster_rank() : 0;
     const int f0 = (blockIdx.x / p.cluster) * kBM;
     const int t0 = blockIdx.y * BN;
-    const int kb_begin = (p.cluster > 1 ? rank : (int)blockIdx.z) * p.kb_per_split;
+    const int head = p.heads > 0 ? (int)blockIdx.z : 0;
+    const int kb_begin = (p.cluster > 1 ? rank : p.heads > 0 ? 0 : (int)blockIdx.z) * p.kb_per_split;
+    const int w_row = head * p.n_features + f0, x_col = head * p.k_blocks * kBK;      // (heads: K is a multiple of a K block)
     const int kb_end = min(p.k_blocks, kb_begin + p.kb_per_split);
     const int n_kb = kb_end - kb_begin;
 
@@ -121,12 +125,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const uint32_t stage = base + i * S::kStage;
             ptx::mbar_expect_tx(full_bar(i), S::kA * (kDual ? 2 : 1) + S::kB);
             const int k = (kb_begin + i) * kBK;
-            ptx::tma_load_2d(stage, &map_w, full_bar(i), k, f0);
-            if (kDual) ptx::tma_load_2d(stage + S::kA, &map_w2, full_bar(i), k, f0);
+            ptx::tma_load_2d(stage, &map_w, full_bar(i), k, w_row);
+            if (kDual) ptx::tma_load_2d(stage + S::kA, &map_w2, full_bar(i), k, w_row);
         }
         chain_wait();
         for (int i = 0; i < ahead; ++i)
-            ptx::tma_load_2d(base + i * S::kStage + S::kA * (kDual ? 2 : 1), &map_x, full_bar(i), (kb_begin + i) * kBK, t0);
+            ptx::tma_load_2d(base + i * S::kStage + S::kA * (kDual ? 2 : 1), &map_x, full_bar(i), x_col + (kb_begin + i) * kBK, t0);
         int issued = ahead;
         for (int i = ahead; i < n_kb; ++i) {
             const int s = i % kStages;
@@ -134,9 +138,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const uint32_t stage = base + s * S::kStage;
             ptx::mbar_expect_tx(full_bar(s), S::kA * (kDual ? 2 : 1) + S::kB);
             const int k = (kb_begin + i) * kBK;
-            ptx::tma_load_2d(stage, &map_w, full_bar(s), k, f0);
-            if (kDual) ptx::tma_load_2d(stage + S::kA, &map_w2, full_bar(s), k, f0);
-            ptx::tma_load_2d(stage + S::kA * (kDual ? 2 : 1), &map_x, full_bar(s), k, t0);
+            ptx::tma_load_2d(stage, &map_w, full_bar(s), k, w_row);
+            if (kDual) ptx::tma_load_2d(stage + S::kA, &map_w2, full_bar(s), k, w_row);
+            ptx::tma_load_2d(stage + S::kA * (kDual ? 2 : 1), &map_x, full_bar(s), x_col + k, t0);
             ++issued;
         }
         if (*abort_flag) {
@@ -170,7 +174,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     // ---- epilogue: TMEM -> registers -> (cluster reduction) -> global ------------------
     const int quad = warp & 3;                  // the TMEM lanes an epilogue warp may read
-    const int f = f0 + quad * 32 + lane;
+    const int f = f0 + quad * 32 + lane, out_col = head * p.n_features + f;
     constexpr int kColsPerWarp = BN / tc_epi_parts<BN>();                // eight epilogue warps: column halves (sixteen: quarters)
     constexpr int kStep = kColsPerWarp < 16 ? 8 : 16;                    // columns read out of tensor memory at a time
     const int c_lo = ((warp - 2) >> 2) * kColsPerWarp, c_hi = c_lo + kColsPerWarp;
@@ -257,9 +261,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         if (MODE == kTcPartial) {
                             p.partial[((size_t)blockIdx.z * p.n_tokens + t) * p.n_features + f] = r;
                         } else if (p.out_f32) {
-                            reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + f] = r;
+                            reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + out_col] = r;
                         } else {
-                            reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + f] = __float2bfloat16_rn(r);
+                            reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + out_col] = __float2bfloat16_rn(r);
                         }
                     }
                 }
@@ -715,11 +719,12 @@ static int run_tc(const void* x, int ldx, const void* w, const void* w2, int K, 
         configured = true;
     }
     CUtensorMap mw, mw2, mx;
-    if (int rc = make_map_2d(&mw, w, (uint64_t)p.n_features, (uint64_t)K, (uint64_t)K * 2, kBM)) return rc;
+    const uint64_t parts = p.heads > 0 ? p.heads : 1;
+    if (int rc = make_map_2d(&mw, w, (uint64_t)p.n_features * parts, (uint64_t)K, (uint64_t)K * 2, kBM)) return rc;
     mw2 = mw;
     if (MODE == kTcSwiGLU)
         if (int rc = make_map_2d(&mw2, w2, (uint64_t)p.n_features, (uint64_t)K, (uint64_t)K * 2, kBM)) return rc;
-    if (int rc = make_map_2d(&mx, x, (uint64_t)p.n_tokens, (uint64_t)K, (uint64_t)ldx * 2, BN)) return rc;
+    if (int rc = make_map_2d(&mx, x, (uint64_t)p.n_tokens, (uint64_t)K * parts, (uint64_t)ldx * 2, BN)) return rc;
     // the staging of the cluster reduction must fit the stage ring: shrink the cluster until it does
     while (p.cluster > 1 && (p.cluster - 1) * (MODE == kTcSwiGLU ? 2 : 1) * BN * kBM * 4 > S::kStages * S::kStage) {
         --p.cluster;
@@ -978,7 +983,7 @@ int mdma_gemm_tc(int mode, const void* x, int ldx, const void* w, const void* w2
         pc.out = out; pc.ldo = ldo; pc.out_f32 = out_f32;
         pc.n_tokens = n_tokens; pc.n_features = n_features; pc.k_blocks = k_blocks;
         pc.kb_per_split = (k_blocks + c - 1) / c;
-        pc.partial = nullptr; pc.status = status; pc.cluster = c; pc.sk_partial = nullptr; pc.sk_flags = nullptr;
+        pc.partial = nullptr; pc.status = status; pc.cluster = c; pc.heads = 0; pc.sk_partial = nullptr; pc.sk_flags = nullptr;
         pc.ending = ending;
         if (mode == kTcStore) return run_tc_bn<kTcStore>(bn, x, ldx, w, w2, K, pc, 1, stream);
         if (mode == kTcAccumulate) return run_tc_bn<kTcAccumulate>(bn, x, ldx, w, w2, K, pc, 1, stream);
@@ -992,7 +997,7 @@ int mdma_gemm_tc(int mode, const void* x, int ldx, const void* w, const void* w2
     p.n_tokens = n_tokens; p.n_features = n_features; p.k_blocks = k_blocks;
     p.kb_per_split = (k_blocks + splits - 1) / splits;
     splits = (k_blocks + p.kb_per_split - 1) / p.kb_per_split;     // no empty split
-    p.partial = nullptr; p.status = status; p.cluster = 1; p.sk_partial = nullptr; p.sk_flags = nullptr;
+    p.partial = nullptr; p.status = status; p.cluster = 1; p.heads = 0; p.sk_partial = nullptr; p.sk_flags = nullptr;
     p.ending = ending;
     if (bn == 512) {           // the two-block kernel (a pair covers 256 features x 256 tokens)
         // scratch: one partial tile per block of every pair (accumulators x 256 x 128 floats each); the flags,
@@ -1019,6 +1024,28 @@ int mdma_gemm_tc(int mode, const void* x, int ldx, const void* w, const void* w2
     if (splits_used) *splits_used = splits;
     if (defer_reduce) return 0;
     return splitk_reduce_run(mode, scratch, splits, n_tokens, n_features, out, ldo, out_f32, store_act, act, stream);
+}
+
+// A projection applied head by head, out[:, h * N ..] = x[:, h * K ..] w[h]^T, as one launch: a block a head, 128 features and
+// a token tile.  w [heads, N, K]; K a multiple of 64, so that no box of x runs into the next head's columns.  Bound by the
+// launch and by reading and writing the rows once: 2,048 tokens, 16 heads of 128 x 128 took 16 launches of 4 to 8 us.
+int mdma_gemm_tc_heads(const void* x, int ldx, const void* w, void* out, int ldo, int heads, int n_tokens, int n_features, int K,
+                       int* status, cudaStream_t stream) {
+    MDMA_REQUIRE(n_tokens >= 0 && n_features > 0 && heads > 0 && heads <= 65535 && K > 0 && K % kBK == 0,
+                 "gemm_tc_heads: %d products of %d x %d (K a multiple of 64)", heads, n_features, K);
+    MDMA_REQUIRE(ldx % 8 == 0 && (long)ldx >= (long)heads * K && (long)ldo >= (long)heads * n_features, "gemm_tc_heads: row pitches %d and %d", ldx, ldo);
+    MDMA_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0, "gemm_tc_heads: operands must be 16-byte aligned");
+    if (n_tokens == 0) return 0;
+    // token tiles of 64 (two blocks an SM) where a block's own work is short, else of 128
+    const int bn = K <= 256 ? 64 : 128;
+    MDMA_REQUIRE((n_tokens + bn - 1) / bn <= 65535, "gemm_tc_heads: too many token tiles");
+    TcParams p;
+    p.out = out; p.ldo = ldo; p.out_f32 = 0;
+    p.n_tokens = n_tokens; p.n_features = n_features; p.k_blocks = K / kBK; p.kb_per_split = p.k_blocks;
+    p.partial = nullptr; p.status = status; p.cluster = 1; p.heads = heads; p.sk_partial = nullptr; p.sk_flags = nullptr;
+    p.pair_tokens = 0;
+    p.ending = Ending{nullptr, nullptr, kF32, kActSilu, 0, 0.f, 1.f};
+    return run_tc_bn<kTcStore>(bn, x, ldx, w, nullptr, K, p, heads, stream);
 }
 
 // Several products of one shape family in one call: run r multiplies rows [first[r], first[r+1]) of x (and writes the

@@ -213,6 +213,20 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = ops.GE
         st.pending = Pending(out, mode, used.value, M, N)
 
 
+def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int, st: Optional[TensorState] = None) -> None:
+    """out[:m, h*N:(h+1)*N] = a[:m, h*K:(h+1)*K] @ w[h].T for every h in one launch; w [heads, N, K], K a multiple of 64."""
+    _need_cuda(a, w, out)
+    if not (a.dtype == w.dtype == out.dtype == torch.bfloat16):
+        raise KernelError("the tensor-core product takes bfloat16 operands")
+    heads, N, K = w.shape
+    assert w.is_contiguous() and a.stride(1) == 1 and out.stride(1) == 1
+    assert a.shape[1] >= heads * K and out.shape[1] >= heads * N and a.shape[0] >= m and out.shape[0] >= m
+    st = st or _device_state(a.device)
+    flush_pending(a.device, st)
+    _call("tensor", "mdma_gemm_tc_heads", _ptr(a), _i(a.stride(0)), _ptr(w), _ptr(out), _i(out.stride(0)), _i(heads), _i(m), _i(N),
+          _i(K), _ptr(st.status), _stream())
+
+
 def gemm_runs(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, first: list, n_features: int,
               mode: int = ops.GEMM_STORE, w2: Optional[torch.Tensor] = None, st: Optional[TensorState] = None,
               act: int = ops.ACT_SILU, act_limit: float = 0.0, act_alpha: float = 1.0, store_act: bool = False) -> None:

@@ -34,9 +34,10 @@ from .linear import Linear
 
 
 class HeadwiseLinear:
-    """out[:, h*N:(h+1)*N] = a[:, h*K:(h+1)*K] @ w[h].T for every head h; w is [heads, N, K].  Steps of
-    many tokens (256 or more) run head by head on the tensor cores when the shapes allow, others as one
-    launch on the CUDA cores."""
+    """out[:, h*N:(h+1)*N] = a[:, h*K:(h+1)*K] @ w[h].T for every head h; w is [heads, N, K].  One launch for all heads: on
+    the tensor cores where K is a multiple of 64, from a few tokens on (16 heads of 128 x 128, CUDA cores against that: 4 tokens
+    2.7 / 2.4 us, 16 tokens 4.5 / 2.6, 128 tokens 29.8 / 3.4, 2,048 tokens 70 / 8.0; K 512: 8 tokens 3.6 / 4.3, 32 tokens 8.9 /
+    5.0), else on the CUDA cores; other sizes of K run head by head on the tensor cores in steps of many tokens."""
 
     TENSOR_TOKENS = 256       # below this a launch per head costs more than the CUDA-core launch for all heads
 
@@ -49,9 +50,13 @@ class HeadwiseLinear:
             self._tensor_ok = ops_tensor.gemm_supported(self.n, self.k) and self.n % 8 == 0
 
     def run(self, a, out, m):
-        if (self._tensor_ok and m >= self.TENSOR_TOKENS and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
+        together = self.k % 64 == 0
+        if (self._tensor_ok and m >= ((8 if self.k <= 256 else 16) if together else self.TENSOR_TOKENS) and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
                 and out.dtype == torch.bfloat16):
             from .. import ops_tensor
+            if together:
+                ops_tensor.gemm_heads(a, self.w, out, m, self.rt.tc)
+                return
             for h in range(self.heads):
                 ops_tensor.gemm(a[:, h * self.k:(h + 1) * self.k], self.w[h], out[:, h * self.n:(h + 1) * self.n],
                                 ops.GEMM_STORE, None, m, st=self.rt.tc)

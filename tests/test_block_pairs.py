@@ -29,3 +29,18 @@ def test_edges(M, N, K, mode):
         if mode == 2:
             ref = ref / (1 + torch.exp(-ref)) * (a.double() @ w2.double().t())
         assert bool(((out[:M].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all())       # one rounding to bfloat16
+
+
+@pytest.mark.parametrize("heads,N,K", [(1, 128, 64), (3, 40, 128), (5, 130, 64), (2, 300, 192), (4, 64, 320)])
+@pytest.mark.parametrize("M", [1, 63, 65, 129, 300])
+def test_one_launch_for_all_heads(heads, N, K, M):
+    from mdma_b200 import ops_tensor
+    torch.manual_seed(M + N)
+    x = (torch.randn(M, heads * K + 16, device=DEV) * 0.5).bfloat16()[:, 8:]       # a pitch wider than the heads, an odd start
+    w = (torch.randn(heads, N, K, device=DEV) * K ** -0.5).bfloat16()
+    out = torch.full((M + 1, heads * N + 3), 9.0, device=DEV, dtype=torch.bfloat16)
+    ops_tensor.gemm_heads(x, w, out, M)
+    ops_tensor.check_status(torch.device(DEV))
+    ref = torch.einsum("mhk,hnk->mhn", x[:, :heads * K].double().reshape(M, heads, K), w.double()).reshape(M, -1)
+    assert bool(((out[:M, :heads * N].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
+    assert bool((out[M:] == 9.0).all()) and bool((out[:, heads * N:] == 9.0).all())
