@@ -36,7 +36,8 @@ struct ChunkScan {
     float* state; size_t state_stride;
     float* states; float* decays;                   // decays: Mamba-2 only
     float* out;                                     // [rows][heads * vdim]
-    int heads, n, vdim, max_chunks, heads_per_block;
+    int heads, n, vdim, max_chunks;
+    int heads_per_block;                            // Mamba-2: a block's heads; else its parts of 64 columns of v
     // linear attention
     const void* proj; int row_stride, q_col, k_col, v_col;
     const float* decay;
@@ -146,7 +147,8 @@ chunk_sums_kernel(const ChunkScan p) {
     const ChunkRows at = chunk_rows(p, blockIdx.x);
     const int n = at.n;
     if (n <= 0) return;
-    const int h0 = blockIdx.y * p.heads_per_block, c0 = blockIdx.z * kScanCols, cw = min(kScanCols, p.vdim - c0);
+    const int h0 = MAMBA ? blockIdx.y * p.heads_per_block : blockIdx.y;
+    int c0 = (MAMBA ? blockIdx.z : blockIdx.z * p.heads_per_block) * kScanCols, cw = min(kScanCols, p.vdim - c0);
     const int NP = scan_padded(p.n), warp = threadIdx.x >> 5;
     float* k = sm;                                  // [64][NP]
     float* u = k + kScanChunk * NP;                 // [64][64], Mamba-2: twice
@@ -177,6 +179,15 @@ chunk_sums_kernel(const ChunkScan p) {
     const int groups = NP >> 3;                     // pairs of quads of n: 4 g .. and NP / 2 + 4 g ..
     for (int hh = 0; hh < p.heads_per_block; ++hh) {
         float* v = u + (MAMBA ? (hh & 1) * kScanChunk * kScanCols : 0);
+        if (!MAMBA && hh > 0) {                     // the next 64 columns
+            c0 += kScanCols;
+            if (c0 >= p.vdim) break;
+            cw = min(kScanCols, p.vdim - c0);
+            __syncthreads();
+            const int silu = p.in.silu;
+            scan_fill(u, kScanCols, kScanCols, reinterpret_cast<const T*>(p.proj) + (size_t)at.t0 * p.row_stride + p.v_col + h0 * p.vdim + c0, p.row_stride, cw, n,
+                      [=](float z, int i) { return lin_act(z, silu) * weight[i]; });
+        }
         if (MAMBA) {
             scan_copies_done();
             __syncthreads();
@@ -191,7 +202,7 @@ chunk_sums_kernel(const ChunkScan p) {
             }
         }
         __syncthreads();
-        float* to = p.states + ((size_t)blockIdx.x * p.heads + h0 + hh) * p.vdim * p.n;
+        float* to = p.states + ((size_t)blockIdx.x * p.heads + (MAMBA ? h0 + hh : h0)) * p.vdim * p.n;
         for (int tile = threadIdx.x; tile < groups * (kScanCols / 4); tile += kScanThreads) {
             const int na = (tile % groups) << 2, nb = na + (NP >> 1), c = (tile / groups) << 2;
             float4 a[4], b[4];
@@ -333,7 +344,8 @@ chunk_out_kernel(const ChunkScan p) {
     const ChunkRows at = chunk_rows(p, blockIdx.x);
     const int n = at.n;
     if (n <= 0) return;
-    const int h0 = blockIdx.y * p.heads_per_block, c0 = blockIdx.z * kScanCols, cw = min(kScanCols, p.vdim - c0);
+    const int h0 = MAMBA ? blockIdx.y * p.heads_per_block : blockIdx.y;
+    int c0 = (MAMBA ? blockIdx.z : blockIdx.z * p.heads_per_block) * kScanCols, cw = min(kScanCols, p.vdim - c0);
     const int NP = scan_padded(p.n), P = NP + 4;
     float* q = sm;                                  // [64][P]
     float* ks = q + kScanChunk * P;                 // k [64][P], then the state's columns [64 v][128]
@@ -372,8 +384,13 @@ chunk_out_kernel(const ChunkScan p) {
     else if (nj == 3) scan_dots<3>(raw, q + row * P, P, ks + tx * P, P, NP);
     else scan_dots<4>(raw, q + row * P, P, ks + tx * P, P, NP);
     for (int hh = 0; hh < p.heads_per_block; ++hh) {
-        const int h = h0 + hh;
-        __syncthreads();                            // k, or the head before this one's state and u, are done with
+        const int h = MAMBA ? h0 + hh : h0;
+        if (!MAMBA && hh > 0) {                     // the next 64 columns: q k^T stays
+            c0 += kScanCols;
+            if (c0 >= p.vdim) break;
+            cw = min(kScanCols, p.vdim - c0);
+        }
+        __syncthreads();                            // k, or the state and u before these, are done with
         const float* S = p.states + ((size_t)blockIdx.x * p.heads + h) * p.vdim * p.n + (size_t)c0 * p.n;
         if ((p.n & 3) == 0) {
             const int quads = NP >> 2, full = p.n >> 2;
@@ -388,12 +405,17 @@ chunk_out_kernel(const ChunkScan p) {
                 ks[scan_state_quad(c, d >> 2) + (d & 3)] = c < cw && d < p.n ? S[(size_t)c * p.n + d] : 0.f;
             }
         }
-        if (MAMBA) scan_fetch(u, kScanCols, kScanCols, conv + h * p.vdim + c0, p.conv_stride, cw, n);
+        if (MAMBA) {
+            scan_fetch(u, kScanCols, kScanCols, conv + h * p.vdim + c0, p.conv_stride, cw, n);
+        } else if (hh > 0) {
+            const int silu = p.in.silu;
+            scan_fill(u, kScanCols, kScanCols, rows + p.v_col + h * p.vdim + c0, p.row_stride, cw, n, [=](float z, int) { return lin_act(z, silu); });
+        }
         const float* steps = MAMBA ? dt + hh * 3 * kScanChunk : dt;
         const float *cum = steps + kScanChunk, *rest = steps + 2 * kScanChunk;        // Mamba-2 only
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (j >= nj) break;
+            if (j >= nj || (!MAMBA && hh > 0)) break;
             const int c = tx + 16 * j;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -474,10 +496,23 @@ static int run_chunk_scan(ChunkScan p, int n_seqs, cudaStream_t stream) {
     if (MAMBA)
         while (p.heads_per_block < kScanMostHeads && (p.heads / p.groups) % (2 * p.heads_per_block) == 0 &&
                slots * (p.heads / (2 * p.heads_per_block)) * parts >= 220) p.heads_per_block *= 2;
-    const dim3 grid((unsigned)slots, p.heads / p.heads_per_block, parts);
+    dim3 grid((unsigned)slots, p.heads / p.heads_per_block, parts);
+    // Linear attention: a block takes all parts of v, so that q, k and their products are made once, unless that leaves more of
+    // the last round of blocks empty (costs of a block of one part in the same units, by count of instructions)
+    auto whole = [&](long at_once, double shared, double each) {
+        const long blocks = slots * p.heads;
+        auto rounds = [&](long n) { return (double)((n + at_once - 1) / at_once); };
+        return rounds(blocks) * (shared + each * parts) <= rounds(blocks * parts) * (shared + each);
+    };
+    auto set_parts = [&](bool all_of_them) { p.heads_per_block = all_of_them ? parts : 1; grid = dim3((unsigned)slots, p.heads, all_of_them ? 1 : parts); };
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (!MAMBA) set_parts(whole(3l * sms, 0.8, 2.6));
     launch_chained(chunk_sums_kernel<T, MAMBA>, grid, dim3(kScanThreads), sums_smem, stream, p);
     const size_t all = (size_t)p.heads * p.vdim * p.n;
     launch_chained(chunk_starts_kernel<MAMBA>, dim3((unsigned)((all + 255) / 256), n_seqs), dim3(256), 0, stream, p);
+    if (!MAMBA) set_parts(whole(2l * sms, 2.9, 3.5));
     launch_chained(chunk_out_kernel<T, MAMBA>, grid, dim3(kScanThreads), out_smem, stream, p);
     MDMA_LAUNCH_OK("chunk_scan");
     return 0;
