@@ -9,8 +9,8 @@
 
 namespace mdma {
 
-// The blocks that stream W are the faster ones as long as (rows of the matrices) x (passes of 8 rows of A) is small, since
-// every pass reads W again (from the second-level cache); both give the same bits.  Measured, few against tile, us (the
+// The blocks that stream W are the faster ones for up to 8 rows, and beyond as long as (rows of the matrices) x (passes of 8
+// rows of A) is small, since every pass reads W again (from the second-level cache); both give the same bits.  Measured, few against tile, us (the
 // tile with one run on its way): 1,024 x 1,024 with 32 rows 10.5 / 14.9, 64 rows 20.2 / 21.1, 128 rows 35.8 / 25.1; 4,096 x
 // 1,024 with 16 rows 19.8 / 23.5, 24 rows 28.5 / 24.1; gated, 4,096 x 1,024, 8 rows 19.2 / 23.8, 12 rows 29.8 / 24.1.
 constexpr long kFewPasses = 8192;
@@ -61,7 +61,8 @@ template <typename TA, typename TW, typename TO, int MODE>
 static void launch_mode(const void* A, int lda, const void* W, const void* W2, void* out, int ldo, int M, int N, int K,
                         const Ending& e, cudaStream_t stream, int batch, long batch_a, long batch_w, long batch_o) {
     constexpr bool kDual = MODE == kSwiGLU;
-    const bool few = (long)N * (kDual ? 2 : 1) * ((M + kFewRows - 1) / kFewRows) <= kFewPasses;
+    const long passes = (M + kFewRows - 1) / kFewRows;
+    const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= kFewPasses;
     const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats, rows = few ? kFewRows : kTileRows;
     const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, true> : gemm_nt_kernel<TA, TW, TO, MODE, false>;
     launch_chained(kernel, dim3((N + feats - 1) / feats, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads),
