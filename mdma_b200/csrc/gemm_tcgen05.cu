@@ -378,10 +378,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const PairWork work = pair_work(pair, n_pairs, f_tiles * t_tiles, p.k_blocks, p.sk_flags != nullptr);
     const int n_seg = work.count();
 
-    // Launched early, the kernel sets up its barriers and waits for the kernel before it BEFORE it takes tensor memory: a
-    // block that held all 512 columns while it waited could keep a block of that kernel, started but not yet at its own
-    // allocation, from ever getting any.  The kernel after it is let in once the columns are taken, for the same reason.
-    // (An early launch takes 3 to 5 us off every product of a prompt: see the launch below.)
+    // This kernel takes no part in programmatic dependent launch: launched early next to the tail of
+    // another kernel it stalled now and then; it is used for many tokens, where a launch gap is
+    // nothing against its run time.
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { ptx::mbar_init(full_bar(s), 1); ptx::mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { ptx::mbar_init(acc_full(b), 1); ptx::mbar_init(acc_empty(b), 2 * tc2_epi_warps<MODE>()); }   // epilogue warps x 2 blocks
@@ -392,14 +391,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         ptx::prefetch_tensormap(&map_x);
         if (kDual) ptx::prefetch_tensormap(&map_w2);
     }
-    chain_wait();
     if (warp == 1) {
         ptx::tmem_alloc_pair(ptx::smem_addr((const void*)tmem_slot), 512);
         ptx::tmem_relinquish_pair();
     }
     ptx::tc_fence_before_sync();
     ptx::cluster_sync();                   // both blocks' barriers exist before either signals the other
-    chain_release();
     ptx::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -785,11 +782,9 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     const int pairs = (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
     cfg.gridDim = dim3(pairs * 2, 1, 1);
     cfg.blockDim = dim3(tc2_threads<MODE>()); cfg.dynamicSmemBytes = S::kBytes; cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // The even split of K blocks saves the empty part of the last round and costs about 25 us (partial tiles through
@@ -810,7 +805,6 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     const long rounds = (tiles + pairs - 1) / pairs;
     const bool uneven = tiles > pairs && (rounds * pairs - tiles) * p.k_blocks >= 56l * pairs;
     if (!(uneven && pairs <= max_pairs)) { p.sk_partial = nullptr; p.sk_flags = nullptr; }
-    cfg.numAttrs = chaining_enabled() ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<MODE>, mw, mw2, mx, p);
     if (e != cudaSuccess) return fail("gemm_tc2: launch failed: %s", cudaGetErrorString(e));
     return 0;
