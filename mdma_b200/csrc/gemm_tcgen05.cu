@@ -36,8 +36,10 @@ constexpr int kTcThreads = 192; // warp 0: TMA, warp 1: MMA + TMEM, warps 2-5: e
 template <int BN> constexpr int tc_epi_parts() { return BN >= 128 ? 4 : 2; }         // epilogue warps per 32 rows
 template <int BN> constexpr int tc_threads() { return (2 + 4 * tc_epi_parts<BN>()) * 32; }
 // block-pair kernel: warps 2 and up are the epilogue, two warps (column halves) per 32 lanes of tensor memory, four
-// (column quarters) for the gated product, whose single accumulator buffer leaves the epilogue exposed
-template <int MODE> constexpr int tc2_epi_warps() { return MODE == 2 ? 16 : 8; }
+// (column quarters) for the gated product, whose single accumulator buffer leaves the epilogue exposed, and for stored ones,
+// whose activation is more than the time of a tile's products for eight warps (1,500 x 8,192, K 2,048, GELU: 79 us with eight,
+// 53 with sixteen; 45 without the activation)
+template <int MODE> constexpr int tc2_epi_warps() { return MODE == 1 ? 8 : 16; }
 template <int MODE> constexpr int tc2_threads() { return (2 + tc2_epi_warps<MODE>()) * 32; }
 
 struct TcParams {
@@ -459,7 +461,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const int quad = warp & 3;
         const int row = quad * 32 + lane;                   // feature row within this block's half
         constexpr int kParts = tc2_epi_warps<MODE>() / 4;                              // column parts: halves or quarters
-        const int c_begin = ((warp - 2) >> 2) * (bn / kParts), c_end = c_begin + bn / kParts;     // this warp's columns
+        // this warp's columns: its part of the sixteens
+        const int part = (warp - 2) >> 2, c_begin = part * (bn / 16) / kParts * 16, c_end = (part + 1) * (bn / 16) / kParts * 16;
         const uint32_t lead_empty[2] = {ptx::cluster_map(acc_empty(0), 0), ptx::cluster_map(acc_empty(1), 0)};
         // partial tiles in global memory: [pair][block of the pair][accumulator][column][128 rows]
         const size_t part_stride = (size_t)kAccs * BN * 128;
@@ -761,16 +764,6 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     mw2 = mw;
     if (MODE == kTcSwiGLU)
         if (int rc = make_map_2d(&mw2, w2, (uint64_t)p.n_features, (uint64_t)K, (uint64_t)K * 2, kBM)) return rc;
-    // token tiles of up to 256, all of one width: the tokens divided evenly over the fewest tiles (320 tokens: two
-    // tiles of 160, not one of 256 and one that is three quarters empty)
-    const int t_tiles = (p.n_tokens + 255) / 256;
-    // (a multiple of 16 columns for every epilogue warp: 32 with column halves, 64 with quarters)
-    constexpr int kGrain = 16 * (tc2_epi_warps<MODE>() / 4);
-    p.pair_tokens = (((p.n_tokens + t_tiles - 1) / t_tiles) + kGrain - 1) / kGrain * kGrain;
-    if (int rc = make_map_2d(&mx, x, (uint64_t)p.n_tokens, (uint64_t)K, (uint64_t)ldx * 2, p.pair_tokens / 2)) return rc;
-    p.cluster = 1;
-    cudaLaunchConfig_t cfg = {};
-    // persistent: one pair per two SMs at most
     static int sm_count = 0;
     if (sm_count == 0) {
         int dev = 0;
@@ -778,6 +771,28 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         if (sm_count < 2) sm_count = 2;
     }
+    // Token tiles of one width, a multiple of 32 up to 256 (what one MMA of a pair takes): the tokens divided evenly over the
+    // fewest tiles (320 tokens: two tiles of 160, not one of 256 and one that is three quarters empty).  Gated products may
+    // take a few more tiles of 224 or 192 where that makes the rounds of tiles cheaper, a round costing its K blocks (0.72 us
+    // for 256 tokens) and 3.4 us of epilogue that lies open.  Measured, 256 against that: 2,385 x 2 x 8,192, K 2,048 130 / 122 us,
+    // 1,800 x 2 x 5,504 80 / 66, K 4,096, 1,000 x 2 x 14,336 205 / 191.  Narrower tiles (160: 2,048 x 2 x 14,336, K 4,096 335 / 347),
+    // and any for one matrix (2,385 x 2,048, K 8,192 71 / 88; 2,048 x 14,336, K 4,096 167 / 240), lose more to the operands' reads.
+    const long f_tiles = (p.n_features + 255) / 256, most_pairs = sm_count / 2;
+    int t_tiles = (p.n_tokens + 255) / 256;
+    if (MODE == kTcSwiGLU) {
+        auto us = [&](int width) {
+            const long n = f_tiles * ((p.n_tokens + width - 1) / width);
+            return ((n + most_pairs - 1) / most_pairs) * (3.4 + p.k_blocks * (0.72 * width / 256 + 0.03));
+        };
+        int width = 256;
+        for (int narrow = 224; narrow >= 192; narrow -= 32)
+            if (p.n_tokens > 256 && us(narrow) < 0.97 * us(width)) width = narrow;
+        t_tiles = (p.n_tokens + width - 1) / width;
+    }
+    p.pair_tokens = ((p.n_tokens + t_tiles - 1) / t_tiles + 31) / 32 * 32;
+    if (int rc = make_map_2d(&mx, x, (uint64_t)p.n_tokens, (uint64_t)K, (uint64_t)ldx * 2, p.pair_tokens / 2)) return rc;
+    p.cluster = 1;
+    cudaLaunchConfig_t cfg = {};
     const long tiles = (long)((p.n_features + 255) / 256) * ((p.n_tokens + p.pair_tokens - 1) / p.pair_tokens);
     const int pairs = (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
     cfg.gridDim = dim3(pairs * 2, 1, 1);

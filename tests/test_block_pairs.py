@@ -9,6 +9,7 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("M,N,K,mode", [(1, 512, 64, 2), (15, 300, 128, 2), (16, 256, 128, 2), (17, 256, 128, 2), (33, 256, 192, 2),
                                         (65, 512, 64, 2), (193, 256, 128, 2), (255, 256, 128, 2), (257, 19000, 128, 2), (500, 19100, 192, 2),
+                                        (2385, 8192, 128, 2), (1800, 5504, 64, 2), (300, 500, 128, 0),
                                         (512, 9728, 3712, 0), (500, 9700, 3720, 1), (512, 9728, 4096, 2), (300, 9728, 3648, 1)])
 def test_edges(M, N, K, mode):
     from mdma_b200 import ops, ops_tensor
