@@ -97,21 +97,11 @@ rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ partial, int spl
 // consecutive elements (16-byte loads of x and of the partial sums).
 template <typename T> struct Pack4;
 template <> struct Pack4<float> {
-    using Raw = float4;
-    static __device__ __forceinline__ Raw fetch(const float* p) { return *reinterpret_cast<const float4*>(p); }
-    static __device__ __forceinline__ float4 widen(const Raw& r) { return r; }
     static __device__ __forceinline__ void store(float* p, float a, float b, float c, float d) {
         *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
     }
 };
 template <> struct Pack4<__nv_bfloat16> {
-    using Raw = uint2;
-    static __device__ __forceinline__ Raw fetch(const __nv_bfloat16* p) { return *reinterpret_cast<const uint2*>(p); }
-    static __device__ __forceinline__ float4 widen(const Raw& u) {
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-        return make_float4(a.x, a.y, b.x, b.y);
-    }
     static __device__ __forceinline__ void store(__nv_bfloat16* p, float a, float b, float c, float d) {
         __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
         uint2 u;
@@ -121,23 +111,16 @@ template <> struct Pack4<__nv_bfloat16> {
 };
 
 template <typename TO, typename TW, int NV>
-__global__ void __launch_bounds__(1024, NV == 1 ? 2 : 1)
+__global__ void __launch_bounds__(1024)
 rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ partial, int splits, size_t split_stride,
                    const TW* __restrict__ w, const int* __restrict__ rows, TO* __restrict__ y, int width, float eps) {
-    // A step of a few rows (NV 1) is bound by latency: the weights are fetched before the kernel before this one is waited
-    // for, the partial sums four at a time (added in split order).  32 registers a thread, so that a block of 1,024 finds room
-    // beside the product's blocks and waits there: with 60 (eight partial sums at a time) 8 rows of 4,096 with 5 partial
-    // sums took 5.0 us in the layer chain, with one load after the other and the weights last 4.6.
-    constexpr bool kFew = NV == 1;
     __shared__ float scratch[32];
     chain_release();
-    const int n4 = width / 4;
-    typename Pack4<TW>::Raw wv;
-    if (kFew && (int)threadIdx.x < n4) wv = Pack4<TW>::fetch(w + 4 * threadIdx.x);
     chain_wait();
     const int r = blockIdx.x;
     const size_t src = (size_t)(rows ? rows[r] : r) * width;
     float4* xr = reinterpret_cast<float4*>(x + src);
+    const int n4 = width / 4;
     float4 v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -145,28 +128,12 @@ rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ partial, int
         v[i] = e < n4 ? xr[e] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (splits > 0) {
-        if (kFew) {
-            const float* pr = partial + src + 4 * threadIdx.x;
-            for (int s0 = 0; s0 < splits; s0 += 4) {
-                float4 q[4];
+        for (int sidx = 0; sidx < splits; ++sidx) {
+            const float4* pr = reinterpret_cast<const float4*>(partial + (size_t)sidx * split_stride + src);
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    q[u] = (int)threadIdx.x < n4 && s0 + u < splits ? *reinterpret_cast<const float4*>(pr + (size_t)(s0 + u) * split_stride)
-                                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (s0 + u >= splits) break;
-                    v[0].x += q[u].x; v[0].y += q[u].y; v[0].z += q[u].z; v[0].w += q[u].w;
-                }
-            }
-        } else {
-            for (int sidx = 0; sidx < splits; ++sidx) {
-                const float4* pr = reinterpret_cast<const float4*>(partial + (size_t)sidx * split_stride + src);
-#pragma unroll
-                for (int i = 0; i < NV; ++i) {
-                    const int e = i * blockDim.x + threadIdx.x;
-                    if (e < n4) { const float4 q = pr[e]; v[i].x += q.x; v[i].y += q.y; v[i].z += q.z; v[i].w += q.w; }
-                }
+            for (int i = 0; i < NV; ++i) {
+                const int e = i * blockDim.x + threadIdx.x;
+                if (e < n4) { const float4 q = pr[e]; v[i].x += q.x; v[i].y += q.y; v[i].z += q.z; v[i].w += q.w; }
             }
         }
 #pragma unroll
@@ -185,8 +152,9 @@ rmsnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ partial, int
     for (int i = 0; i < NV; ++i) {
         const int e = i * blockDim.x + threadIdx.x;
         if (e < n4) {
-            const float4 f = Pack4<TW>::widen(kFew ? wv : Pack4<TW>::fetch(w + 4 * e));
-            Pack4<TO>::store(yr + 4 * e, v[i].x * scale * f.x, v[i].y * scale * f.y, v[i].z * scale * f.z, v[i].w * scale * f.w);
+            const TW* wp = w + 4 * e;
+            Pack4<TO>::store(yr + 4 * e, v[i].x * scale * to_float(wp[0]), v[i].y * scale * to_float(wp[1]),
+                             v[i].z * scale * to_float(wp[2]), v[i].w * scale * to_float(wp[3]));
         }
     }
 }
@@ -487,7 +455,7 @@ static void launch_rmsnorm(float* x, const float* partial, int splits, size_t sp
                            const int* rows, TO* y, int n_rows, int width, float eps, cudaStream_t stream) {
     auto threads_for = [&](int per) { int t = ((width + per - 1) / per + 31) / 32 * 32; return t < 64 ? 64 : t; };
     const bool aligned = width % 4 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)partial & 15) == 0 &&
-                         ((uintptr_t)y & 15) == 0 && split_stride % 4 == 0 && ((uintptr_t)w & (4 * sizeof(TW) - 1)) == 0;
+                         ((uintptr_t)y & 15) == 0 && split_stride % 4 == 0;
     if (aligned && width <= 16384) {
         // 16-byte accesses; many rows: few threads per row (more rows in flight), few rows: many threads
         if (n_rows >= 512 && width > 1024)
