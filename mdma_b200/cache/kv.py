@@ -268,15 +268,16 @@ class SequenceCache:
             raise ValueError(f"cannot truncate a sequence of {old} tokens to {length}")
         if self.states:
             raise ValueError("a cache with fixed-size per-sequence state cannot be rewound")
+        last = (length - 1) // self.page_size if length else -1
+        # every group is asked before any gives a page back: a refused call leaves the sequence as it was, with the page of
+        # its last token held (`_growing` relies on that)
         for g in self.groups:
             have = g.seq_pages.get(slot, {})
-            if g.need.bounded:
-                first_needed = g.need.first_key(length) // self.page_size
-                last = (length - 1) // self.page_size if length else -1
-                if any(p not in have for p in range(first_needed, last + 1)):
-                    raise ValueError("a windowed group has already released pages of the kept part")
-            keep_last = (length - 1) // self.page_size if length else -1
-            for p in [p for p in have if p > keep_last]:
+            if g.need.bounded and any(p not in have for p in range(g.need.first_key(length) // self.page_size, last + 1)):
+                raise ValueError("a windowed group has already released pages of the kept part")
+        for g in self.groups:
+            have = g.seq_pages.get(slot, {})
+            for p in [p for p in have if p > last]:
                 g.pages.release(have.pop(p))
         self.lengths[slot] = length
 

@@ -169,3 +169,21 @@ def test_token_by_token_growth_holds_exactly_the_pages_it_needs():
         c.extend({a: 1}); c.commit({a: 1})
     c.check()
     assert all(set(g.seq_pages[a]) == {0, 1, 2} for g in c.groups)
+
+
+def test_a_refused_truncate_leaves_every_group_as_it_was():
+    """A group without a window lies before one with a window: the second refuses, and the first must still hold the page of
+    the last token, or the next token would be written into a page that another sequence may own by then."""
+    c = SequenceCache([KVNeed(2, 16, 0), KVNeed(2, 16, 8)], [None, None], 4 * 24, 2, 64, torch.float32, "cpu", page_size=4)
+    a, b = c.acquire(), c.acquire()
+    c.extend({a: 30}); c.commit({a: 30})
+    held = [dict(g.seq_pages[a]) for g in c.groups]
+    with pytest.raises(ValueError, match="windowed"):
+        c.truncate(a, 5)
+    assert c.length(a) == 30 and [g.seq_pages[a] for g in c.groups] == held
+    c.extend({b: 20}); c.commit({b: 20})
+    c.extend({a: 1}); c.commit({a: 1})
+    c.check()
+    for g in c.groups:
+        assert g.table_host[a, 30 // 4] == g.seq_pages[a][30 // 4]
+        assert g.table_host[a, 30 // 4] not in g.seq_pages[b].values()
