@@ -208,7 +208,7 @@ class SequenceCache:
 
     def can_extend(self, extensions: dict[int, int]) -> Optional[str]:
         """None if every slot in {slot: new tokens} can grow, else the reason."""
-        for slot, n_new in extensions.items():
+        for slot, n_new in extensions.items() if self.groups else ():        # (fixed-size state takes any length)
             reach = self.lengths[slot] + n_new
             if reach > self.max_context:
                 return (f"sequence in slot {slot} would reach {reach} tokens, "

@@ -121,6 +121,20 @@ def test_context_limit():
     assert c.can_extend({s: 128}) is None
 
 
+def test_the_context_bounds_keys_and_not_fixed_size_state():
+    """Layers that keep no keys (recurrences only) go on beyond the context, in one extension or token by token."""
+    c = SequenceCache([None, None], [StateNeed((4,)), StateNeed((8,))], 64 * 4, 2, 128, torch.float32, "cpu", page_size=64)
+    assert not c.groups
+    s = c.acquire()
+    assert c.can_extend({s: 129}) is None
+    c.extend({s: 127}); c.commit({s: 127})
+    for _ in range(3):
+        assert c.can_extend({s: 1}) is None
+        c.extend({s: 1}); c.commit({s: 1})
+    assert c.length(s) == 130
+    c.check()
+
+
 def test_truncate_gives_pages_back_and_refuses_what_cannot_be_rewound():
     needs = [KVNeed(2, 16, 0)]
     c = SequenceCache(needs, [None], 64 * 8, 2, 512, torch.float32, "cpu", page_size=64)
