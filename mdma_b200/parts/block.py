@@ -178,8 +178,8 @@ class SandwichBlock:
         x += post1(mixer(norm1(x)));   x += post2(feed_forward(norm2(x)))       (if the layer has one)
 
     The two norms on the results come from `LayerSpec.extras`: "mixer_post_norm" and "ffn_post_norm"; they must offer
-    `add_normed(ctx, y, x)` (x += norm(y) over float rows).  A sublayer that offers `produce` stores its result, any other
-    adds it into a zeroed float buffer through its ordinary `forward`."""
+    `add_normed(ctx, y, x)` (x += norm(y) over float rows).  A sublayer that offers `produce` stores its result where the
+    norm takes stored results (`adds_stored`), any other adds it into a zeroed float buffer through its ordinary `forward`."""
 
     def __init__(self, spec: LayerSpec):
         self.spec = spec
@@ -215,8 +215,7 @@ class SandwichBlock:
 
     @staticmethod
     def _sublayer(ctx, part, norm, h, x, y, *more):
-        # (a norm in groups takes partial sums of an added result only)
-        if hasattr(part, "produce") and norm.groups == 1:
+        if hasattr(part, "produce") and getattr(norm, "adds_stored", False):
             part.produce(ctx, h, y, *more, defer=True)
             norm.add_normed(ctx, y, x, stored=True)
         else:

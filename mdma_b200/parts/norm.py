@@ -30,6 +30,8 @@ class RMSNorm(Part):
             raise ValueError(f"a row of {self.width} numbers does not split into {self.groups} equal parts")
         if self.groups > 1:
             self.fuses_pending = False      # the grouped kernel reads complete rows of x
+        # `add_normed(.., stored=True)` completes a stored product's partial sums itself (the grouped kernel: an added one's only)
+        self.adds_stored = self.groups == 1
 
     def tensor_specs(self):
         return {"weight": TensorSpec((self.width,), "vector")}
