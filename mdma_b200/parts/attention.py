@@ -218,16 +218,18 @@ class Attention(Part):
         """The result as float rows; `defer`: the last product may leave K-split partial sums of `out` for the caller's next
         kernel."""
         if self.extended:
-            return self._forward_extended(ctx, h, out, view, owns_cache, True, defer)
-        out[:ctx.n_tokens].zero_()
-        self.forward(ctx, h, out, view, owns_cache)
-        if self.rt.gemm == "tensor":
-            from .. import ops_tensor
-            ops_tensor.flush_pending(out.device, self.rt.tc)
+            self._forward_extended(ctx, h, out, view, owns_cache, True, defer)
+        else:
+            self.o_proj.store(self._attend(ctx, h, view, owns_cache), out, ctx.n_tokens, defer=defer)
 
     def forward(self, ctx, h, x, view, owns_cache=True):
         if self.extended:
-            return self._forward_extended(ctx, h, x, view, owns_cache)
+            self._forward_extended(ctx, h, x, view, owns_cache)
+        else:
+            self.o_proj.accumulate(self._attend(ctx, h, view, owns_cache), x, ctx.n_tokens)
+
+    def _attend(self, ctx, h, view, owns_cache):
+        """The heads' outputs, as the last product reads them."""
         n = ctx.n_tokens
         qkv = ctx.buf("qkv", self.row_width)
         out = ctx.buf("attn_out", self.q_width)
@@ -239,8 +241,7 @@ class Attention(Part):
             self.qkv_proj.store(h, qkv, n, defer=True)
             ops_tensor.attention_decode_rotary(ctx, qkv, view, out, self.n_heads, self.n_kv_heads, self.head_dim,
                                                self.window, self.scale, inv_freq, rotary_dim, interleaved, st=self.rt.tc)
-            self.o_proj.accumulate(out, x, n)
-            return
+            return out
         self.qkv_proj.store(h, qkv, n, defer=getattr(self.position, "fuses_pending", False))
         self.position.encode_and_store(ctx, qkv, self.n_heads, self.n_kv_heads, self.head_dim, view, write)
         if self.rt.attention == "fast" and self._fast_ok:
@@ -254,7 +255,7 @@ class Attention(Part):
             ops.attention_simple(qkv, n, view.k, view.v, ctx.tok_seq, ctx.tok_pos, ctx.seq_slot,
                                  view.page_table, view.max_pages, view.page_size, out,
                                  self.n_heads, self.n_kv_heads, self.head_dim, self.window, self.scale)
-        self.o_proj.accumulate(out, x, n)
+        return out
 
     def _fusable(self, ctx, view) -> bool:
         """Whether this step's attention kernel should do the position encoding and the cache write
