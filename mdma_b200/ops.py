@@ -402,14 +402,15 @@ def mamba2_scan(conv, proj, dt_col: int, dt_bias, a_log, d, seq_start, seq_slot,
     assert conv.dtype == proj.dtype == y.dtype == torch.float32 and conv.stride(1) == 1 and proj.stride(1) == 1
     assert y.is_contiguous() and y.shape[1] == heads * vdim and conv.shape[1] == heads * vdim + 2 * groups * n_state
     sp, ss = _state(state)
+    w_dtype = _same_dtype(dt_bias, a_log, d)
     if chunk_rows > 0 and chunk_rows == chunk_scan_rows(n_state, vdim) and not wide_state and scratch.data_ptr() % 16 == 0:
         _call("core", "mdma_mamba2_chunks", _ptr(conv), _i(conv.stride(0)), _ptr(proj), _i(proj.stride(0)), _i(dt_col),
-              _ptr(dt_bias), _ptr(a_log), _ptr(d), _i(dtype_code(d.dtype)), _ptr(seq_start), _ptr(seq_slot), sp, ss, _ptr(y),
+              _ptr(dt_bias), _ptr(a_log), _ptr(d), _i(w_dtype), _ptr(seq_start), _ptr(seq_slot), sp, ss, _ptr(y),
               _i(n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(max_chunks), _ptr(scratch),
               ctypes.c_long(scratch.numel()), _stream(), launches=3)
         return
     _call("core", "mdma_mamba2_scan", _ptr(conv), _i(conv.stride(0)), _ptr(proj), _i(proj.stride(0)), _i(dt_col),
-          _ptr(dt_bias), _ptr(a_log), _ptr(d), _i(_same_dtype(dt_bias, a_log, d)), _ptr(seq_start), _ptr(seq_slot),
+          _ptr(dt_bias), _ptr(a_log), _ptr(d), _i(w_dtype), _ptr(seq_start), _ptr(seq_slot),
           sp, ss, _ptr(y), _i(n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(chunk_rows), _i(max_chunks),
           _ptr(scratch), ctypes.c_long(scratch.numel() if scratch is not None else 0), _i(int(wide_state)), _stream(),
           launches=3 if chunk_rows > 0 else 1)

@@ -114,3 +114,23 @@ def test_mamba2(lengths, heads, groups, vdim, N):
 def test_heads_beyond_the_kernels():
     from mdma_b200 import ops
     assert ops.chunk_scan_rows(129, 64) == 0 and ops.chunk_scan_rows(256, 64) == 0 and ops.chunk_scan_rows(128, 300) == 64
+
+
+@pytest.mark.parametrize("chunk_rows", [0, 64])
+@pytest.mark.parametrize("odd", ["dt_bias", "a_log", "d", "strided"])
+def test_small_vectors_of_several_dtypes_are_refused_before_any_launch(chunk_rows, odd):
+    from mdma_b200 import ops
+    heads, vdim, N, T = 4, 8, 8, 70
+    vectors = {name: torch.zeros(heads, device=DEV, dtype=torch.bfloat16) for name in ("dt_bias", "a_log", "d")}
+    if odd == "strided":
+        vectors["a_log"] = torch.zeros(2 * heads, device=DEV, dtype=torch.bfloat16)[::2]
+    else:
+        vectors[odd] = vectors[odd].float()
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    conv, proj = torch.zeros(T, heads * vdim + 2 * N, device=DEV), torch.zeros(T, heads, device=DEV)
+    y = torch.full((T, heads * vdim), 9.0, device=DEV)
+    before = ops.LAUNCHES
+    with pytest.raises(AssertionError, match="one dtype"):
+        ops.mamba2_scan(conv, proj, 0, vectors["dt_bias"], vectors["a_log"], vectors["d"], i32(0, T), i32(0), torch.zeros(1, heads * N * vdim, device=DEV),
+                        y, 1, heads, vdim, N, 1, chunk_rows, 2, torch.zeros(2 * (heads * N * vdim + heads), device=DEV))
+    assert ops.LAUNCHES == before and bool((y == 9.0).all())
