@@ -118,7 +118,8 @@ __device__ __forceinline__ void scan_steps(const ChunkScan& p, int h, int t0, in
     double upto = a0 + a1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const double v = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += v; }
-    const double first = upto - a1;
+    // (from the rows before, not as upto - a1: a later row that is not finite must leave this one alone)
+    const double before = __shfl_up_sync(0xffffffffu, upto, 1), first = (lane > 0 ? before : 0.0) + a0;
     dt[2 * lane] = d0; dt[2 * lane + 1] = d1;
     cum[2 * lane] = (float)first; rest[2 * lane] = (float)(first - (double)(float)first);
     cum[2 * lane + 1] = (float)upto; rest[2 * lane + 1] = (float)(upto - (double)(float)upto);
@@ -333,7 +334,7 @@ __device__ __forceinline__ void scan_dots_state(float (&acc)[4][4], const float*
 }
 
 // Block = (chunk, heads_per_block heads, 64 columns of v).  Warp w owns rows 8 w .. 8 w + 7, so it needs the columns of
-// q k^T and the rows of u up to 8 w + 7 only; a thread owns four neighbouring rows, of q k^T the columns tx, tx + 16, ..,
+// q k^T and the rows of u up to 8 w + 7 only (a thread's rows take none beyond their own); a thread owns four neighbouring rows, of q k^T the columns tx, tx + 16, ..,
 // of the result the columns 4 tx .. 4 tx + 3.
 template <typename T, bool MAMBA>
 __global__ void __launch_bounds__(kScanThreads, 2)
@@ -420,9 +421,9 @@ chunk_out_kernel(const ChunkScan p) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = row + i;
-                float f = 0.f;
-                if (c <= r) f = MAMBA ? scan_decay(cum, rest, r, c) * steps[c] : steps[r - c];
-                A[r * kScanPitch + c] = raw[i][j] * f;
+                float f = 0.f;                      // (chosen, not multiplied: a later row may hold anything)
+                if (c <= r) f = raw[i][j] * (MAMBA ? scan_decay(cum, rest, r, c) * steps[c] : steps[r - c]);
+                A[r * kScanPitch + c] = f;
             }
         }
         scan_copies_done();
@@ -435,11 +436,12 @@ chunk_out_kernel(const ChunkScan p) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] *= start;
         }
-        for (int j0 = 0; j0 < 8 * warp + 8; j0 += kScanTerms) {
+        // the thread's rows see the rows of u up to their own, no later one: 0 times a number that is not finite is not 0
+        for (int j0 = 0; j0 < row + 4; j0 += kScanTerms) {
             float4 o[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            const int stop = min(8 * warp + 8, j0 + kScanTerms);
+            const int stop = min(row, j0 + kScanTerms);
 #pragma unroll 2
             for (int j = j0; j < stop; j += 4) {
                 float4 x[4], y[4];
@@ -449,6 +451,14 @@ chunk_out_kernel(const ChunkScan p) {
                 for (int e = 0; e < 4; ++e) y[e] = ld4(u + (j + e) * kScanCols + 4 * tx);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) { fma4(o[i], x[i].x, y[0]); fma4(o[i], x[i].y, y[1]); fma4(o[i], x[i].z, y[2]); fma4(o[i], x[i].w, y[3]); }
+            }
+            if (row < j0 + kScanTerms) {            // the thread's own four rows
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float4 y = ld4(u + (row + e) * kScanCols + 4 * tx);
+#pragma unroll
+                    for (int i = e; i < 4; ++i) fma4(o[i], A[(row + i) * kScanPitch + row + e], y);
+                }
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) { acc[i][0] += o[i].x; acc[i][1] += o[i].y; acc[i][2] += o[i].z; acc[i][3] += o[i].w; }

@@ -134,3 +134,51 @@ def test_small_vectors_of_several_dtypes_are_refused_before_any_launch(chunk_row
         ops.mamba2_scan(conv, proj, 0, vectors["dt_bias"], vectors["a_log"], vectors["d"], i32(0, T), i32(0), torch.zeros(1, heads * N * vdim, device=DEV),
                         y, 1, heads, vdim, N, 1, chunk_rows, 2, torch.zeros(2 * (heads * N * vdim + heads), device=DEV))
     assert ops.LAUNCHES == before and bool((y == 9.0).all())
+
+
+@pytest.mark.parametrize("at", [0, 1, 2, 5, 8, 12, 35, 63, 64, 77, 127])
+@pytest.mark.parametrize("where", ["k", "v"])
+def test_a_row_that_is_not_finite_leaves_the_rows_before_it_alone_linear_attention(at, where):
+    from mdma_b200 import ops
+    H, dim, vdim, T = 2, 32, 70, 130
+    g = torch.Generator(device=DEV).manual_seed(at)
+    proj = torch.randn(T, 2 * H * dim + H * vdim, device=DEV, generator=g)
+    start, slot = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([0, T], [0]))
+    decay = torch.tensor([0.99, 0.2], device=DEV)
+    outs = []
+    for bad in (None, float("inf"), float("nan")):
+        rows = proj.clone()
+        if bad is not None:
+            rows[at, H * dim + 3 if where == "k" else 2 * H * dim + 5] = bad
+        out = torch.empty(T, H * vdim, device=DEV)
+        ops.linear_attention(rows, 0, H * dim, 2 * H * dim, decay, start, slot, torch.zeros(1, H * dim * vdim, device=DEV), out, 1, H, dim,
+                             vdim, True, 64, 3, torch.empty(3 * H * dim * vdim, device=DEV), silu=False)
+        outs.append(out)
+    assert torch.isfinite(outs[0]).all()
+    for out in outs[1:]:
+        assert torch.equal(out[:at], outs[0][:at]) and not torch.isfinite(out[at]).all()
+
+
+@pytest.mark.parametrize("at", [0, 1, 2, 5, 8, 12, 35, 63, 64, 77, 127])
+@pytest.mark.parametrize("where", ["x", "B", "dt"])
+def test_a_row_that_is_not_finite_leaves_the_rows_before_it_alone_mamba2(at, where):
+    from mdma_b200 import ops
+    heads, vdim, N, T = 2, 70, 32, 130
+    g = torch.Generator(device=DEV).manual_seed(at)
+    conv, proj = torch.randn(T, heads * vdim + 2 * N, device=DEV, generator=g), torch.randn(T, heads, device=DEV, generator=g)
+    start, slot = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([0, T], [0]))
+    zeros = torch.zeros(heads, device=DEV)
+    outs = []
+    for bad in (None, float("inf"), float("nan")):
+        c, p = conv.clone(), proj.clone()
+        if bad is not None and where == "dt":
+            p[at, 0] = bad
+        elif bad is not None:
+            c[at, 5 if where == "x" else heads * vdim + 3] = bad
+        y = torch.empty(T, heads * vdim, device=DEV)
+        ops.mamba2_scan(c, p, 0, zeros, zeros, zeros, start, slot, torch.zeros(1, heads * N * vdim, device=DEV), y, 1, heads, vdim, N, 1, 64, 3,
+                        torch.empty(3 * (heads * N * vdim + heads), device=DEV))
+        outs.append(y)
+    assert torch.isfinite(outs[0]).all()
+    for y in outs[1:]:
+        assert torch.equal(y[:at], outs[0][:at]) and not torch.isfinite(y[at]).all()
