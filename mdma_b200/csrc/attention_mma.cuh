@@ -835,8 +835,9 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         for (int w = 0; w < NW; ++w) m = fmaxf(m, top[w * 16 + r]);
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
-            const float mw = top[w * 16 + r], f = mw != -INFINITY ? exp2f(mw - m) : 0.f;
-            l += f * top[(NW + w) * 16 + r];
+            const float mw = top[w * 16 + r];
+            float f = -1.f;                                 // a warp without keys has no share
+            if (mw != -INFINITY) { f = exp2f(mw - m); l += f * top[(NW + w) * 16 + r]; }
             top[(2 * NW + w) * 16 + r] = f;
         }
         top[r] = m; top[NW * 16 + r] = l;
@@ -851,7 +852,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             const float f = top[(2 * NW + w) * 16 + r];
-            if (f != 0.f) {                                 // (a warp without keys has nothing but zeros)
+            if (f != -1.f) {                                // (a share that underflows still meets values that are not finite)
                 const float2 x = *reinterpret_cast<const float2*>(comb + ((size_t)w * 16 + r) * kRowF + d);
                 acc.x = fmaf(f, x.x, acc.x); acc.y = fmaf(f, x.y, acc.y);
             }

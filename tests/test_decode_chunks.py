@@ -63,3 +63,35 @@ def test_decode_in_pieces(H, K, hd, splits, keys):
     want = reference_attention(qkv2[:, :H * hd].double().cpu().reshape(B, H, hd), dense, list(range(B)), cached, scale, 0)
     close(out[:B], want, 2e-2, 2e-2)
     assert bool((out[B:] == 9.0).all())
+
+
+def _decode(H, K, hd, cached, splits, fill, st=None):
+    """One token for each sequence over filled pages (`fill(keys, values)` changes them first); the pages' plain decode form."""
+    from mdma_b200 import ops_tensor
+    from test_kernels import DEV, StepMeta, fill_cache
+    page, B = 64, len(cached)
+    kc, vc, table, max_pages, _ = fill_cache([c + 1 for c in cached], K, hd, page, torch.bfloat16, seed=hd, poison=False)
+    fill(kc, vc, table)
+
+    class View:
+        pass
+    view = View()
+    view.k, view.v, view.page_table, view.max_pages, view.page_size = kc, vc, table, max_pages, page
+    g = torch.Generator(device=DEV).manual_seed(5)
+    qkv = torch.rand(B, (H + 2 * K) * hd, device=DEV, generator=g).bfloat16()
+    out = torch.full((B, H * hd), 9.0, device=DEV, dtype=torch.bfloat16)
+    ops_tensor.attention(StepMeta(cached, [1] * B), qkv, view, out, H, K, hd, 0, 1.0 / math.sqrt(hd), splits=splits, st=st)
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("splits", [1, 2])
+@pytest.mark.parametrize("B", [1, 120])
+def test_a_value_that_is_not_finite_shows_however_small_its_share(B, splits):
+    """A key whose weight underflows beside another warp's: 0 times infinity is not a number, here as anywhere."""
+    def fill(k, v, table):
+        k.zero_()
+        k[table[0, 0].item(), 0] = 1e4                          # a score of tens of thousands beside zeros
+        v[table[0, 1].item(), 7] = float("inf")
+    out = _decode(4, 2, 64, [127] * B, splits, fill)
+    assert not torch.isfinite(out[0]).any() and torch.isfinite(out[1:]).all()
