@@ -843,7 +843,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
         top[r] = m; top[NW * 16 + r] = l;
     }
     __syncthreads();
-    const bool even = (((uintptr_t)p.out & 3) | ((uintptr_t)p.out_f32 & 7)) == 0;
+    const bool even = (((uintptr_t)p.out & 3) | (((uintptr_t)p.out_f32 | (uintptr_t)p.part_o) & 7)) == 0;     // any address will do
     for (int i = threadIdx.x; i < G * (DV / 2); i += NW * 32) {
         const int r = i / (DV / 2), d = 2 * (i - r * (DV / 2));
         const float m = top[r];
@@ -873,7 +873,9 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             }
         } else {
             const size_t slot = out_row * p.splits + split;
-            *reinterpret_cast<float2*>(p.part_o + slot * DV + d) = acc;
+            float* to = p.part_o + slot * DV + d;
+            if (even) *reinterpret_cast<float2*>(to) = acc;
+            else { to[0] = acc.x; to[1] = acc.y; }
             if (d == 0) { p.part_ml[slot * 2] = m; p.part_ml[slot * 2 + 1] = l; }
         }
     }

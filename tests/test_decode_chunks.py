@@ -95,3 +95,16 @@ def test_a_value_that_is_not_finite_shows_however_small_its_share(B, splits):
         v[table[0, 1].item(), 7] = float("inf")
     out = _decode(4, 2, 64, [127] * B, splits, fill)
     assert not torch.isfinite(out[0]).any() and torch.isfinite(out[1:]).all()
+
+
+@pytest.mark.gpu
+def test_partial_sums_on_a_boundary_of_four_bytes():
+    """Scratch is any array of floats: an odd one gives the bits of an even one."""
+    from mdma_b200 import ops_tensor
+    from test_kernels import DEV
+    outs = []
+    for first in (0, 1):
+        st = ops_tensor.TensorState(torch.device(DEV), 0, scratch=torch.full((6 * 8 * 3 * 66 + 1,), float("nan"), device=DEV)[first:])
+        outs.append(_decode(8, 2, 64, [0, 63, 64, 200, 129, 31], 3, lambda *pages: None, st))
+        ops_tensor.check_status(torch.device(DEV), st)
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
