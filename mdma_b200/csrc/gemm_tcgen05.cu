@@ -504,8 +504,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     const int valid = p.n_tokens - (t0 + c);
 #pragma unroll
                     for (int q = 0; q < 16; ++q) {
-                        const float g = v[q] + b1;
-                        const __nv_bfloat16 r = __float2bfloat16_rn(__fdividef(g * (u[q] + b2), 1.0f + __expf(-g)));
+                        const __nv_bfloat16 r = __float2bfloat16_rn(gated_pair_fast(v[q] + b1, u[q] + b2, kActSilu, 0.f, 1.f));
                         if (q < valid) *o = r;
                         o += p.ldo;
                     }

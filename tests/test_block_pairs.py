@@ -45,3 +45,27 @@ def test_one_launch_for_all_heads(heads, N, K, M):
     ref = torch.einsum("mhk,hnk->mhn", x[:, :heads * K].double().reshape(M, heads, K), w.double()).reshape(M, -1)
     assert bool(((out[:M, :heads * N].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5).all())
     assert bool((out[M:] == 9.0).all()) and bool((out[:, heads * N:] == 9.0).all())
+
+
+@pytest.mark.parametrize("bn", [512, 128])
+def test_gates_far_from_zero(bn):
+    """Gates whose exponential nearly overflows, or does, beside inputs of any size: silu(g) is rounded before it meets u, so
+    that neither a quotient by more than 2^126 nor a product of g and u beyond the floats shows.  Bound: the result's rounding
+    to bfloat16 (2^-9) and the fast exponential's 2 + 1.2 |g| units of a float (2^-16 at 88)."""
+    from mdma_b200 import ops, ops_tensor
+    dev = torch.device("cuda:0")
+    gates, ups = [-88.0, -80.0, -20.0, -1.0, 0.0, 3.0, 88.0, -1e20, -3e38], [1e30, -1e25, 1e-20, 1.0, 1e20]
+    M, N, K = 300, 256, 64
+    x = torch.zeros(M, K, device=dev, dtype=torch.bfloat16)
+    x[:, 0] = 1.0
+    w, w2 = (torch.zeros(N, K, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    for f in range(N):
+        w[f, 0], w2[f, 0] = gates[f % 9], ups[f // 9 % 5]
+    out = torch.empty(M, N, device=dev, dtype=torch.bfloat16)
+    ops_tensor.gemm(x, w, out, ops.GEMM_SWIGLU, w2, M, bn=bn, splits=1)
+    ops_tensor.check_status(dev)
+    g, u = w[:, 0].double(), w2[:, 0].double()
+    want = g / (1.0 + torch.exp(-g)) * u
+    assert torch.isfinite(out).all()
+    # (what is below the smallest normal float may come out as 0)
+    assert bool(((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2.0 ** -126 * u.abs().clamp(min=1.0)).all())
