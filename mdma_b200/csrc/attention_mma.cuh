@@ -895,12 +895,11 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
     float l = 0.f;
     for (int s = 0; s < splits; ++s) if (ml[s * 2] != -INFINITY) l += exp2f(ml[s * 2] - m) * ml[s * 2 + 1];
     if (sink_log2) l += exp2f(sink_log2[th % n_heads] - m);          // the sink counts once, whatever the split
-    const float inv = 1.0f / l;
     for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
         float acc = 0.f;
         for (int s = 0; s < splits; ++s)
             if (ml[s * 2] != -INFINITY) acc += exp2f(ml[s * 2] - m) * part_o[(th * splits + s) * head_dim + d];
-        out[th * head_dim + d] = __float2bfloat16_rn(acc * inv);
+        out[th * head_dim + d] = __float2bfloat16_rn(acc / l);      // (as the kernel itself ends where nothing is split)
     }
 }
 

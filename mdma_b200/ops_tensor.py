@@ -39,9 +39,9 @@ def scratch_floats_bound(sms: int, max_tokens: int, max_seqs: int, attention_sha
     products, need = need, 0          # a projection's partial sums and the attention's can be alive together
     for heads, kv_heads, head_dim in attention_shapes:
         group = max(1, heads // max(kv_heads, 1))
-        # Keys are split only while the grid is short of blocks (see `attention_splits`): decode has
-        # sequences x kv heads blocks < 2 x SMs and splits <= 3 x SMs / blocks + 1, so tokens x splits
-        # < 5 x SMs / kv heads; other steps have tokens <= blocks x tile tokens / kv heads and
+        # While the grid is short of blocks (see `attention_splits`) decode has sequences x kv heads blocks
+        # < 2 x SMs and splits <= 3 x SMs / blocks + 1, so tokens x splits < 5 x SMs / kv heads; where blocks cover
+        # the device, `decode_chunks` keeps to the same number of them; other steps have tokens <= blocks x tile tokens / kv heads and
         # splits <= 2 x SMs / blocks + 1, so tokens x splits < 4 x SMs x tile tokens / kv heads.
         tile_tokens = max(1, 64 // group)
         need = max(need, 5 * sms * group * (head_dim + 2), 4 * sms * tile_tokens * group * (head_dim + 2))
@@ -301,17 +301,25 @@ def attention_splits(n_seqs: int, max_new: int, max_len: int, n_heads: int, n_kv
 CHUNK_KEYS = 1024        # (512 measures the same)
 
 
-def decode_chunks(n_seqs: int, max_len: int, n_kv_heads: int, sms: int) -> tuple[int, int]:
+def decode_chunks(n_seqs: int, max_len: int, n_kv_heads: int, sms: int, most_seqs: Optional[int] = None,
+                  most_len: Optional[int] = None) -> tuple[int, int]:
     """(splits, keys per split) of a single-token step whose blocks, one per (sequence, kv head), already cover the
     device (`attention_splits` gives 1): contexts beyond 1,024 are cut into pieces of the same number of keys for
-    every sequence, so that the device does not wait for the longest one's blocks.  No more than 5 x SMs blocks (the
-    scratch that engines reserve); (1, 0): whole contexts.  Measured, 8 sequences of 255 to 2,040 tokens, 32 kv heads of 128:
-    a whole decode step of 32 layers 4.26 -> 3.77 ms with the merge that the pieces need."""
-    longest = -(-max_len // 1024) * 1024           # as the replayed decode graphs see it
-    splits = min(longest // CHUNK_KEYS, 5 * sms // (n_seqs * n_kv_heads))
-    if longest <= 1024 or n_seqs * n_kv_heads < sms or splits < 2:
+    every sequence, so that the device does not wait for the longest one's blocks.  The length of a piece, a multiple of
+    1,024, follows from the most sequences and the longest context that the engine can hold, whose pieces are no more than
+    5 x SMs blocks (the scratch that engines reserve); only their number follows the live ones.  A sequence's keys are
+    therefore cut at the same places whoever its batch mates are (one that lies within a piece is summed up as if it were not
+    cut at all).  (1, 0): whole contexts.  Measured, 8 sequences of 255 to 2,040 tokens, 32 kv heads of 128: a whole
+    decode step of 32 layers 4.26 -> 3.77 ms with the merge that the pieces need."""
+    if n_seqs * n_kv_heads < sms:
         return 1, 0
-    return splits, -(-longest // splits // 64) * 64
+    most = -(-max(max_len, most_len or 0) // CHUNK_KEYS)          # in pieces of the shortest kind
+    pieces = 5 * sms // (max(n_seqs, most_seqs or 0) * n_kv_heads)
+    if pieces < 2 or most < 2:
+        return 1, 0
+    keys = -(-most // pieces) * CHUNK_KEYS
+    splits = -(-max_len // keys)
+    return (splits, keys) if splits > 1 else (1, 0)
 
 
 def attention_tc_supported(n_heads: int, n_kv_heads: int, head_dim: int, page_size: int) -> bool:
@@ -417,7 +425,8 @@ def attention_decode_rotary(ctx, qkv: torch.Tensor, view, out: torch.Tensor, n_h
     if splits is None:
         splits = attention_splits(ctx.n_seqs, 1, ctx.max_len, n_heads, n_kv_heads, st.sms, getattr(ctx, "most_seqs", None))
         if splits == 1 and not window:
-            splits, chunk_keys = decode_chunks(ctx.n_seqs, ctx.max_len, n_kv_heads, st.sms)
+            splits, chunk_keys = decode_chunks(ctx.n_seqs, -(-ctx.max_len // 1024) * 1024, n_kv_heads, st.sms,
+                                               getattr(ctx, "most_seqs", None), getattr(ctx, "most_len", None))
     assert chunk_keys == 0 or chunk_keys * splits >= ctx.max_len
     # the attention's own partials (keys split over blocks) lie behind the projection's
     used = -(-proj_splits * stride // 64) * 64
