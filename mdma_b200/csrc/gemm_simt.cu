@@ -27,7 +27,7 @@ template <typename TA, typename TW, typename TO, int MODE, bool FEW>
 __global__ void __launch_bounds__(kRowsThreads)
 gemm_nt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, const TW* __restrict__ W2,
                TO* __restrict__ out, int ldo, int M, int N, int K, const Ending e,
-               long batch_a, long batch_w, long batch_o) {
+               long batch_a, long batch_w, long batch_o, int w_fixed) {
     constexpr bool kDual = MODE == kSwiGLU;
     extern __shared__ __align__(16) float smem[];
     chain_release();
@@ -38,7 +38,9 @@ gemm_nt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, cons
     out += (size_t)blockIdx.z * batch_o;
     constexpr int kRows = FEW ? kFewRows : kTileRows;
     const bool vec_a = rows_of_four(A, lda, K), vec_w = rows_of_four(W, K, K) && (!kDual || rows_of_four(W2, K, K));
-    if (!FEW) chain_wait();
+    // A matrix that no kernel on its way can write (a model's weight) is asked for while the kernel before this one ends: 4 % of
+    // a generation of the 32-bit engine.
+    if (!FEW || !w_fixed) chain_wait();
     for (int m0 = blockIdx.y * kRows; m0 < M; m0 += gridDim.y * kRows) {
         const int rows = min(kRows, M - m0);
         auto row_of = [&](int m) { return A + (size_t)(m0 + m) * lda; };
@@ -59,7 +61,7 @@ gemm_nt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, cons
 
 template <typename TA, typename TW, typename TO, int MODE>
 static void launch_mode(const void* A, int lda, const void* W, const void* W2, void* out, int ldo, int M, int N, int K,
-                        const Ending& e, cudaStream_t stream, int batch, long batch_a, long batch_w, long batch_o) {
+                        const Ending& e, int w_fixed, cudaStream_t stream, int batch, long batch_a, long batch_w, long batch_o) {
     constexpr bool kDual = MODE == kSwiGLU;
     const long passes = (M + kFewRows - 1) / kFewRows;
     const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= kFewPasses;
@@ -67,17 +69,17 @@ static void launch_mode(const void* A, int lda, const void* W, const void* W2, v
     const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, true> : gemm_nt_kernel<TA, TW, TO, MODE, false>;
     launch_chained(kernel, dim3((N + feats - 1) / feats, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads),
                    rows_product_smem(kernel, few), stream, (const TA*)A, lda,
-                   (const TW*)W, (const TW*)W2, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o);
+                   (const TW*)W, (const TW*)W2, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o, w_fixed);
 }
 
 template <typename TA, typename TW, typename TO>
 static int launch_gemm(int mode, const void* A, int lda, const void* W, const void* W2, void* out, int ldo,
-                       int M, int N, int K, const Ending& e, cudaStream_t stream,
+                       int M, int N, int K, const Ending& e, int w_fixed, cudaStream_t stream,
                        int batch = 1, long batch_a = 0, long batch_w = 0, long batch_o = 0) {
-    if (mode == kStore) launch_mode<TA, TW, TO, kStore>(A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
-    else if (mode == kAccumulate) launch_mode<TA, TW, TO, kAccumulate>(A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
-    else if (mode == kSwiGLU) launch_mode<TA, TW, TO, kSwiGLU>(A, lda, W, W2, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
-    else if (mode == kStoreAct) launch_mode<TA, TW, TO, kStoreAct>(A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+    if (mode == kStore) launch_mode<TA, TW, TO, kStore>(A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
+    else if (mode == kAccumulate) launch_mode<TA, TW, TO, kAccumulate>(A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
+    else if (mode == kSwiGLU) launch_mode<TA, TW, TO, kSwiGLU>(A, lda, W, W2, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
+    else if (mode == kStoreAct) launch_mode<TA, TW, TO, kStoreAct>(A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
     else return fail("gemm_simt: unknown mode %d", mode);
     MDMA_LAUNCH_OK("gemm_simt");
     return 0;
@@ -89,7 +91,7 @@ using namespace mdma;
 extern "C" int mdma_gemm_simt(int mode, const void* A, int a_dtype, int lda, const void* W, const void* W2,
                               int w_dtype, void* out, int out_dtype, int ldo, int M, int N, int K,
                               const void* bias, const void* bias2, int bias_dtype, int act, float act_limit, float act_alpha,
-                              cudaStream_t stream) {
+                              int w_fixed, cudaStream_t stream) {
     MDMA_REQUIRE(M >= 0 && N > 0 && K > 0 && lda >= K && ldo >= N, "gemm_simt: bad sizes M=%d N=%d K=%d lda=%d ldo=%d", M, N, K, lda, ldo);
     MDMA_REQUIRE(mode != kSwiGLU || W2 != nullptr, "gemm_simt: SwiGLU needs two weights");
     MDMA_REQUIRE(mode != kAccumulate || out_dtype == kF32, "gemm_simt: the residual stream is float");
@@ -100,11 +102,11 @@ extern "C" int mdma_gemm_simt(int mode, const void* A, int a_dtype, int lda, con
     if (M == 0) return 0;
     const Ending e{bias, mode == kSwiGLU ? bias2 : nullptr, bias_dtype, act, 0, act_limit, act_alpha};
     if (a_dtype == kF32 && w_dtype == kF32 && out_dtype == kF32)
-        return launch_gemm<float, float, float>(mode, A, lda, W, W2, out, ldo, M, N, K, e, stream);
+        return launch_gemm<float, float, float>(mode, A, lda, W, W2, out, ldo, M, N, K, e, w_fixed, stream);
     if (a_dtype == kBF16 && w_dtype == kBF16 && out_dtype == kBF16)
-        return launch_gemm<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(mode, A, lda, W, W2, out, ldo, M, N, K, e, stream);
+        return launch_gemm<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(mode, A, lda, W, W2, out, ldo, M, N, K, e, w_fixed, stream);
     if (a_dtype == kBF16 && w_dtype == kBF16 && out_dtype == kF32)
-        return launch_gemm<__nv_bfloat16, __nv_bfloat16, float>(mode, A, lda, W, W2, out, ldo, M, N, K, e, stream);
+        return launch_gemm<__nv_bfloat16, __nv_bfloat16, float>(mode, A, lda, W, W2, out, ldo, M, N, K, e, w_fixed, stream);
     return fail("gemm_simt: unsupported dtypes a=%d w=%d out=%d", a_dtype, w_dtype, out_dtype);
 }
 
@@ -113,18 +115,18 @@ extern "C" int mdma_gemm_simt(int mode, const void* A, int a_dtype, int lda, con
 // applied head by head is one call: the heads lie side by side in the rows of A and of out.
 extern "C" int mdma_gemm_simt_batched(const void* A, int a_dtype, int lda, long batch_a, const void* W, int w_dtype,
                                       long batch_w, void* out, int out_dtype, int ldo, long batch_o, int batch,
-                                      int M, int N, int K, cudaStream_t stream) {
+                                      int M, int N, int K, int w_fixed, cudaStream_t stream) {
     MDMA_REQUIRE(M >= 0 && N > 0 && K > 0 && batch > 0 && batch <= 65535, "gemm_simt_batched: bad sizes M=%d N=%d K=%d batch=%d", M, N, K, batch);
     MDMA_REQUIRE((M + 63) / 64 <= 65535, "gemm_simt_batched: too many rows (%d)", M);
     if (M == 0) return 0;
     const Ending e{nullptr, nullptr, kF32, kActSilu};
     if (a_dtype == kF32 && w_dtype == kF32 && out_dtype == kF32)
-        return launch_gemm<float, float, float>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+        return launch_gemm<float, float, float>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
     if (a_dtype == kBF16 && w_dtype == kBF16 && out_dtype == kBF16)
-        return launch_gemm<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+        return launch_gemm<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
     if (a_dtype == kBF16 && w_dtype == kBF16 && out_dtype == kF32)
-        return launch_gemm<__nv_bfloat16, __nv_bfloat16, float>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+        return launch_gemm<__nv_bfloat16, __nv_bfloat16, float>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
     if (a_dtype == kF32 && w_dtype == kBF16 && out_dtype == kF32)       // float rows through matrices kept in bfloat16 (a recurrence's gates)
-        return launch_gemm<float, __nv_bfloat16, float>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, stream, batch, batch_a, batch_w, batch_o);
+        return launch_gemm<float, __nv_bfloat16, float>(kStore, A, lda, W, nullptr, out, ldo, M, N, K, e, w_fixed, stream, batch, batch_a, batch_w, batch_o);
     return fail("gemm_simt_batched: unsupported dtypes a=%d w=%d out=%d", a_dtype, w_dtype, out_dtype);
 }

@@ -127,9 +127,10 @@ def ending_args(n_features: int, bias: Optional[torch.Tensor], bias2: Optional[t
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = GEMM_STORE,
               w2: Optional[torch.Tensor] = None, m: Optional[int] = None, bias: Optional[torch.Tensor] = None,
               bias2: Optional[torch.Tensor] = None, act: int = ACT_SILU, act_limit: float = 0.0,
-              act_alpha: float = 1.0) -> None:
+              act_alpha: float = 1.0, w_fixed: bool = False) -> None:
     """out[:m] (=, +=) a[:m] @ w.T (+ bias) on the CUDA cores; the gated mode takes gate=w, up=w2 and
-    gives act(gate) * up."""
+    gives act(gate) * up.  `w_fixed`: no kernel launched so far still writes the matrices (a model's weights), so that they
+    may be read while the kernel before this one ends."""
     _need_cuda(a, w, out, w2)
     assert a.dim() == 2 and w.dim() == 2 and out.dim() == 2
     assert a.stride(1) == 1 and out.stride(1) == 1 and w.is_contiguous()
@@ -140,7 +141,8 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = G
         assert w2.shape == w.shape and w2.dtype == w.dtype and w2.is_contiguous()
     _call("core", "mdma_gemm_simt", _i(mode), _ptr(a), _i(dtype_code(a.dtype)), _i(a.stride(0)),
           _ptr(w), _ptr(w2), _i(dtype_code(w.dtype)), _ptr(out), _i(dtype_code(out.dtype)),
-          _i(out.stride(0)), _i(M), _i(N), _i(K), *ending_args(N, bias, bias2, act, act_limit, act_alpha), _stream())
+          _i(out.stride(0)), _i(M), _i(N), _i(K), *ending_args(N, bias, bias2, act, act_limit, act_alpha), _i(int(w_fixed)),
+          _stream())
 
 
 def rope_cache_write(qkv: torch.Tensor, n_tokens: int, tok_seq, tok_pos, seq_slot, inv_freq,
@@ -426,16 +428,16 @@ def gated_group_rmsnorm(y, z, w, out, n_rows: int, groups: int, eps: float) -> N
           _i(dtype_code(w.dtype)), _ptr(out), _i(dtype_code(out.dtype)), _i(n_rows), _i(width), _i(groups), _f(eps), _stream())
 
 
-def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int) -> None:
+def gemm_simt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int, w_fixed: bool = False) -> None:
     """out[:m, z*N:(z+1)*N] = a[:m, z*K:(z+1)*K] @ w[z].T for every z: w [batch, N, K]; the pieces of a
-    row (one per head) lie side by side in a and in out."""
+    row (one per head) lie side by side in a and in out.  `w_fixed`: as in `gemm_simt`."""
     _need_cuda(a, w, out)
     batch, N, K = w.shape
     assert w.is_contiguous() and a.stride(1) == 1 and out.stride(1) == 1
     assert a.shape[1] >= batch * K and out.shape[1] >= batch * N and a.shape[0] >= m and out.shape[0] >= m
     _call("core", "mdma_gemm_simt_batched", _ptr(a), _i(dtype_code(a.dtype)), _i(a.stride(0)), ctypes.c_long(K),
           _ptr(w), _i(dtype_code(w.dtype)), ctypes.c_long(N * K), _ptr(out), _i(dtype_code(out.dtype)),
-          _i(out.stride(0)), ctypes.c_long(N), _i(batch), _i(m), _i(N), _i(K), _stream())
+          _i(out.stride(0)), ctypes.c_long(N), _i(batch), _i(m), _i(N), _i(K), _i(int(w_fixed)), _stream())
 
 
 # ---- attention over a cached latent (csrc/latent_attention.cu) ------------------------------------------------

@@ -64,7 +64,7 @@ class HeadwiseLinear:
         if self.rt.gemm == "tensor":
             from .. import ops_tensor
             ops_tensor.flush_pending(a.device, self.rt.tc)
-        ops.gemm_simt_batched(a, self.w, out, m)
+        ops.gemm_simt_batched(a, self.w, out, m, w_fixed=True)
 
 
 @MIXERS.register("latent_attention")

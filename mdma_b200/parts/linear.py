@@ -40,7 +40,8 @@ class Linear:
             if self.rt.gemm == "tensor":
                 from .. import ops_tensor
                 ops_tensor.flush_pending(a.device, self.rt.tc)
-            ops.gemm_simt(a, self.w, out, mode, self.w2, m, self.bias, self.bias2, self.act, self.act_limit, self.act_alpha)
+            ops.gemm_simt(a, self.w, out, mode, self.w2, m, self.bias, self.bias2, self.act, self.act_limit, self.act_alpha,
+                          w_fixed=True)
 
     def store(self, a, out, m, defer: bool = False):
         """out = a W^T.  `defer`: a K-split product may leave its partial sums for the

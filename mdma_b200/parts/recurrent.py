@@ -272,8 +272,8 @@ class RGLRU(_StatefulMixer):
         ops.causal_conv_silu(p, w, self.conv_w, self.conv_b, self.taps, w, ctx.tok_seq, ctx.seq_start, ctx.seq_slot,
                              conv_state, u, n, ctx.n_seqs, silu=False)
         # the gates' block-diagonal products read the float rows; float sums on the CUDA cores in both engines
-        ops.gemm_simt_batched(u, self.ra, r, n)
-        ops.gemm_simt_batched(u, self.ri, i, n)
+        ops.gemm_simt_batched(u, self.ra, r, n, w_fixed=True)
+        ops.gemm_simt_batched(u, self.ri, i, n, w_fixed=True)
         # long prompts in the serving engine: runs of a sequence side by side; the 32-bit engine keeps the row-by-row
         # order, so that its results do not depend on how a prompt was cut
         runs = ctx.max_new >= self.RUNS_FROM and s.dtype != torch.float32

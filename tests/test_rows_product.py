@@ -70,3 +70,31 @@ def test_experts_by_expert(tokens, experts, top, width, ff, gated):
         want = want + share * (z @ D.double()[e * width:(e + 1) * width].t())
     # two products of up to 256 and 130 terms of order one
     assert bool(((x - want).abs() <= 2e-5 * (1 + want.abs())).all())
+
+
+@pytest.mark.parametrize("batch", [0, 4])
+def test_a_matrix_that_the_kernel_before_writes(batch):
+    """The matrix is read after its writer has ended, unless the caller says that nothing writes it (`w_fixed`)."""
+    from mdma_b200 import ops
+    N, K, M = 4096, 1024, 4
+    sources = [torch.randn(N, K, device=DEV) for _ in range(2)]
+    w = torch.zeros(N, K, device=DEV, dtype=torch.bfloat16)
+    a = torch.randn(M, max(batch, 1) * K, device=DEV).bfloat16()
+
+    def product(out, **more):
+        if batch:
+            ops.gemm_simt_batched(a, w.view(batch, N // batch, K), out, M, **more)
+        else:
+            ops.gemm_simt(a, w, out, **more)
+    want = [torch.empty(M, N, device=DEV) for _ in range(2)]
+    for source, out in zip(sources, want):
+        w.copy_(source)
+        torch.cuda.synchronize()
+        product(out, w_fixed=True)
+        torch.cuda.synchronize()
+    outs = [torch.empty(M, N, device=DEV) for _ in range(20)]
+    for i, out in enumerate(outs):
+        ops.copy_rows(sources[i % 2], w, N)
+        product(out)
+    assert not torch.equal(*want)
+    assert all(torch.equal(out, want[i % 2]) for i, out in enumerate(outs))
