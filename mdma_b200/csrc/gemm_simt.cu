@@ -10,10 +10,13 @@
 namespace mdma {
 
 // The blocks that stream W are the faster ones for up to 8 rows, and beyond as long as (rows of the matrices) x (passes of 8
-// rows of A) is small, since every pass reads W again (from the second-level cache); both give the same bits.  Measured, few against tile, us (the
-// tile with one run on its way): 1,024 x 1,024 with 32 rows 10.5 / 14.9, 64 rows 20.2 / 21.1, 128 rows 35.8 / 25.1; 4,096 x
-// 1,024 with 16 rows 19.8 / 23.5, 24 rows 28.5 / 24.1; gated, 4,096 x 1,024, 8 rows 19.2 / 23.8, 12 rows 29.8 / 24.1.
-constexpr long kFewPasses = 8192;
+// rows of A) is small, since every pass reads W again (from the second-level cache): 8,192 for two passes, 6,144 for more.  Both
+// give the same bits.  Measured, few against tile, us (called from Python, 9 us at least): 1,024 x 1,024 with 24 rows 10.6 / 14.4,
+// 48 rows (6,144) 16.0 / 17.9, 64 rows (8,192) 20.9 / 18.2; 2,048 x 1,024 with 24 rows (6,144) 15.8 / 17.0, 32 rows 20.7 / 17.7;
+// 4,096 x 1,024 with 12 rows (two passes, 8,192) 16.3 / 20.1, 16 rows 19.5 / 20.3, 24 rows 27.9 / 20.7; 1,024 x 4,096 with
+// 48 rows (6,144) 59.1 / 65.7, 64 rows 77.8 / 63.5; gated, 4,096 x 1,024, 8 rows 19.2 / 21.9, 12 rows 29.5 / 22.0, 1,024 x 1,024,
+// 16 rows 11.2 / 16.6, 24 rows (6,144) 16.3 / 16.0, 32 rows 21.4 / 16.3.
+constexpr long kFewTwoPasses = 8192, kFewMorePasses = 6144;
 
 enum GemmMode : int {
     kStore = 0,        // out = acc
@@ -64,7 +67,7 @@ static void launch_mode(const void* A, int lda, const void* W, const void* W2, v
                         const Ending& e, int w_fixed, cudaStream_t stream, int batch, long batch_a, long batch_w, long batch_o) {
     constexpr bool kDual = MODE == kSwiGLU;
     const long passes = (M + kFewRows - 1) / kFewRows;
-    const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= kFewPasses;
+    const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= (passes == 2 ? kFewTwoPasses : kFewMorePasses);
     const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats, rows = few ? kFewRows : kTileRows;
     const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, true> : gemm_nt_kernel<TA, TW, TO, MODE, false>;
     launch_chained(kernel, dim3((N + feats - 1) / feats, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads),
