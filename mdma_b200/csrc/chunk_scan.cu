@@ -500,12 +500,15 @@ static int run_chunk_scan(ChunkScan p, int n_seqs, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(chunk_sums_kernel<T, MAMBA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sums_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(chunk_out_kernel<T, MAMBA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out_smem);
     if (e != cudaSuccess) return fail("chunk_scan: cannot reserve shared memory: %s", cudaGetErrorString(e));
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // Mamba-2: up to eight heads of a group a block, as long as the blocks are three quarters of what the device holds of
     // them at once (two an SM)
     p.heads_per_block = 1;
     if (MAMBA)
         while (p.heads_per_block < kScanMostHeads && (p.heads / p.groups) % (2 * p.heads_per_block) == 0 &&
-               slots * (p.heads / (2 * p.heads_per_block)) * parts >= 220) p.heads_per_block *= 2;
+               2 * slots * (p.heads / (2 * p.heads_per_block)) * parts >= 3l * sms) p.heads_per_block *= 2;
     dim3 grid((unsigned)slots, p.heads / p.heads_per_block, parts);
     // Linear attention: a block takes all parts of v, so that q, k and their products are made once, unless that leaves more of
     // the last round of blocks empty (costs of a block of one part in the same units, by count of instructions)
@@ -515,9 +518,6 @@ static int run_chunk_scan(ChunkScan p, int n_seqs, cudaStream_t stream) {
         return rounds(blocks) * (shared + each * parts) <= rounds(blocks * parts) * (shared + each);
     };
     auto set_parts = [&](bool all_of_them) { p.heads_per_block = all_of_them ? parts : 1; grid = dim3((unsigned)slots, p.heads, all_of_them ? 1 : parts); };
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (!MAMBA) set_parts(whole(3l * sms, 0.8, 2.6));
     launch_chained(chunk_sums_kernel<T, MAMBA>, grid, dim3(kScanThreads), sums_smem, stream, p);
     const size_t all = (size_t)p.heads * p.vdim * p.n;
