@@ -10,13 +10,15 @@
 namespace mdma {
 
 // The blocks that stream W are the faster ones for up to 8 rows, and beyond as long as (rows of the matrices) x (passes of 8
-// rows of A) is small, since every pass reads W again (from the second-level cache): 8,192 for two passes, 6,144 for more.  Both
-// give the same bits.  Measured, few against tile, us (called from Python, 9 us at least): 1,024 x 1,024 with 24 rows 10.6 / 14.4,
-// 48 rows (6,144) 16.0 / 17.9, 64 rows (8,192) 20.9 / 18.2; 2,048 x 1,024 with 24 rows (6,144) 15.8 / 17.0, 32 rows 20.7 / 17.7;
-// 4,096 x 1,024 with 12 rows (two passes, 8,192) 16.3 / 20.1, 16 rows 19.5 / 20.3, 24 rows 27.9 / 20.7; 1,024 x 4,096 with
-// 48 rows (6,144) 59.1 / 65.7, 64 rows 77.8 / 63.5; gated, 4,096 x 1,024, 8 rows 19.2 / 21.9, 12 rows 29.5 / 22.0, 1,024 x 1,024,
-// 16 rows 11.2 / 16.6, 24 rows (6,144) 16.3 / 16.0, 32 rows 21.4 / 16.3.
-constexpr long kFewTwoPasses = 8192, kFewMorePasses = 6144;
+// rows of A) is small, since every pass reads W again (from the second-level cache).  Up to K = 512, where a block takes 16 rows
+// of the matrices: 9,216, nearly what four blocks an SM hold; beyond, with 8 rows a block: 8,192 for two passes, 6,144 for
+// more (a second round of blocks, which costs less than a second row of tiles).  Both give the same bits.  Measured in a
+// graph, few against tile, us: K 512, 1,024 rows of the matrix x 64 rows of A (8,192) 8.8 / 10.3, 1,536 x 48 (9,216) 9.1 / 11.1,
+// 1,024 x 80 (10,240) 12.4 / 11.1; K 768, 1,536 x 24 (4,608) 10.2 / 10.8, x 32 (6,144) 14.8 / 11.0, x 40 (7,680) 19.0 / 15.7;
+// K 1,024, 1,024 x 32 (4,096) 10.3 / 13.9, x 48 (6,144) 15.2 / 18.4, x 56 (7,168) 18.4 / 18.4, x 64 (8,192) 20.0 / 18.0,
+// 2,048 x 24 (6,144) 15.2 / 17.9, x 32 20.0 / 17.7, 4,096 x 16 (two passes, 8,192) 19.0 / 20.3; K 4,096, 1,024 x 48 58.3 / 65.0,
+// x 64 77.0 / 62.3; gated, K 1,024, 1,024 x 24 (6,144) 15.8 / 17.2, x 32 20.7 / 17.8, 2,048 x 16 (two passes, 8,192) 19.7 / 20.3.
+inline long few_rows_limit(int K, long passes) { return few_rows_chunk(K) == 32 ? 9216 : passes == 2 ? 8192 : 6144; }
 
 enum GemmMode : int {
     kStore = 0,        // out = acc
@@ -67,7 +69,7 @@ static void launch_mode(const void* A, int lda, const void* W, const void* W2, v
                         const Ending& e, int w_fixed, cudaStream_t stream, int batch, long batch_a, long batch_w, long batch_o) {
     constexpr bool kDual = MODE == kSwiGLU;
     const long passes = (M + kFewRows - 1) / kFewRows;
-    const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= (passes == 2 ? kFewTwoPasses : kFewMorePasses);
+    const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= few_rows_limit(K, passes);
     const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats, rows = few ? kFewRows : kTileRows;
     const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, true> : gemm_nt_kernel<TA, TW, TO, MODE, false>;
     launch_chained(kernel, dim3((N + feats - 1) / feats, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads),
