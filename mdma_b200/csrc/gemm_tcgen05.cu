@@ -371,7 +371,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     auto acc_empty = [&](int b) { return bar0 + 8u * (2 * kStages + 2 + b); };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * kStages + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * kStages + 5);
-    const uint32_t ep_bar = bar0 + 8u * (2 * kStages + 6);      // this block's eight epilogue warps meet here (bounded)
+    const uint32_t ep_bar = bar0 + 8u * (2 * kStages + 6);      // this block's epilogue warps meet here (bounded)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)ptx::cluster_rank();
@@ -580,7 +580,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             }
             release();
             if (sg.kind == kSegHead || sg.kind == kSegTail) {
-                // the eight epilogue warps of this block: all partial rows written (read) before the flag moves
+                // the epilogue warps of this block: all partial rows written (read) before the flag moves
                 // (an mbarrier, not bar.sync: a warp that gave up elsewhere must not leave the others waiting for ever)
                 __threadfence();
                 ptx::mbar_arrive(ep_bar);
@@ -773,9 +773,12 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     // Token tiles of one width, a multiple of 32 up to 256 (what one MMA of a pair takes): the tokens divided evenly over the
     // fewest tiles (320 tokens: two tiles of 160, not one of 256 and one that is three quarters empty).  Gated products may
     // take a few more tiles of 224 or 192 where that makes the rounds of tiles cheaper, a round costing its K blocks (0.72 us
-    // for 256 tokens) and 3.4 us of epilogue that lies open.  Measured, 256 against that: 2,385 x 2 x 8,192, K 2,048 130 / 122 us,
-    // 1,800 x 2 x 5,504 80 / 66, K 4,096, 1,000 x 2 x 14,336 205 / 191.  Narrower tiles (160: 2,048 x 2 x 14,336, K 4,096 335 / 347),
-    // and any for one matrix (2,385 x 2,048, K 8,192 71 / 88; 2,048 x 14,336, K 4,096 167 / 240), lose more to the operands' reads.
+    // for 256 tokens) and 3.4 us of epilogue that lies open.  (Whether the wide tiles' last round would be split, below, is
+    // not asked: the narrower tiles beat that too.)  Measured in turn, eight launches after a pause, 256 whole / 256 split /
+    // what is taken: 2,385 x 2 x 8,192, K 2,048 145 / 161 / 133 us (224), 1,800 x 2 x 5,504 90 / 108 / 73 (192), K 4,096,
+    // 1,000 x 2 x 14,336 199 / 193 / 187 (224), 820 x 2 x 14,336 178 / 175 / 161 (192), 1,000 x 2 x 11,008 151 / 159 / 143 (224).
+    // Narrower tiles (160: 2,048 x 2 x 14,336, K 4,096 335 / 347), and any for one matrix (2,385 x 2,048, K 8,192 71 / 88;
+    // 2,048 x 14,336, K 4,096 167 / 240), lose more to the operands' reads.
     const long f_tiles = (p.n_features + 255) / 256, most_pairs = sm_count / 2;
     int t_tiles = (p.n_tokens + 255) / 256;
     if (MODE == kTcSwiGLU) {
@@ -803,10 +806,10 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     cfg.numAttrs = 1;
     // The even split of K blocks saves the empty part of the last round and costs about 25 us (partial tiles through
     // global memory, and pairs that no longer share operands): it pays from about 56 K blocks of saved work per pair on.
-    // Measured, split against whole tiles: gated, 3,000 x 14,336, K 4,096 (9.08 rounds) 520 against 558 us, 1,000 tokens
-    // (3.03 rounds) 190 against 194, 2,048 (6.05 rounds) 344 against 343, 700 (2.27 rounds) 154 against 144; K 2,048, 2,385 x
-    // 8,192 (4.32 rounds) 150 against 131; accumulated, 2,385 x 2,048 (1.08 rounds) with K 8,192 89 against 112 us, with K
-    // 2,048 43 against 40.
+    // Measured, split against whole tiles: gated, K 4,096, 1,000 x 14,336 as 256-wide tiles (3.03 rounds) 193 against 199 us,
+    // 2,048 (6.05 rounds) 347 against 349, 3,000 (9.08 rounds) 502 against 500, 700 (2.27 rounds) 155 against 151; K 2,048,
+    // 2,385 x 8,192 (4.32 rounds) 161 against 145; accumulated, 2,385 x 2,048 (1.08 rounds) with K 8,192 89 against 112 us,
+    // with K 2,048 43 against 40.
     // A pair that finishes a shared tile waits for the pair before it (a lower block index, so it has
     // been started no later), with a limit.  The split is only used when the device can hold all pairs
     // at once (asked once); the launch is an ordinary cluster launch, which profilers take.

@@ -270,8 +270,9 @@ def attention_splits(n_seqs: int, max_new: int, max_len: int, n_heads: int, n_kv
     group = n_heads // n_kv_heads
     key_blocks = max(1, -(-max_len // 64))
     if max_new == 1 and group <= 16:
-        # decode kernel: a block's warps each take 32-key tiles in turn.  One block of eight warps per
-        # (sequence, kv head) and no merge kernel, unless that leaves most of the device idle:
+        # decode kernel: a block's warps each take 32-key tiles in turn (64-key tiles of narrow heads).  One block of
+        # twelve warps per (sequence, kv head) and no merge kernel, unless that leaves most of the device idle (the figures
+        # here are of blocks of eight warps):
         #  - an engine for a handful of sequences (their blocks x 4 within three quarters of the SMs): four blocks per
         #    (sequence, kv head), six for long contexts; a round of tiles costs a block about 1.3 us and a
         #    merge kernel about as much (measured in the layer chain at the 8B shape, context 580: batch 1

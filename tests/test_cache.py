@@ -201,3 +201,39 @@ def test_a_refused_truncate_leaves_every_group_as_it_was():
     for g in c.groups:
         assert g.table_host[a, 30 // 4] == g.seq_pages[a][30 // 4]
         assert g.table_host[a, 30 // 4] not in g.seq_pages[b].values()
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_the_uploaded_table_names_every_page_a_step_reads_or_writes(seed):
+    """Random steps of single tokens and portions, rewinds and reuse: pages are looked at only where a sequence leaves its last
+    one, and several rows of the table go up as one piece; what a kernel reads of it must be right after every step."""
+    rng = random.Random(seed)
+    needs = [KVNeed(2, 16, 0), KVNeed(1, 8, 10), KVNeed(1, 8, 0, chunk=12), KVNeed(1, 8, 9, keep_first=3)]
+    c = SequenceCache(needs, [None] * 4, 4 * 60, 5, 70, torch.float32, "cpu", page_size=4)
+    live, steps = [], 0
+    for _ in range(600):
+        what = rng.random()
+        if live and what < 0.1:
+            c.release(live.pop(rng.randrange(len(live))))
+        elif len(live) < 5 and what < 0.25:
+            live.append(c.acquire())
+        elif live and what < 0.35:
+            try:
+                c.truncate(rng.choice(live), rng.randint(0, 70))
+            except ValueError:
+                pass
+        elif live:
+            ext = {s: rng.choice([1, 1, 1, rng.randint(1, 20)]) for s in rng.sample(live, rng.randint(1, len(live)))}
+            if c.can_extend(ext) is not None:
+                continue
+            start = {s: c.length(s) for s in ext}
+            c.extend(ext, checked=rng.random() < 0.5)
+            for g in c.groups:
+                for s, n in ext.items():
+                    reads = set(range(g.need.first_key(start[s]), start[s] + n)) | set(range(min(g.need.keep_first, start[s] + n)))
+                    for p in {pos // 4 for pos in reads}:
+                        assert g.table_dev[s, p] == g.seq_pages[s][p]
+            c.commit(ext)
+            steps += 1
+        c.check()
+    assert steps > 150

@@ -306,7 +306,7 @@ class StepMeta:
 @pytest.mark.parametrize("poison", [False, True])
 def test_attention_tensor(H, K, hd, window, case, poison):
     """The tensor-core attention against the float64 statement of the reference's loop:
-    whole prompts, prompts on top of a cached prefix, single tokens (one block of eight warps; keys
+    whole prompts, prompts on top of a cached prefix, single tokens (one block of twelve warps; keys
     split over blocks, by hand and by the kernel's own choice for a long context; so many sequences
     that blocks of four, three and two warps and of one warp are taken; pages that the tile loads cannot use), with and
     without NaN in every cache row that belongs to nobody."""
