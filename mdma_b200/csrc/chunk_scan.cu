@@ -16,8 +16,8 @@
 // take several heads each: C B^T is the same for all heads of a group and stays in registers.
 //
 // Measured against the runs of 128 (256) rows that walk their chunks one after another: linear attention, 1,500 rows, 16
-// heads of 128 x 128, 209 -> 147 us (801 rows 112 -> 92); Mamba-2, 2,048 rows, 64 heads of 128 x 64, 560 -> 235 us (801 rows
-// 366 -> 100).  Of that chunk_out takes 95 (62) us, about half of the multiply-adds' rate: two blocks an SM are what the
+// heads of 128 x 128, 209 -> 147 us (801 rows 112 -> 92); Mamba-2, 2,048 rows, 64 heads of 128 x 64, 560 -> 235 us (250 in
+// a chain of calls; 801 rows 366 -> 100).  Of that chunk_out takes 95 (62) us, about half of the multiply-adds' rate: two blocks an SM are what the
 // registers and the shared memory allow.
 //
 // States between the launches: `states` [sequence * max_chunks + chunk][head][v][n], and for Mamba-2 every chunk's whole
@@ -334,8 +334,8 @@ __device__ __forceinline__ void scan_dots_state(float (&acc)[4][4], const float*
 }
 
 // Block = (chunk, heads_per_block heads, 64 columns of v).  Warp w owns rows 8 w .. 8 w + 7, so it needs the columns of
-// q k^T and the rows of u up to 8 w + 7 only (a thread's rows take none beyond their own); a thread owns four neighbouring rows, of q k^T the columns tx, tx + 16, ..,
-// of the result the columns 4 tx .. 4 tx + 3.
+// q k^T and the rows of u up to 8 w + 7 only (a thread's rows take none beyond their own); a thread owns four neighbouring
+// rows, of q k^T the columns tx, tx + 16, .., of the result the columns 4 tx .. 4 tx + 3.
 template <typename T, bool MAMBA>
 __global__ void __launch_bounds__(kScanThreads, 2)
 chunk_out_kernel(const ChunkScan p) {
