@@ -840,3 +840,34 @@ def test_random_configurations(seed):
             check(out, [(refs[0], 67 + j), (refs[2], 282 + j)], dtype, f"seed {seed} {dtype}: decoded {j}")
         eng.cache.check()
         eng.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths", [[5, 40, 40, 1, 0, 17], [3 + i % 7 for i in range(33)]])
+def test_delta_chunks_of_a_sequence_are_the_same_among_others(lengths):
+    """Sequences are walked longest first (beyond 32 as they stand): each gives the bits that it gives alone."""
+    from mdma_b200 import ops
+    H, D, V, taps = 2, 32, 48, 4
+    ch = 2 * H * D + H * V
+    g = torch.Generator(device="cuda").manual_seed(len(lengths))
+    draw = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    conv, a_log, dt = (0.5 * draw(ch, taps)).bfloat16(), (draw(H) - 1).bfloat16(), (draw(H * D) - 1).bfloat16()
+    n = len(lengths)
+    proj, raw = draw(sum(lengths), ch + H), draw(sum(lengths), H * D)
+    first = draw(n, H * D * V + (taps - 1) * ch)                 # the state, then the convolutions' kept inputs
+
+    def run(which, slots):
+        rows = torch.cat([torch.arange(sum(lengths[:s]), sum(lengths[:s + 1])) for s in which]).cuda()
+        ctx = _Step([lengths[s] for s in which], [0] * len(which), slots)
+        state, out = first.clone(), torch.zeros(len(rows), H * V, device="cuda")
+        scratch = torch.empty((len(rows) // 16 + len(which) + 1) * ops.delta_chunk_floats(H, D, V), device="cuda")
+        ops.delta_chunks(proj[rows].contiguous(), raw[rows].contiguous(), conv, taps, a_log, dt, state[:, H * D * V:], scratch, ctx, state[:, :H * D * V],
+                         out, H, H, D, V, 1e-6, D ** -0.5)
+        return out, state
+    together, state = run(list(range(n)), list(range(n)))
+    at = 0
+    for s in range(n):
+        if lengths[s]:
+            alone, one = run([s], [s])
+            assert torch.equal(alone, together[at:at + lengths[s]]) and torch.equal(one[s], state[s])
+        at += lengths[s]
