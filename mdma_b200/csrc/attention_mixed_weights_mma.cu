@@ -116,13 +116,23 @@ mixed_rows_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const _
         if (r < rows) v = *reinterpret_cast<const uint4*>(q + (size_t)(t0 + r0 + r) * q_row_stride + (size_t)h * dim + d8 * 8);
         *reinterpret_cast<uint4*>(sq + (size_t)r * qp + d8 * 8) = v;
     }
+    // The cache rows of a chunk's keys, a lane a key, looked up a chunk ahead of their copies: key by key, a warp waits for each
+    // word of the page table before it asks for the next key (four prompts of 100 to 801 rows, 16 heads of 128: 88 us, 110 so).
+    static_assert(kMwChunk == 32, "a lane a key");
+    auto rows_of = [&](int e0) -> int {
+        const int e = e0 + lane;
+        return e < n_keys ? (int)cache.row(e < kept ? e : e + gap) : 0;
+    };
+    int key_rows = rows_of(0);
     auto issue = [&](int e0, int buf) {
+        const int now = key_rows;
+        key_rows = rows_of(e0 + kMwChunk);
         for (int j = warp; j < kMwChunk; j += kMwWarps) {
             __nv_bfloat16* dk = sk + ((size_t)buf * kMwChunk + j) * qp;
             __nv_bfloat16* dv = sv + ((size_t)buf * kMwChunk + j) * vp;
             const int e = e0 + j;
+            const size_t row = __shfl_sync(0xffffffffu, now, j);
             if (e < n_keys) {
-                const size_t row = cache.row(e < kept ? e : e + gap);
                 const __nv_bfloat16* gk = k_cache + (row * n_kv_heads + kvh) * dim;
                 const __nv_bfloat16* gv = v_cache + row * total + c0;
                 for (int d8 = lane; d8 < dim / 8; d8 += 32) mw_copy16(dk + d8 * 8, gk + d8 * 8);
@@ -323,14 +333,21 @@ mixed_step_kernel(const __nv_bfloat16* __restrict__ q, int q_row_stride, const _
     float* scorr = sl + kMwMaxHeads;
     const int* pages = page_table + (size_t)seq_slot[s] * max_pages;
     const uint4 zero4 = make_uint4(0, 0, 0, 0);
+    // (the keys' rows a lane a key and a chunk ahead, as in mixed_rows_kernel)
+    auto rows_of = [&](int chunk) -> int {
+        const int e = chunk * kMwChunk + lane, p = e < kept ? e : e + gap;
+        return e < n_keys ? pages[p / page_size] * page_size + p % page_size : 0;
+    };
+    int key_rows = rows_of(chunk0);
     auto issue = [&](int chunk, int buf) {
+        const int now = key_rows;
+        key_rows = rows_of(chunk + 1);
         for (int j = warp; j < kMwChunk; j += kMwStepWarps) {
             __nv_bfloat16* dk = sk + ((size_t)buf * kMwChunk + j) * kp;
             __nv_bfloat16* dv = sv + ((size_t)buf * kMwChunk + j) * vp;
             const int e = chunk * kMwChunk + j;
+            const size_t row = __shfl_sync(0xffffffffu, now, j);
             if (e < n_keys) {
-                const int p = e < kept ? e : e + gap;
-                const size_t row = (size_t)pages[p / page_size] * page_size + (size_t)(p % page_size);
                 for (int d8 = lane; d8 < kw / 8; d8 += 32) mw_copy16(dk + d8 * 8, k_cache + row * kw + d8 * 8);
                 for (int d8 = lane; d8 < total / 8; d8 += 32) mw_copy16(dv + d8 * 8, v_cache + row * total + d8 * 8);
             } else {

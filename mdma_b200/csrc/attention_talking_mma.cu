@@ -127,14 +127,23 @@ talking_attention_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfl
     const int n_chunks = (last + 1 - first + kTmChunk - 1) / kTmChunk, per_split = (n_chunks + splits - 1) / splits;
     const int c_begin = first + split * per_split * kTmChunk;
     const int c_end = min(last, first + (split + 1) * per_split * kTmChunk - 1);
+    // The cache rows of a chunk's keys, a lane a key, looked up a chunk ahead of their copies: key by key, a warp waits for each
+    // word of the page table before it asks for the next key (8 sequences of 600, 16 heads of 128 over 4: 34 us, 43 so).
+    static_assert(kTmChunk == 32, "a lane a key");
+    auto rows_of = [&](int c0) -> int {
+        const int p = c0 + lane;
+        return p <= last ? pages[p / page_size] * page_size + p % page_size : 0;
+    };
+    int ahead = rows_of(c_begin);
     for (int c0 = c_begin; c0 <= c_end; c0 += kTmChunk) {
-        const int n_keys = min(kTmChunk, last + 1 - c0);
+        const int n_keys = min(kTmChunk, last + 1 - c0), key_rows = ahead;
+        ahead = rows_of(c0 + kTmChunk);
         __syncthreads();                                   // every warp is done with the chunk before
         for (int j = warp; j < kTmChunk; j += warps) {
             __nv_bfloat16* dst = sk + (size_t)j * qp;
+            const size_t row = __shfl_sync(0xffffffffu, key_rows, j);
             if (j < n_keys) {
-                const int p = c0 + j;
-                const __nv_bfloat16* src = k_cache + ((size_t)pages[p / page_size] * page_size + (size_t)(p % page_size)) * kd;
+                const __nv_bfloat16* src = k_cache + row * kd;
                 for (int d8 = lane; d8 < k_cols; d8 += 32) tm_copy16(dst + d8 * 8, src + d8 * 8);
             } else {
                 for (int d8 = lane; d8 < k_cols; d8 += 32) *reinterpret_cast<uint4*>(dst + d8 * 8) = zero4;
@@ -144,9 +153,9 @@ talking_attention_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfl
             // value rows: the block's warps share the work when they share the kv head, else every warp its own
             for (int j = shared_v ? warp : 0; j < kTmChunk; j += shared_v ? warps : 1) {
                 __nv_bfloat16* dst = sv + (size_t)j * vp;
+                const size_t row = __shfl_sync(0xffffffffu, key_rows, j);
                 if (j < n_keys) {
-                    const int p = c0 + j;
-                    const __nv_bfloat16* src = v_cache + (((size_t)pages[p / page_size] * page_size + (size_t)(p % page_size)) * n_kv_heads + kvh) * v_dim;
+                    const __nv_bfloat16* src = v_cache + (row * n_kv_heads + kvh) * v_dim;
                     for (int d8 = lane; d8 < v_cols; d8 += 32) tm_copy16(dst + d8 * 8, src + d8 * 8);
                 } else {
                     for (int d8 = lane; d8 < v_cols; d8 += 32) *reinterpret_cast<uint4*>(dst + d8 * 8) = zero4;
