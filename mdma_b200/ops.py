@@ -771,15 +771,17 @@ def group_rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, groups: int, out
 
 
 def group_rmsnorm_add(x: torch.Tensor, y: torch.Tensor, w: torch.Tensor, eps: float, groups: int, n_rows: int,
-                      partial: Optional[torch.Tensor] = None, splits: int = 0, split_stride: int = 0) -> None:
+                      partial: Optional[torch.Tensor] = None, splits: int = 0, split_stride: int = 0,
+                      only_partial: bool = False) -> None:
     """x[t] += group norm of y[t] times w; x and y float rows.  With `partial` [splits, rows, width], y is first
-    completed by those sums (a K-split product not yet added up)."""
+    completed by those sums (a K-split product not yet added up), or becomes their sum (`only_partial`)."""
     _need_cuda(x, y, w, partial)
     width = x.shape[1]
     assert x.dtype == y.dtype == torch.float32 and x.is_contiguous() and y.is_contiguous() and y.shape[1] == width
     assert w.numel() == width and w.is_contiguous()
     _call("core", "mdma_group_rmsnorm_add", _ptr(x), _ptr(y), _ptr(partial), _i(splits if partial is not None else 0),
-          ctypes.c_long(split_stride), _ptr(w), _i(dtype_code(w.dtype)), _i(n_rows), _i(width), _i(groups), _f(eps), _stream())
+          ctypes.c_long(split_stride), _i(int(only_partial)), _ptr(w), _i(dtype_code(w.dtype)), _i(n_rows), _i(width), _i(groups),
+          _f(eps), _stream())
 
 
 def depth_mix(x: torch.Tensor, x0: torch.Tensor, history: torch.Tensor, depth: int, run: int, w: torch.Tensor,

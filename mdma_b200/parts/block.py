@@ -179,7 +179,7 @@ class SandwichBlock:
 
     The two norms on the results come from `LayerSpec.extras`: "mixer_post_norm" and "ffn_post_norm"; they must offer
     `add_normed(ctx, y, x)` (x += norm(y) over float rows).  A sublayer that offers `produce` stores its result where the
-    norm takes stored results (`adds_stored`), any other adds it into a zeroed float buffer through its ordinary `forward`."""
+    norm takes stored results (`adds_stored` or `completes_stored`), any other adds it into a zeroed float buffer through its ordinary `forward`."""
 
     def __init__(self, spec: LayerSpec):
         self.spec = spec
@@ -215,7 +215,7 @@ class SandwichBlock:
 
     @staticmethod
     def _sublayer(ctx, part, norm, h, x, y, *more):
-        if hasattr(part, "produce") and getattr(norm, "adds_stored", False):
+        if hasattr(part, "produce") and (getattr(norm, "adds_stored", False) or getattr(norm, "completes_stored", False)):
             part.produce(ctx, h, y, *more, defer=True)
             norm.add_normed(ctx, y, x, stored=True)
         else:

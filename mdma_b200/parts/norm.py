@@ -30,8 +30,9 @@ class RMSNorm(Part):
             raise ValueError(f"a row of {self.width} numbers does not split into {self.groups} equal parts")
         if self.groups > 1:
             self.fuses_pending = False      # the grouped kernel reads complete rows of x
-        # `add_normed(.., stored=True)` completes a stored product's partial sums itself (the grouped kernel: an added one's only)
-        self.adds_stored = self.groups == 1
+        # `add_normed(.., stored=True)` completes a stored product's partial sums itself; of the two, only the plain norm
+        # leaves a copy of the stream
+        self.adds_stored, self.completes_stored = self.groups == 1, True
 
     def tensor_specs(self):
         return {"weight": TensorSpec((self.width,), "vector")}
@@ -68,7 +69,7 @@ class RMSNorm(Part):
         if self.rt.gemm == "tensor":
             from .. import ops_tensor
             mode = ops.GEMM_STORE if stored else ops.GEMM_ACCUMULATE
-            pend = ops_tensor.take_pending(y, mode, ctx.n_tokens, self.rt.tc) if not (stored and self.groups > 1) else None
+            pend = ops_tensor.take_pending(y, mode, ctx.n_tokens, self.rt.tc)
             if pend is not None:
                 partial, splits, stride = pend
                 only = stored
@@ -77,7 +78,7 @@ class RMSNorm(Part):
         if self.groups > 1:
             if copy is not None:
                 raise ValueError("the norm in groups leaves no copy of the stream")
-            ops.group_rmsnorm_add(x, y, self.weight, self.eps, self.groups, ctx.n_tokens, partial, splits, stride)
+            ops.group_rmsnorm_add(x, y, self.weight, self.eps, self.groups, ctx.n_tokens, partial, splits, stride, only)
             return
         ops.rmsnorm_add(x, y, self.weight, self.eps, ctx.n_tokens, partial, splits, stride, only, copy)
 
