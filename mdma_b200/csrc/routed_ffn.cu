@@ -84,8 +84,12 @@ __device__ __forceinline__ int warp_largest(const float* v, int n, int lane) {
 }
 
 // ---------------------------------------------------------------- router
+constexpr int kRouteWarps = 32;
+
+// A block a token; a warp an output, as long as there are no more than kRouteWarps (and one for the shared gate): the sums side
+// by side are one round trip (4 tokens, 16 outputs and a gate of 1,024 floats 8 us, 11 with eight warps).
 template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kRouteWarps * 32)
 route_kernel(const TA* __restrict__ h, int h_stride, const TW* __restrict__ router, const TC* __restrict__ correction,
              const TW* __restrict__ shared_gate, int width, int n_routed, int top, int n_groups, int keep_groups,
              int scoring, int group_top, int renormalize, int logit_bias, float weight_scale,
@@ -106,13 +110,12 @@ route_kernel(const TA* __restrict__ h, int h_stride, const TW* __restrict__ rout
     const TA* row = h + (size_t)t * h_stride;
     const bool vec_row = width % 8 == 0 && ((uintptr_t)row & 15) == 0;
     const bool vec = vec_row && ((uintptr_t)router & 15) == 0, vec_gate = vec_row && ((uintptr_t)shared_gate & 15) == 0;
-    for (int e = warp; e < n_routed; e += n_warps) {
-        const float v = warp_dot(row, router + (size_t)e * width, width, lane, vec);
-        if (lane == 0) z[e] = v + (logit_bias ? to_float(correction[e]) : 0.f);
-    }
-    if (shared_gate != nullptr && warp == n_warps - 1) {
-        const float v = warp_dot(row, shared_gate, width, lane, vec_gate);
-        if (lane == 0) shared_scale[t] = 1.0f / (1.0f + expf(-v));
+    for (int e = warp; e < n_routed + (shared_gate != nullptr); e += n_warps) {
+        const bool gate = e == n_routed;
+        const float v = warp_dot(row, gate ? shared_gate : router + (size_t)e * width, width, lane, gate ? vec_gate : vec);
+        if (lane != 0) continue;
+        if (gate) shared_scale[t] = 1.0f / (1.0f + expf(-v));
+        else z[e] = v + (logit_bias ? to_float(correction[e]) : 0.f);
     }
     __syncthreads();
     // the rest is a few hundred operations of one warp: exponentials, group scores and the search for a largest score side
@@ -478,9 +481,11 @@ int mdma_route(const void* h, int h_dtype, int h_stride, const void* router, int
                  "route: %d groups (keep %d) over %d outputs", n_groups, keep_groups, n_routed);
     MDMA_REQUIRE(shared_gate == nullptr || shared_scale != nullptr, "route: the shared gate needs a place for its result");
     if (n_tokens == 0) return 0;
+    int warps = n_routed + (shared_gate != nullptr);
+    warps = warps < 8 ? 8 : warps > kRouteWarps ? kRouteWarps : warps;
     MDMA_DISPATCH_2(h_dtype, TA, w_dtype, TW,
         MDMA_DISPATCH_DTYPE(c_dtype, TC,
-            launch_chained(route_kernel<TA, TW, TC>, dim3(n_tokens), dim3(256), 0, stream, (const TA*)h, h_stride,
+            launch_chained(route_kernel<TA, TW, TC>, dim3(n_tokens), dim3(warps * 32), 0, stream, (const TA*)h, h_stride,
                            (const TW*)router, (const TC*)correction, (const TW*)shared_gate, width, n_routed, top,
                            n_groups, keep_groups, scoring, group_top, renormalize, logit_bias, weight_scale, chosen, weights, shared_scale)));
     MDMA_LAUNCH_OK("route");
