@@ -285,7 +285,7 @@ constexpr int kScanTerms = 16;
 template <int NJ>
 __device__ __forceinline__ void scan_dots(float (&acc)[4][4], const float* a, int pa, const float* b, int pb, int len) {
     for (int d0 = 0; d0 < len; d0 += kScanTerms) {
-        float part[4][NJ] = {};
+        float2 part[4][NJ] = {};
         const int stop = min(len, d0 + kScanTerms);
 #pragma unroll 2
         for (int d = d0; d < stop; d += 4) {
@@ -297,12 +297,12 @@ __device__ __forceinline__ void scan_dots(float (&acc)[4][4], const float* a, in
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < NJ; ++j) part[i][j] = dot4(x[i], y[j], part[i][j]);
+                for (int j = 0; j < NJ; ++j) dot4(part[i][j], x[i], y[j]);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) acc[i][j] += part[i][j];
+            for (int j = 0; j < NJ; ++j) acc[i][j] += part[i][j].x + part[i][j].y;
     }
 }
 // acc[i][j] += sum_d a[row i][d] b[4 tx + j][d], b's rows of 128 numbers with their quads permuted (`scan_state_quad`)
@@ -311,7 +311,7 @@ __device__ __forceinline__ void scan_dots_state(float (&acc)[4][4], const float*
     const float* bt = b + 4 * tx * kScanMostN;
     const int turn = tx & 7;
     for (int d0 = 0; d0 < len; d0 += kScanTerms) {
-        float part[4][4] = {};
+        float2 part[4][4] = {};
         const int stop = min(len, d0 + kScanTerms);
 #pragma unroll 2
         for (int d = d0; d < stop; d += 4) {
@@ -324,12 +324,12 @@ __device__ __forceinline__ void scan_dots_state(float (&acc)[4][4], const float*
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) part[i][j] = dot4(x[i], y[j], part[i][j]);
+                for (int j = 0; j < 4; ++j) dot4(part[i][j], x[i], y[j]);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
+            for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j].x + part[i][j].y;
     }
 }
 
