@@ -47,7 +47,8 @@ kv_store_kernel(const T* __restrict__ proj, int proj_stride, int k_col, int v_co
 }
 
 // ---------------------------------------------------------------- plain kernel
-template <typename T, typename TO>
+// PER: numbers of a key (a value) a lane has: dimensions up to 32 * PER
+template <typename T, typename TO, int PER>
 __global__ void __launch_bounds__(128)
 attention_distance_plain_kernel(const T* __restrict__ q, int q_row_stride, const T* __restrict__ k_cache,
                                 const T* __restrict__ v_cache, const int* __restrict__ tok_seq,
@@ -70,59 +71,89 @@ attention_distance_plain_kernel(const T* __restrict__ q, int q_row_stride, const
     const int first = rule_first(rule, pos), kept = min(rule.keep_first, first);
     const float slope = slopes ? slopes[h] : 0.f;
 
-    float qv[kMaxDim / 32], acc[kMaxDim / 32];
+    float qv[PER], acc[PER];
     const T* qp = q + (size_t)t * q_row_stride + (size_t)hm * dim;
 #pragma unroll
-    for (int j = 0; j < kMaxDim / 32; ++j) {
+    for (int j = 0; j < PER; ++j) {
         const int d = lane + 32 * j;
         qv[j] = d < dim ? to_float(qp[d]) : 0.f;
         acc[j] = 0.f;
     }
     float m = -INFINITY, l = 0.f;
     const int* pages = page_table + (size_t)slot * max_pages;
-    // Four keys' rows and scores at a time, so that a warp waits for memory and for the sum over its lanes once for four
-    // keys; the softmax then takes them one by one in order, as if they had come alone.  (Bound by that latency: 4 sequences
-    // of 60 keys, 8 heads of 128 floats, 102 us with one key at a time, 30 with four.)
+    // Four keys' rows and scores at a time, the next four's on their way, so that a warp waits for the sum over its lanes once
+    // for four keys and for memory hardly at all; the softmax then takes them one by one in order, as if they had come alone.
+    // (Bound by that latency: 4 sequences of 60 keys, 8 heads of 128 floats, 102 us with one key at a time, 29 with four and
+    // none on their way, 22 so.)
     constexpr int kKeys = 4;
-    for (int p = kept > 0 ? 0 : first; p <= pos;) {
-        float kv[kKeys][kMaxDim / 32], vv[kKeys][kMaxDim / 32], s[kKeys];
-        int n = 0;
+    struct Keys { float k[kKeys][PER], v[kKeys][PER], away[kKeys]; int n; };
+    int p = kept > 0 ? 0 : first;
+    auto fetch = [&](Keys& f) {
+        // (no branch between the lookups: one after the other they cost more than the keys being ahead saves)
+        int at[kKeys];
+        size_t row[kKeys];
+        f.n = 0;
 #pragma unroll
         for (int u = 0; u < kKeys; ++u) {
             const bool there = p <= pos;
-            const int at = there ? p : pos;
-            const size_t row = (size_t)pages[at / page_size] * page_size + (size_t)(at % page_size);
-            const T* kp = k_cache + (row * n_kv_heads * maps + key_head) * dim;
-            const T* vp = v_cache + (row * n_kv_heads + kvh) * v_dim;
+            at[u] = there ? p : pos;
+            f.n += there;
+            p = !there ? p : p + 1 == kept ? first : p + 1;
+        }
 #pragma unroll
-            for (int j = 0; j < kMaxDim / 32; ++j) {
+        for (int u = 0; u < kKeys; ++u) row[u] = (size_t)pages[at[u] / page_size] * page_size + (size_t)(at[u] % page_size);
+#pragma unroll
+        for (int u = 0; u < kKeys; ++u) {
+            const T* kp = k_cache + (row[u] * n_kv_heads * maps + key_head) * dim;
+            const T* vp = v_cache + (row[u] * n_kv_heads + kvh) * v_dim;
+            f.away[u] = slope * (float)(pos - at[u]);
+#pragma unroll
+            for (int j = 0; j < PER; ++j) {
                 const int d = lane + 32 * j;
-                kv[u][j] = there && d < dim ? to_float(kp[d]) : 0.f;
-                vv[u][j] = there && d < v_dim ? to_float(vp[d]) : 0.f;
+                f.k[u][j] = u < f.n && d < dim ? to_float(kp[d]) : 0.f;
+                f.v[u][j] = u < f.n && d < v_dim ? to_float(vp[d]) : 0.f;
             }
-            s[u] = slope * (float)(pos - at);
-            if (there) { ++n; p = p + 1 == kept ? first : p + 1; }
         }
+    };
+    auto take = [&](const Keys& f) {
+        float s[kKeys];
 #pragma unroll
         for (int u = 0; u < kKeys; ++u) {
-            float part = 0.f;
+            s[u] = 0.f;
 #pragma unroll
-            for (int j = 0; j < kMaxDim / 32; ++j) part = fmaf(qv[j], kv[u][j], part);
-            float score = warp_sum(part) * scale;
+            for (int j = 0; j < PER; ++j) s[u] = fmaf(qv[j], f.k[u][j], s[u]);
+        }
+        // (the sums over the lanes side by side)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < kKeys; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+        for (int u = 0; u < kKeys; ++u) {
+            float score = s[u] * scale;
             if (softcap > 0.f) score = softcap * tanhf(score / softcap);
-            s[u] = score - s[u];
+            s[u] = score - f.away[u];
         }
 #pragma unroll
         for (int u = 0; u < kKeys; ++u) {
-            if (u >= n) break;
+            if (u >= f.n) break;
             const float m_new = fmaxf(m, s[u]);
             const float corr = m_new == m ? 1.f : expf(m - m_new);     // exp(-inf) = 0 on the first key
             const float pe = expf(s[u] - m_new);
             l = fmaf(l, corr, pe);
 #pragma unroll
-            for (int j = 0; j < kMaxDim / 32; ++j) acc[j] = fmaf(pe, vv[u][j], acc[j] * corr);
+            for (int j = 0; j < PER; ++j) acc[j] = fmaf(pe, f.v[u][j], acc[j] * corr);
             m = m_new;
         }
+    };
+    Keys one, two;
+    fetch(one);
+    while (one.n > 0) {
+        fetch(two);
+        take(one);
+        if (two.n == 0) break;
+        fetch(one);
+        take(two);
     }
     if (sinks) {
         const float sink = sinks[h];
@@ -130,13 +161,13 @@ attention_distance_plain_kernel(const T* __restrict__ q, int q_row_stride, const
         const float corr = expf(m - m_new);
         l = l * corr + expf(sink - m_new);
 #pragma unroll
-        for (int j = 0; j < kMaxDim / 32; ++j) acc[j] *= corr;
+        for (int j = 0; j < PER; ++j) acc[j] *= corr;
     }
     TO* op = out + ((size_t)t * n_heads * maps + hm) * v_dim;
     const T* gp = gate ? gate + (size_t)t * gate_stride + (gate_heads ? (size_t)h : (size_t)h * v_dim) : nullptr;
     const float inv = out_scale / l;
 #pragma unroll
-    for (int j = 0; j < kMaxDim / 32; ++j) {
+    for (int j = 0; j < PER; ++j) {
         const int d = lane + 32 * j;
         if (d < v_dim) {
             float o = acc[j] * inv;
@@ -429,14 +460,14 @@ int mdma_attention_distance(const void* q, int dtype, int q_row_stride, const vo
         return 0;
     }
     dim3 grid(n_tokens, (n_heads * maps + 3) / 4);
-#define MDMA_PLAIN_LAUNCH(TO)                                                                                              \
-        launch_chained(attention_distance_plain_kernel<T, TO>, grid, dim3(128), 0, stream, (const T*)q, q_row_stride,      \
+#define MDMA_PLAIN_LAUNCH(TO, PER)                                                                                         \
+        launch_chained(attention_distance_plain_kernel<T, TO, PER>, grid, dim3(128), 0, stream, (const T*)q, q_row_stride,      \
                        (const T*)k_cache, (const T*)v_cache, tok_seq, tok_pos, seq_slot, page_table, max_pages, page_size, \
                        slopes, (const T*)gate, gate_stride, (TO*)out, n_heads, n_kv_heads, dim, v_dim, rule, scale,        \
                        sinks, gate_heads, out_scale, softcap, maps)
     MDMA_DISPATCH_DTYPE(dtype, T, {
-        if (out_f32) MDMA_PLAIN_LAUNCH(float);
-        else MDMA_PLAIN_LAUNCH(T);
+        if (dim <= 128 && v_dim <= 128) { if (out_f32) MDMA_PLAIN_LAUNCH(float, 4); else MDMA_PLAIN_LAUNCH(T, 4); }
+        else { if (out_f32) MDMA_PLAIN_LAUNCH(float, kMaxDim / 32); else MDMA_PLAIN_LAUNCH(T, kMaxDim / 32); }
     });
 #undef MDMA_PLAIN_LAUNCH
     MDMA_LAUNCH_OK("attention_distance");

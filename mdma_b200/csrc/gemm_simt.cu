@@ -5,6 +5,8 @@
 // shapes the tensor-core kernel refuses.  The order of additions is that of
 // rows_product.cuh: one order for every shape, so a row's result does not
 // depend on how many other rows are in the call.
+#include <type_traits>
+
 #include "rows_product.cuh"
 
 namespace mdma {
@@ -27,13 +29,14 @@ enum GemmMode : int {
     kStoreAct = 3,     // out = act(acc): a feed-forward without a gate
 };
 
-// FEW: blocks of up to 8 rows that stream W; else tiles of 32 rows.
-template <typename TA, typename TW, typename TO, int MODE, bool FEW>
+// SHAPE: blocks of up to 8 rows that stream W (kFew: a group of features each, kStream: one group after another); else tiles
+// of 32 rows.
+template <typename TA, typename TW, typename TO, int MODE, int SHAPE>
 __global__ void __launch_bounds__(kRowsThreads)
 gemm_nt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, const TW* __restrict__ W2,
                TO* __restrict__ out, int ldo, int M, int N, int K, const Ending e,
                long batch_a, long batch_w, long batch_o, int w_fixed) {
-    constexpr bool kDual = MODE == kSwiGLU;
+    constexpr bool kDual = MODE == kSwiGLU, FEW = SHAPE != kTile;
     extern __shared__ __align__(16) float smem[];
     chain_release();
     // blockIdx.z: one of several products of the same sizes (a head each), operands `batch_*` elements apart
@@ -57,7 +60,9 @@ gemm_nt_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, cons
             else if (MODE == kStoreAct) *o = from_float<TO>(gate_activation(r, e.act));
             else *o = from_float<TO>(gated_pair(r, acc2 + ending_bias(e.bias2, e.bias_dtype, n), e.act, e.act_limit, e.act_alpha));
         };
-        if (FEW) few_rows_product<TA, TW, kDual>(rows, row_of, W, W2, blockIdx.x * few_rows_features(K, kDual), N, K, vec_a, vec_w,
+        if constexpr (SHAPE == kStream)
+            few_rows_stream<TA, kDual>(rows, row_of, W, W2, blockIdx.x, gridDim.x, N, K, vec_a, smem, [] { chain_wait(); }, store);
+        else if (FEW) few_rows_product<TA, TW, kDual>(rows, row_of, W, W2, blockIdx.x * few_rows_features(K, kDual), N, K, vec_a, vec_w,
                                                  smem, [] { chain_wait(); }, store);
         else tile_product<TA, TW, kDual>(rows, row_of, W, W2, blockIdx.x * (kDual ? kTileFeats / 2 : kTileFeats), N, K, vec_a, vec_w, smem, store);
         __syncthreads();
@@ -70,11 +75,23 @@ static void launch_mode(const void* A, int lda, const void* W, const void* W2, v
     constexpr bool kDual = MODE == kSwiGLU;
     const long passes = (M + kFewRows - 1) / kFewRows;
     const bool few = passes == 1 || (long)N * (kDual ? 2 : 1) * passes <= few_rows_limit(K, passes);
-    const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats, rows = few ? kFewRows : kTileRows;
-    const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, true> : gemm_nt_kernel<TA, TW, TO, MODE, false>;
-    launch_chained(kernel, dim3((N + feats - 1) / feats, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads),
-                   rows_product_smem(kernel, few), stream, (const TA*)A, lda,
-                   (const TW*)W, (const TW*)W2, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o, w_fixed);
+    const auto launch = [&](auto kernel, int rows, int across, size_t smem) {
+        launch_chained(kernel, dim3(across, min((M + rows - 1) / rows, 65535), batch), dim3(kRowsThreads), smem, stream, (const TA*)A, lda,
+                       (const TW*)W, (const TW*)W2, (TO*)out, ldo, M, N, K, e, batch_a, batch_w, batch_o, w_fixed);
+    };
+    const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats;
+    const int groups = (N + feats - 1) / feats;
+    if constexpr (std::is_same<TW, float>::value) {
+        // from two groups a block on
+        const int most = few_rows_stream_blocks();
+        if (passes == 1 && batch == 1 && groups >= 2 * most && few_rows_streams(W, W2, K)) {
+            const auto kernel = gemm_nt_kernel<TA, TW, TO, MODE, kStream>;
+            launch(kernel, kFewRows, most, few_rows_stream_smem(kernel, M, K));
+            return;
+        }
+    }
+    const auto kernel = few ? gemm_nt_kernel<TA, TW, TO, MODE, kFew> : gemm_nt_kernel<TA, TW, TO, MODE, kTile>;
+    launch(kernel, few ? kFewRows : kTileRows, groups, rows_product_smem(kernel, few));
 }
 
 template <typename TA, typename TW, typename TO>

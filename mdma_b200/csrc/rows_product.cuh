@@ -11,6 +11,9 @@
 //                     out of shared memory; the runs' sums meet in shared memory.
 //                     Measured, 1,024 x 1,024 floats: 4 rows 3.3 us (a tile of 64 rows x 64 features walked by one block
 //                     without anything on its way took 67), 8 rows 4.5.
+//   few_rows_stream   the same for float matrices of K up to 1,024 that are larger than what the blocks hold at once: a block
+//                     walks over groups of features, the next groups' rows on their way by cp.async in two stages of shared
+//                     memory (laid out for a thread's run, while the loads are of whole lines).  Measured, 4 rows x 32,000 x 1,024: 34 us, a block a group 50.
 //   tile_product      32 rows x 32 rows of W per block of 256 threads.  Bound by the fused multiply-adds: each quarter
 //                     of K belongs to 64 threads (4 x 4 outputs each, 16 multiply-adds for two 16-byte shared-memory
 //                     reads); float rows have three runs on their way while one is computed.
@@ -20,6 +23,7 @@
 
 namespace mdma {
 
+enum RowsShape : int { kTile = 0, kFew = 1, kStream = 2 };
 constexpr int kRun = 16;                       // values of k summed from zero
 constexpr int kFewRows = 8;                    // rows of A of one few_rows_product
 constexpr int kTileRows = 32, kTileFeats = 32; // of one tile_product
@@ -136,6 +140,93 @@ __device__ __forceinline__ void few_rows_product(int rows, RowOf row_of, const T
     }
 }
 
+// ---- the same, streaming -----------------------------------------------------------------------------------------------
+constexpr int kStreamStage = 2 * kRowsThreads * kRun;     // floats of a stage: two rows' runs a thread
+constexpr int kStreamMaxK = 64 * kRun;
+// shared memory: two stages, the rows of A, the runs' sums (2 pairs x rows x (chunk + 1)), their totals
+__host__ __device__ inline int few_rows_stream_floats(int rows, int K) {
+    const int chunk = few_rows_chunk(K);
+    return 2 * kStreamStage + rows * chunk * kRun + 2 * (kRowsThreads / chunk) * (rows * (chunk + 1) + kFewRows) + 64;
+}
+// whether a product of float matrices takes this form: their rows lie on 16 bytes
+__host__ __device__ inline bool few_rows_streams(const void* W, const void* W2, int K) {
+    return K <= kStreamMaxK && K % 4 == 0 && (((uintptr_t)W | (uintptr_t)W2) & 15) == 0;
+}
+
+// As few_rows_product for the groups of features `group`, `group` + `groups`, ..; the same sums in the same order.
+template <typename TA, bool DUAL, class RowOf, class Arrived, class Store>
+__device__ __forceinline__ void few_rows_stream(int rows, RowOf row_of, const float* __restrict__ W, const float* __restrict__ W2,
+                                                int group, int groups, int N, int K, bool vec_a, float* smem, Arrived arrived, Store store) {
+    const int chunk = few_rows_chunk(K), t = threadIdx.x;
+    const int run_l = t & (chunk - 1), pair = t / chunk, pairs = kRowsThreads / chunk, feats = DUAL ? pairs : 2 * pairs;
+    const int R = (K + kRun - 1) / kRun, q = quarter_runs(K), turn = (run_l >> 1) & 3;
+    float* const rows_a = smem + 2 * kStreamStage;
+    float* const run_sums = rows_a + rows * chunk * kRun;            // [row of W][row of A][run]
+    float* const total = run_sums + 2 * pairs * rows * (chunk + 1);  // [row of W][row of A of kFewRows]
+    auto issue = [&](int f0, int stage) {
+        float* to = smem + stage * kStreamStage;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            const int i = t + x * kRowsThreads, r = i / (chunk * 4), at = i - r * chunk * 4, run = at >> 2, quad = at & 3, k = run * kRun + 4 * quad;
+            const int f = DUAL ? f0 + (r >> 1) : f0 + r;
+            const bool there = f < N && k < K;
+            const float* src = there ? (DUAL && (r & 1) ? W2 : W) + (size_t)f * K + k : W;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to + (r * chunk + run) * kRun + 4 * (quad ^ ((run >> 1) & 3)))),
+                         "l"(src), "r"(there ? 16 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int step = groups * feats;
+    issue(group * feats, 0);
+    issue(group * feats + step, 1);
+    arrived();
+    for (int i = t; i < rows * chunk * 4; i += kRowsThreads) {
+        const int m = i / (chunk * 4), at = i - m * chunk * 4, run = at >> 2, quad = at & 3;
+        st4(rows_a + (m * chunk + run) * kRun + 4 * (quad ^ ((run >> 1) & 3)), load4_of(row_of(m), run * kRun + 4 * quad, K, vec_a));
+    }
+    for (int f0 = group * feats, stage = 0; f0 < N; f0 += step, stage ^= 1) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float* wa = smem + stage * kStreamStage + (2 * pair * chunk + run_l) * kRun;
+        float4 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { a[i] = ld4(wa + 4 * (i ^ turn)); b[i] = ld4(wa + chunk * kRun + 4 * (i ^ turn)); }
+#pragma unroll
+        for (int m = 0; m < kFewRows; ++m) {
+            if (m >= rows) break;
+            const float* x = rows_a + (m * chunk + run_l) * kRun;
+            float sa = 0.f, sb = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 v = ld4(x + 4 * (i ^ turn));
+                sa = dot4(v, a[i], sa);
+                sb = dot4(v, b[i], sb);
+            }
+            run_sums[(2 * pair * rows + m) * (chunk + 1) + run_l] = sa;
+            run_sums[((2 * pair + 1) * rows + m) * (chunk + 1) + run_l] = sb;
+        }
+        __syncthreads();
+        issue(f0 + 2 * step, stage);
+        // a quarter of K a thread: (row of W, row of A, quarter)
+        for (int i = t; i < 2 * pairs * rows * 4; i += kRowsThreads) {
+            const float* p = run_sums + (i >> 2) * (chunk + 1);
+            const int lo = (i & 3) * q, hi = min(((i & 3) + 1) * q, R);
+            float acc = 0.f;
+            for (int r = lo; r < hi; ++r) acc += p[r];
+            const float v1 = __shfl_down_sync(0xffffffffu, acc, 1), v2 = __shfl_down_sync(0xffffffffu, acc, 2), v3 = __shfl_down_sync(0xffffffffu, acc, 3);
+            if ((i & 3) == 0) total[(i >> 2) / rows * kFewRows + (i >> 2) % rows] = ((acc + v1) + v2) + v3;
+        }
+        __syncthreads();
+        for (int i = t; i < feats * rows; i += kRowsThreads) {
+            const int f = i % feats, m = i / feats;
+            if (f0 + f >= N) continue;
+            if (DUAL) store(m, f0 + f, total[2 * f * kFewRows + m], total[(2 * f + 1) * kFewRows + m]);
+            else store(m, f0 + f, total[f * kFewRows + m], 0.f);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 constexpr int kTileStages = 4;                 // runs of a quarter on their way or being computed
 constexpr int kTileBuf = (kTileRows + kTileFeats) * kRunPitch;
 constexpr int kTileSmemBytes = 4 * kTileStages * kTileBuf * (int)sizeof(float);
@@ -249,6 +340,20 @@ __device__ __forceinline__ void tile_product(int rows, RowOf row_of, const TW* _
             if (f < N) store(m, f, r[j], DUAL ? r[j + 2] : 0.f);
         }
     }
+}
+
+// Blocks of few_rows_stream that the device holds: two an SM (one with more than four rows of A).
+static inline int few_rows_stream_blocks() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return 2 * (sms > 0 ? sms : 1);
+}
+template <class Kernel>
+static inline size_t few_rows_stream_smem(Kernel kernel, int rows, int K) {
+    const int bytes = few_rows_stream_floats(rows < kFewRows ? rows : kFewRows, K) * (int)sizeof(float);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, few_rows_stream_floats(kFewRows, kStreamMaxK) * (int)sizeof(float));
+    return bytes;
 }
 
 // The shared memory of a kernel made of either, which is allowed to it (per launch: the attribute belongs to the device).

@@ -98,3 +98,27 @@ def test_a_matrix_that_the_kernel_before_writes(batch):
         product(out)
     assert not torch.equal(*want)
     assert all(torch.equal(out, want[i % 2]) for i, out in enumerate(outs))
+
+
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 8])
+@pytest.mark.parametrize("N,K", [(4736, 1024), (4739, 1000), (9472, 512), (9473, 20), (11000, 516)])
+def test_matrices_larger_than_the_blocks_hold(M, N, K):
+    """Blocks that walk over groups of features: the bits of a row among 40 others, which takes the tiles."""
+    from mdma_b200 import ops
+    torch.manual_seed(M + N + K)
+    a, w, w2 = (torch.randn(n, K, device=DEV) for n in (M, N, N))
+    out = torch.full((M + 1, N), 9.0, device=DEV)
+    ops.gemm_simt(a, w, out, m=M, w_fixed=True)
+    assert bool(((out[:M] - a.double() @ w.double().t()).abs() <= bound(a, w)).all()) and bool((out[M:] == 9.0).all())
+    rows = torch.cat([a, torch.randn(40, K, device=DEV)])
+    many = torch.empty(M + 40, N, device=DEV)
+    ops.gemm_simt(rows, w, many)
+    assert torch.equal(many[:M], out[:M])
+    x = torch.randn(M, N, device=DEV)
+    x0 = x.clone()
+    ops.gemm_simt(a, w, x, ops.GEMM_ACCUMULATE)
+    assert torch.equal(x, x0 + out[:M])
+    gated, many = torch.empty(M, N, device=DEV), torch.empty(M + 40, N, device=DEV)
+    ops.gemm_simt(a, w, gated, ops.GEMM_SWIGLU, w2)
+    ops.gemm_simt(rows, w, many, ops.GEMM_SWIGLU, w2)
+    assert torch.equal(many[:M], gated)
