@@ -310,10 +310,10 @@ struct PairWork {
     int n_full, first_full;              // then consecutive whole tiles of the evenly split rest
     int head_tile, head_kb1;             // -1: none
     int tail_tile, tail_kb0;             // -1: none
-    int n_kb;
+    int kb_first, n_kb;                  // K blocks of the whole tiles (a K split: the pair's part of them)
     __device__ int count() const { return n_round + n_full + (head_tile >= 0) + (tail_tile >= 0); }
     __device__ Segment get(int i) const {
-        if (i < n_round) return Segment{pair + i * n_pairs, 0, n_kb, kSegFull};
+        if (i < n_round) return Segment{pair + i * n_pairs, kb_first, n_kb, kSegFull};
         i -= n_round;
         if (i < n_full) return Segment{first_full + i, 0, n_kb, kSegFull};
         if (head_tile >= 0 && i == n_full) return Segment{head_tile, 0, head_kb1, kSegHead};
@@ -326,7 +326,7 @@ struct PairWork {
 // two pairs at most.
 __device__ inline PairWork pair_work(int pair, int n_pairs, int n_tiles, int n_kb, bool even_split) {
     PairWork w;
-    w.n_kb = n_kb; w.head_tile = w.tail_tile = -1; w.head_kb1 = w.tail_kb0 = 0;
+    w.kb_first = 0; w.n_kb = n_kb; w.head_tile = w.tail_tile = -1; w.head_kb1 = w.tail_kb0 = 0;
     w.pair = pair; w.n_pairs = n_pairs; w.n_full = 0; w.first_full = 0;
     if (!even_split || n_tiles < n_pairs) {
         w.n_round = pair < n_tiles ? (n_tiles - pair + n_pairs - 1) / n_pairs : 0;
@@ -342,6 +342,14 @@ __device__ inline PairWork pair_work(int pair, int n_pairs, int n_tiles, int n_k
     if (last_end < n_kb) { w.head_tile = base + last_tile; w.head_kb1 = last_end; --last_tile; }
     w.first_full = base + first_tile;
     w.n_full = last_tile >= first_tile ? last_tile - first_tile + 1 : 0;
+    return w;
+}
+// A K split (kTcPartial): pair = split * tiles + tile, one tile and one part of its K blocks.
+__device__ inline PairWork pair_split_work(int pair, int n_pairs, int n_tiles, int n_kb, int kb_per_split) {
+    PairWork w = pair_work(pair % n_tiles, n_pairs, n_tiles, n_kb, false);
+    w.n_round = 1;
+    w.kb_first = pair / n_tiles * kb_per_split;
+    w.n_kb = min(n_kb, w.kb_first + kb_per_split);
     return w;
 }
 
@@ -377,7 +385,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int rank = (int)ptx::cluster_rank();
     const int n_pairs = gridDim.x / 2, pair = blockIdx.x / 2;
     const int f_tiles = (p.n_features + 255) / 256, t_tiles = (p.n_tokens + bn - 1) / bn;
-    const PairWork work = pair_work(pair, n_pairs, f_tiles * t_tiles, p.k_blocks, p.sk_flags != nullptr);
+    const int n_tiles = f_tiles * t_tiles;
+    const PairWork work = MODE == kTcPartial ? pair_split_work(pair, n_pairs, n_tiles, p.k_blocks, p.kb_per_split)
+                                             : pair_work(pair, n_pairs, n_tiles, p.k_blocks, p.sk_flags != nullptr);
     const int n_seg = work.count();
 
     // This kernel takes no part in programmatic dependent launch: launched early next to the tail of
@@ -466,6 +476,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         const uint32_t lead_empty[2] = {ptx::cluster_map(acc_empty(0), 0), ptx::cluster_map(acc_empty(1), 0)};
         // partial tiles in global memory: [pair][block of the pair][accumulator][column][128 rows]
         const size_t part_stride = (size_t)kAccs * BN * 128;
+        // a K split's partial sums; the bias goes into the first split's
+        const int split = MODE == kTcPartial ? pair / n_tiles : 0;
+        float* split_out = MODE == kTcPartial ? p.partial + (size_t)split * p.n_tokens * p.n_features : nullptr;
         float* my_part = p.sk_partial ? p.sk_partial + ((size_t)pair * 2 + rank) * part_stride + row : nullptr;
         const float* prev_part = p.sk_partial && pair > 0 ? p.sk_partial + ((size_t)(pair - 1) * 2 + rank) * part_stride + row : nullptr;
         bool ok = true;
@@ -475,7 +488,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             const int buf = si % kBufs;
             const int f = (sg.tile / t_tiles) * 256 + rank * 128 + row;
             const int t0 = (sg.tile % t_tiles) * bn;
-            const float b1 = f < p.n_features ? ending_bias(p.ending.bias, p.ending.bias_dtype, f) : 0.f;
+            const float b1 = f < p.n_features && split == 0 ? ending_bias(p.ending.bias, p.ending.bias_dtype, f) : 0.f;
             const float b2 = kDual && f < p.n_features ? ending_bias(p.ending.bias2, p.ending.bias_dtype, f) : 0.f;
             ok = __all_sync(0xffffffffu, ptx::mbar_wait(acc_full(buf), (si / kBufs) & 1, abort_flag));
             if (!ok) break;
@@ -572,7 +585,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                             float r = v[q] + b1;
                             if (MODE == kTcSwiGLU) r = gated_pair_fast(r, u[q] + b2, p.ending.act, p.ending.act_limit, p.ending.act_alpha);
                             if (MODE == kTcStore && p.ending.store_act) r = gate_activation_fast(r, p.ending.act);
-                            if (p.out_f32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + f] = r;
+                            if (MODE == kTcPartial) split_out[(size_t)t * p.n_features + f] = r;
+                            else if (p.out_f32) reinterpret_cast<float*>(p.out)[(size_t)t * p.ldo + f] = r;
                             else reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)t * p.ldo + f] = __float2bfloat16_rn(r);
                         }
                     }
@@ -796,7 +810,8 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
     p.cluster = 1;
     cudaLaunchConfig_t cfg = {};
     const long tiles = (long)((p.n_features + 255) / 256) * ((p.n_tokens + p.pair_tokens - 1) / p.pair_tokens);
-    const int pairs = (int)(tiles < sm_count / 2 ? tiles : sm_count / 2);
+    const int splits = MODE == kTcPartial ? (p.k_blocks + p.kb_per_split - 1) / p.kb_per_split : 1;
+    const int pairs = (int)(MODE == kTcPartial ? tiles * splits : tiles < sm_count / 2 ? tiles : sm_count / 2);
     cfg.gridDim = dim3(pairs * 2, 1, 1);
     cfg.blockDim = dim3(tc2_threads<MODE>()); cfg.dynamicSmemBytes = S::kBytes; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -820,7 +835,7 @@ static int run_tc2(const void* x, int ldx, const void* w, const void* w2, int K,
         max_pairs = n;
     }
     const long rounds = (tiles + pairs - 1) / pairs;
-    const bool uneven = tiles > pairs && (rounds * pairs - tiles) * p.k_blocks >= 56l * pairs;
+    const bool uneven = MODE != kTcPartial && tiles > pairs && (rounds * pairs - tiles) * p.k_blocks >= 56l * pairs;
     if (!(uneven && pairs <= max_pairs)) { p.sk_partial = nullptr; p.sk_flags = nullptr; }
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc2_kernel<MODE>, mw, mw2, mx, p);
     if (e != cudaSuccess) return fail("gemm_tc2: launch failed: %s", cudaGetErrorString(e));
@@ -874,6 +889,20 @@ int mdma_gemm_tc_plan(int mode, int n_tokens, int n_features, int K, int sm_coun
         // and a K split that gives every SM a block takes 50.1 us and 24.8 us there (512 tokens: 79.9 against
         // 89.1 us and 29.5 against 32.9 us).  Two weight matrices (SwiGLU) stay with the pairs (61 against 95 us).
         const long pair_tiles = (long)((n_features + 255) / 256) * ((n_tokens + 255) / 256);
+        // A product into the residual stream leaves partial sums for the norm behind it, so its K is divided among pairs that
+        // would idle (product and norm, us; without the split / with): 768 tokens 2,048 x 2,048 22.1 / 16.8, K 8,192 50.3 / 27.4,
+        // 1,024 x 4,096 29.9 / 15.7; 1,024 tokens 2,048 x 8,192 51.8 / 33.4; 2,048 tokens 1,024 x 4,096 32.2 / 23.3.  Of 257-512
+        // tokens where there are 32 tiles for two splits and enough K or tokens (against the one-block kernel): 512 tokens
+        // 4,096 x 4,096 27.7 / 23.5, K 14,336 58.1 / 53.2; 384 tokens K 14,336 55.3 / 48.4, but K 4,096 22.8 / 23.1, 2,048 x 2,048
+        // (16 tiles) 11.4 / 13.7.  Not for a stored product: the sum of its parts costs more (768 tokens 3,072 x 2,048 17.7 / 27.7).
+        if (mode == kTcAccumulate) {
+            const int k_blocks = (K + kBK - 1) / kBK;
+            int splits = (int)(sm_count / 2 / pair_tiles);
+            if (splits > 8) splits = 8;
+            if (splits > k_blocks / 4) splits = k_blocks / 4;
+            const bool wide = 10 * splits * pair_tiles >= (long)(sm_count / 2) * 8 && 3 * pair_tiles > sm_count / 2;
+            if (splits >= 2 && (n_tokens > 512 || (n_tokens > 256 && wide && (K >= 8192 || n_tokens > 384)))) { *bn_out = 512; *splits_out = splits; return 0; }
+        }
         if (mode != kTcSwiGLU && n_tokens <= 512 && pair_tiles * 10 < (long)(sm_count / 2) * 6) {
             // Token tiles of 128, or of 256 where that puts more blocks on the SMs at once (O and down of 384
             // tokens: 64 tiles of 256 x 2 splits against 96 tiles of 128).  Not for a product that is stored
@@ -908,13 +937,20 @@ int mdma_gemm_tc_plan(int mode, int n_tokens, int n_features, int K, int sm_coun
     const int k_blocks = (K + kBK - 1) / kBK;
     const long tiles = (long)((n_features + kBM - 1) / kBM) * ((n_tokens + bn - 1) / bn);
     int splits = 1;
+    if (mode == kTcSwiGLU && bn == 64 && 2 * tiles <= sm_count) {
+        // ... and of 33-64 tokens where one block a tile leaves half of the device idle: norm and product of 64 tokens, us, one
+        // block / pairs: 8,192 x 2,048 26.9 / 24.8, 5,632 x 2,048 26.4 / 23.6, 2,752 x 1,024 17.4 / 15.2 (14,336 x 4,096 52.3 / 52.3)
+        *bn_out = 512; *splits_out = 1; return 0;
+    }
     if (mode == kTcSwiGLU && bn <= 32 && tiles < sm_count && k_blocks >= 8) {
         // The SwiGLU ending needs complete sums, so its K split stays inside a cluster of two blocks
         // (measured at batch 8: 37.4 us against 41.8 us unsplit; larger clusters and cluster splits
         // of the other products were slower than partial sums through global memory).  With 64 tokens
         // the partial sums are four times as large and one block per SM with a deep ring is faster
-        // (44.4 us against 48.4 us).
-        *bn_out = bn; *splits_out = -2; return 0;
+        // (44.4 us against 48.4 us).  Four blocks where they still fit two an SM and there are 4 K blocks for each (norm and product
+        // of 8 tokens, us, clusters of 2 / 4): 8,192 x 2,048 18.6 / 16.2, 5,632 x 2,048 16.0 / 13.7, 2,752 x 1,024 9.9 / 8.5,
+        // 8,192 x 3,072 24.2 / 21.4, but 11,008 x 4,096 (86 tiles) 34.7 / 40.5; 32 tokens 22.3 / 22.3.
+        *bn_out = bn; *splits_out = bn == 16 && 4 * tiles <= 2 * sm_count && k_blocks >= 16 ? -4 : -2; return 0;
     }
     if (mode != kTcSwiGLU && tiles < sm_count) {
         // As many blocks as can be resident at once, not more: two per SM for token tiles up to 64
@@ -1018,6 +1054,15 @@ int mdma_gemm_tc(int mode, const void* x, int ldx, const void* w, const void* w2
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const long part_floats = (long)sms * (mode == kTcSwiGLU ? 2 : 1) * 256 * 128;
         p.sk_partial = nullptr; p.sk_flags = nullptr;
+        if (splits > 1) {
+            const long need = (long)splits * n_tokens * n_features;
+            MDMA_REQUIRE(scratch && scratch_floats >= need, "gemm_tc: a %d-way K split needs %ld floats of scratch, %ld given", splits, need, scratch_floats);
+            p.partial = scratch;
+            if (int rc = run_tc2<kTcPartial>(x, ldx, w, w2, K, p, stream)) return rc;
+            if (splits_used) *splits_used = splits;
+            if (defer_reduce) return 0;
+            return splitk_reduce_run(mode, scratch, splits, n_tokens, n_features, out, ldo, out_f32, store_act, act, stream);
+        }
         if (sk_flags != nullptr && scratch != nullptr && scratch_floats >= part_floats) { p.sk_partial = scratch; p.sk_flags = sk_flags; }
         if (mode == kTcStore) return run_tc2<kTcStore>(x, ldx, w, w2, K, p, stream);
         if (mode == kTcAccumulate) return run_tc2<kTcAccumulate>(x, ldx, w, w2, K, p, stream);

@@ -130,9 +130,11 @@ def _gemm_plan(mode: int, n_tokens: int, n_features: int, k: int, sms: int) -> t
 
 def gemm_scratch_floats(bn: int, splits: int, m: int, n: int, sms: int) -> int:
     """Floats of scratch a product of m tokens x n features needs with this token tile and K split: the partial
-    sums of a split through global memory, or the partial tiles of the block-pair kernel (`bn` 512)."""
+    sums of a split through global memory, or the partial tiles of the block-pair kernel (`bn` 512) where it has more tiles than pairs."""
     if bn == 512:
-        return pair_scratch_floats(sms)
+        if splits > 1:
+            return splits * m * n
+        return pair_scratch_floats(sms) if -(-m // 256) * -(-n // 256) > sms // 2 else 0
     return splits * m * n if splits > 1 else 0
 
 
@@ -263,10 +265,10 @@ def attention_supported(n_heads: int, n_kv_heads: int, head_dim: int) -> bool:
 
 
 def attention_splits(n_seqs: int, max_new: int, max_len: int, n_heads: int, n_kv_heads: int, sms: int,
-                     most_seqs: Optional[int] = None) -> int:
-    """How many ways to divide a tile's keys so that the grid fills the device.  `most_seqs`: the most
-    sequences the engine can hold; the choice for a handful of sequences is made from it, not from the
-    live batch, so that a request's arithmetic does not change when a batch mate ends."""
+                     most_seqs: Optional[int] = None, most_len: Optional[int] = None, head_dim: int = 0) -> int:
+    """How many ways to divide a tile's keys so that the grid fills the device.  `most_seqs`, `most_len`: the most
+    sequences and the longest context the engine can hold; the choice for a handful of sequences is made from them, not from
+    the live batch, so that a request's arithmetic does not change when a batch mate ends."""
     group = n_heads // n_kv_heads
     key_blocks = max(1, -(-max_len // 64))
     if max_new == 1 and group <= 16:
@@ -286,6 +288,8 @@ def attention_splits(n_seqs: int, max_new: int, max_len: int, n_heads: int, n_kv
         if blocks >= sms:
             return 1
         few = (most_seqs or n_seqs) * n_kv_heads * 4 <= (3 * sms) // 4
+        if few and most_len is not None and most_len <= 12 * (64 if head_dim <= 64 else 32):
+            return 1                               # one tile a warp of one block: nothing to divide, and no merge
         if max_len <= 1024:
             return 4 if few else 1
         if few:
@@ -379,7 +383,7 @@ def attention(ctx, qkv: torch.Tensor, view, out: torch.Tensor, n_heads: int, n_k
     flush_pending(qkv.device, st)
     if splits is None:
         splits = attention_splits(ctx.n_seqs, ctx.max_new, ctx.max_len, n_heads, n_kv_heads, st.sms,
-                                  getattr(ctx, "most_seqs", None))
+                                  getattr(ctx, "most_seqs", None), getattr(ctx, "most_len", None), head_dim)
     st.need(ctx.n_tokens * n_heads * splits * (head_dim + 2) if splits > 1 else 0, "attention over split keys")
     args = (_ptr(qkv), _i(qkv.stride(0)), _ptr(view.k), _ptr(view.v),
             _i(view.k.shape[0] if view.k.is_contiguous() and view.v.is_contiguous() else 0), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(ctx.seq_slot), _ptr(view.page_table),
@@ -424,7 +428,8 @@ def attention_decode_rotary(ctx, qkv: torch.Tensor, view, out: torch.Tensor, n_h
     else:
         flush_pending(qkv.device, st)
     if splits is None:
-        splits = attention_splits(ctx.n_seqs, 1, ctx.max_len, n_heads, n_kv_heads, st.sms, getattr(ctx, "most_seqs", None))
+        splits = attention_splits(ctx.n_seqs, 1, ctx.max_len, n_heads, n_kv_heads, st.sms, getattr(ctx, "most_seqs", None),
+                                  getattr(ctx, "most_len", None), head_dim)
         if splits == 1 and not window:
             splits, chunk_keys = decode_chunks(ctx.n_seqs, -(-ctx.max_len // 1024) * 1024, n_kv_heads, st.sms,
                                                getattr(ctx, "most_seqs", None), getattr(ctx, "most_len", None))

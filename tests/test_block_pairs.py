@@ -69,3 +69,46 @@ def test_gates_far_from_zero(bn):
     assert torch.isfinite(out).all()
     # (what is below the smallest normal float may come out as 0)
     assert bool(((out.double() - want).abs() <= 2 ** -8 * want.abs() + 2.0 ** -126 * u.abs().clamp(min=1.0)).all())
+
+
+def _product(M, N, K, mode, bias, act, **forced):
+    """(result, reference, bound) of a product through the planner or as `forced`; partial sums are added up at once."""
+    from mdma_b200 import ops, ops_tensor
+    torch.manual_seed(M + N + K)
+    a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    w = (torch.randn(N, K, device=DEV) * K ** -0.5).bfloat16()
+    b = torch.randn(N, device=DEV).bfloat16() if bias else None
+    x0 = torch.randn(M + 1, N, device=DEV)
+    out = x0.clone() if mode == 1 else torch.full((M + 1, N), 9.0, device=DEV, dtype=torch.bfloat16)
+    keep = out[M:].clone()
+    ops_tensor.gemm(a, w, out, mode, None, M, bias=b, store_act=act, act=ops.ACT_GELU_TANH if act else ops.ACT_SILU, **forced)
+    ops_tensor.check_status(torch.device(DEV))
+    assert torch.equal(out[M:], keep)
+    ref = a.double() @ w.double().t() + (b.double() if bias else 0.0)
+    if mode == 1:
+        return out[:M].double(), ref + x0[:M].double(), 1e-5 * (1 + ref.abs())          # sums of K products of order 0.5 / sqrt(K) in float
+    if act:
+        ref = torch.nn.functional.gelu(ref, approximate="tanh")
+    return out[:M].double(), ref, 2.0 ** -8 * ref.abs() + 2e-5                          # one rounding to bfloat16
+
+
+@pytest.mark.parametrize("M,N,K,splits", [(129, 256, 256, 2), (130, 300, 1000, 3), (256, 512, 4096, 8), (257, 260, 520, 2), (600, 1000, 1024, 4), (2048, 1024, 512, 2)])
+@pytest.mark.parametrize("mode,bias,act", [(1, False, False), (1, True, False), (0, True, True)])
+def test_pairs_that_divide_k(M, N, K, splits, mode, bias, act):
+    got, want, tol = _product(M, N, K, mode, bias, act, bn=512, splits=splits)
+    assert bool(((got - want).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("M,N,K,plan", [(1, 8192, 2048, (16, -4)), (8, 2752, 1024, (16, -4)), (16, 330, 1032, (16, -4)), (40, 8192, 2048, (512, 1)), (33, 300, 1024, (512, 1)), (64, 2750, 1032, (512, 1))])
+def test_gated_products_of_few_tiles(M, N, K, plan):
+    from mdma_b200 import ops, ops_tensor
+    assert ops_tensor.gemm_plan(2, M, N, K, 148) == plan
+    torch.manual_seed(M + N)
+    a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    w, w2 = ((torch.randn(N, K, device=DEV) * K ** -0.5).bfloat16() for _ in range(2))
+    out = torch.full((M + 1, N), 9.0, device=DEV, dtype=torch.bfloat16)
+    ops_tensor.gemm(a, w, out, ops.GEMM_SWIGLU, w2, M)
+    ops_tensor.check_status(torch.device(DEV))
+    ref = a.double() @ w.double().t()
+    ref = ref / (1 + torch.exp(-ref)) * (a.double() @ w2.double().t())
+    assert bool((out[M:] == 9.0).all()) and bool(((out[:M].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all())

@@ -66,3 +66,12 @@ def test_every_choice_of_key_splits_fits_the_scratch_reserved_for_attention(head
                     worst = max(worst, need)
                     assert need <= reserved, (n_seqs, max_new, max_len, most, splits, need, reserved)
     assert worst > 0          # the sweep did reach split cases
+
+
+def test_contexts_of_one_tile_a_warp_are_not_divided():
+    """An engine for a handful of sequences whose longest context is one tile for each of a block's twelve warps: no pieces,
+    whatever its sequences hold; a longer one is cut as before."""
+    splits = lambda most_len, dim: {ops_tensor.attention_splits(n, 1, length, 32, 8, 148, 2, most_len, dim) for n in (1, 2) for length in (1, 64, most_len)}  # noqa: E731
+    assert splits(384, 128) == {1} and splits(768, 64) == {1} and splits(100, 64) == {1}
+    assert splits(385, 128) == {4} and splits(769, 64) == {4} and splits(1000, 128) == {4}
+    assert ops_tensor.attention_splits(1, 1, 100, 32, 8, 148, 2) == 4
