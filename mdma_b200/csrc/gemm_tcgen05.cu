@@ -721,6 +721,11 @@ static int make_map_2d(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_
 
 using namespace mdma;
 
+// Whether a cluster of the one-block kernel may start beside the end of the kernel in front of it.  One of two blocks is placed
+// as ordinary blocks are, two on a TPC; a wider one needs room on several TPCs at once, which clusters that still wait for
+// theirs and blocks that hold it could deny each other.
+static bool cluster_starts_early(int blocks) { return blocks <= 2 && chaining_enabled(); }
+
 template <int BN, int MODE>
 static int run_tc(const void* x, int ldx, const void* w, const void* w2, int K, TcParams p, int splits,
                   cudaStream_t stream) {
@@ -752,7 +757,7 @@ static int run_tc(const void* x, int ldx, const void* w, const void* w2, int K, 
         attr[0].val.clusterDim.x = p.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr; cfg.numAttrs = chaining_enabled() ? 2 : 1;
+        cfg.attrs = attr; cfg.numAttrs = cluster_starts_early(p.cluster) ? 2 : 1;
         cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, MODE>, mw, mw2, mx, p);
         if (e != cudaSuccess) return fail("gemm_tc: cluster launch failed: %s", cudaGetErrorString(e));
         return 0;
@@ -875,6 +880,9 @@ int mdma_wait_probe(int mode, const int* flag, int* status, cudaStream_t stream)
     return 0;
 }
 
+// Returns 1 if a product whose K is split inside clusters of so many blocks is launched to start early.
+int mdma_gemm_tc_starts_early(int cluster) { return cluster_starts_early(cluster) ? 1 : 0; }
+
 // Returns 1 if the tensor-core kernel takes this weight shape.
 int mdma_gemm_tc_supported(int n_features, int K) { return (K % 8 == 0 && K >= 8 && n_features >= 1) ? 1 : 0; }
 
@@ -947,10 +955,10 @@ int mdma_gemm_tc_plan(int mode, int n_tokens, int n_features, int K, int sm_coun
         // (measured at batch 8: 37.4 us against 41.8 us unsplit; larger clusters and cluster splits
         // of the other products were slower than partial sums through global memory).  With 64 tokens
         // the partial sums are four times as large and one block per SM with a deep ring is faster
-        // (44.4 us against 48.4 us).  Four blocks where they still fit two an SM and there are 4 K blocks for each (norm and product
-        // of 8 tokens, us, clusters of 2 / 4): 8,192 x 2,048 18.6 / 16.2, 5,632 x 2,048 16.0 / 13.7, 2,752 x 1,024 9.9 / 8.5,
-        // 8,192 x 3,072 24.2 / 21.4, but 11,008 x 4,096 (86 tiles) 34.7 / 40.5; 32 tokens 22.3 / 22.3.
-        *bn_out = bn; *splits_out = bn == 16 && 4 * tiles <= 2 * sm_count && k_blocks >= 16 ? -4 : -2; return 0;
+        // (44.4 us against 48.4 us).  Clusters of four may not start early (`cluster_starts_early`), and without that they lose
+        // (norm and product of 8 tokens, us, two / four: 8,192 x 2,048 21.1 / 21.1, 5,632 x 2,048 18.1 / 19.1, 2,752 x 1,024
+        // 10.9 / 12.9; a decode step of Llama-3.2-1B, 1 sequence 811 / 804, 8 863 / 867, 16 905 / 926).
+        *bn_out = bn; *splits_out = -2; return 0;
     }
     if (mode != kTcSwiGLU && tiles < sm_count) {
         // As many blocks as can be resident at once, not more: two per SM for token tiles up to 64

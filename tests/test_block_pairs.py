@@ -99,7 +99,7 @@ def test_pairs_that_divide_k(M, N, K, splits, mode, bias, act):
     assert bool(((got - want).abs() <= tol).all())
 
 
-@pytest.mark.parametrize("M,N,K,plan", [(1, 8192, 2048, (16, -4)), (8, 2752, 1024, (16, -4)), (16, 330, 1032, (16, -4)), (40, 8192, 2048, (512, 1)), (33, 300, 1024, (512, 1)), (64, 2750, 1032, (512, 1))])
+@pytest.mark.parametrize("M,N,K,plan", [(1, 8192, 2048, (16, -2)), (8, 2752, 1024, (16, -2)), (16, 330, 1032, (16, -2)), (40, 8192, 2048, (512, 1)), (33, 300, 1024, (512, 1)), (64, 2750, 1032, (512, 1))])
 def test_gated_products_of_few_tiles(M, N, K, plan):
     from mdma_b200 import ops, ops_tensor
     assert ops_tensor.gemm_plan(2, M, N, K, 148) == plan

@@ -43,6 +43,16 @@ def test_choices_that_the_measurements_rest_on():
     assert plan(STORE, 8, 128256, 4096) == (16, 1)           # the head: more tiles than SMs, no split
 
 
+def test_clusters_that_start_early_have_two_blocks():
+    """A cluster is placed as ordinary blocks are up to two blocks; wider ones are launched in stream order and never planned."""
+    from mdma_b200.csrc import build
+    early = build.load("tensor").mdma_gemm_tc_starts_early
+    assert [early(c) for c in (3, 4, 8)] == [0, 0, 0]
+    for m in (1, 8, 16, 17, 32):
+        for n, k in ((8192, 2048), (5632, 2048), (2752, 1024), (8192, 3072), (331, 640), (14336, 4096), (128, 65536)):
+            assert ops_tensor.gemm_plan(GATED, m, n, k, 148)[1] in (-2, 1), (m, n, k)
+
+
 @pytest.mark.parametrize("sms", [148, 78])
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(32, 8, 128), (32, 32, 128), (32, 8, 64), (16, 8, 16), (6, 3, 48), (64, 1, 32), (40, 2, 64)])
 def test_every_choice_of_key_splits_fits_the_scratch_reserved_for_attention(heads, kv_heads, head_dim, sms):
