@@ -84,12 +84,19 @@ __device__ __forceinline__ int warp_largest(const float* v, int n, int lane) {
 }
 
 // ---------------------------------------------------------------- router
-constexpr int kRouteWarps = 32;
+constexpr int kRouteWide = 32, kRouteNarrow = 8;
 
-// A block a token; a warp an output, as long as there are no more than kRouteWarps (and one for the shared gate): the sums side
-// by side are one round trip (4 tokens, 16 outputs and a gate of 1,024 floats 8 us, 11 with eight warps).
-template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(kRouteWarps * 32)
+// Warps of a token's block.  Where every token has an SM of its own, a warp an output (and one for the shared gate), as long as
+// there are no more than kRouteWide: the sums side by side are one round trip.  Of more tokens eight warps, six blocks an SM: one
+// warp's serial tail then lies under other tokens' sums.  16 outputs and a gate of 2,048 in bfloat16, us, wide / eight: 4 tokens
+// 7.9 / 9.9, 148 8.2 / 10.4, 200 14.3 / 10.5, 512 16 / 13.3, 6,000 142 / 70; 64 outputs 12 / 18, 12 / 18, 23 / 19, 46 / 32, 459 / 166.
+static int route_warps(int n_tokens, int outputs, int sm_count) {
+    if (n_tokens > sm_count || outputs <= kRouteNarrow) return kRouteNarrow;
+    return outputs < kRouteWide ? outputs : kRouteWide;
+}
+
+template <typename TA, typename TW, typename TC, int MAX_WARPS>
+__global__ void __launch_bounds__(MAX_WARPS * 32, MAX_WARPS == kRouteNarrow ? 6 : 1)
 route_kernel(const TA* __restrict__ h, int h_stride, const TW* __restrict__ router, const TC* __restrict__ correction,
              const TW* __restrict__ shared_gate, int width, int n_routed, int top, int n_groups, int keep_groups,
              int scoring, int group_top, int renormalize, int logit_bias, float weight_scale,
@@ -467,6 +474,9 @@ using namespace mdma;
 
 extern "C" {
 
+// Warps of a token's block in mdma_route for so many outputs, the shared gate's among them.
+int mdma_route_warps(int n_tokens, int outputs, int sm_count) { return route_warps(n_tokens, outputs, sm_count); }
+
 int mdma_route(const void* h, int h_dtype, int h_stride, const void* router, int w_dtype, const void* correction,
                int c_dtype, const void* shared_gate, int n_tokens, int width, int n_routed, int top, int n_groups,
                int keep_groups, int scoring, int group_top, int renormalize, int logit_bias, float weight_scale, int* chosen,
@@ -481,11 +491,14 @@ int mdma_route(const void* h, int h_dtype, int h_stride, const void* router, int
                  "route: %d groups (keep %d) over %d outputs", n_groups, keep_groups, n_routed);
     MDMA_REQUIRE(shared_gate == nullptr || shared_scale != nullptr, "route: the shared gate needs a place for its result");
     if (n_tokens == 0) return 0;
-    int warps = n_routed + (shared_gate != nullptr);
-    warps = warps < 8 ? 8 : warps > kRouteWarps ? kRouteWarps : warps;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int warps = route_warps(n_tokens, n_routed + (shared_gate != nullptr), sms);
     MDMA_DISPATCH_2(h_dtype, TA, w_dtype, TW,
         MDMA_DISPATCH_DTYPE(c_dtype, TC,
-            launch_chained(route_kernel<TA, TW, TC>, dim3(n_tokens), dim3(warps * 32), 0, stream, (const TA*)h, h_stride,
+            launch_chained(warps == kRouteNarrow ? route_kernel<TA, TW, TC, kRouteNarrow> : route_kernel<TA, TW, TC, kRouteWide>,
+                           dim3(n_tokens), dim3(warps * 32), 0, stream, (const TA*)h, h_stride,
                            (const TW*)router, (const TC*)correction, (const TW*)shared_gate, width, n_routed, top,
                            n_groups, keep_groups, scoring, group_top, renormalize, logit_bias, weight_scale, chosen, weights, shared_scale)));
     MDMA_LAUNCH_OK("route");
