@@ -889,7 +889,8 @@ int mdma_gemm_tc_supported(int n_features, int K) { return (K % 8 == 0 && K >= 8
 // Bytes of float scratch a call with these sizes needs (0 when it does not split K).
 // `splits` <= 0 asks the library to choose.
 // `splits_out` < 0 means: split K that many ways inside a cluster (no scratch, reduced in shared memory).
-int mdma_gemm_tc_plan(int mode, int n_tokens, int n_features, int K, int sm_count, int* bn_out, int* splits_out) {
+// `folded`: the kernel behind the product reads its rows anyway (a norm, a gate) and adds partial sums up on its way.
+int mdma_gemm_tc_plan(int mode, int folded, int n_tokens, int n_features, int K, int sm_count, int* bn_out, int* splits_out) {
     if (n_tokens > 128) {
         // Many tokens: block pairs, 256 features x 256 tokens per pair (`bn` code 512).  But with few
         // feature tiles and 129-512 tokens the pairs leave most of the device idle (the down product of 256
@@ -897,13 +898,14 @@ int mdma_gemm_tc_plan(int mode, int n_tokens, int n_features, int K, int sm_coun
         // and a K split that gives every SM a block takes 50.1 us and 24.8 us there (512 tokens: 79.9 against
         // 89.1 us and 29.5 against 32.9 us).  Two weight matrices (SwiGLU) stay with the pairs (61 against 95 us).
         const long pair_tiles = (long)((n_features + 255) / 256) * ((n_tokens + 255) / 256);
-        // A product into the residual stream leaves partial sums for the norm behind it, so its K is divided among pairs that
+        // Where a norm behind a product into the residual stream adds the partial sums up, K is divided among pairs that
         // would idle (product and norm, us; without the split / with): 768 tokens 2,048 x 2,048 22.1 / 16.8, K 8,192 50.3 / 27.4,
         // 1,024 x 4,096 29.9 / 15.7; 1,024 tokens 2,048 x 8,192 51.8 / 33.4; 2,048 tokens 1,024 x 4,096 32.2 / 23.3.  Of 257-512
         // tokens where there are 32 tiles for two splits and enough K or tokens (against the one-block kernel): 512 tokens
         // 4,096 x 4,096 27.7 / 23.5, K 14,336 58.1 / 53.2; 384 tokens K 14,336 55.3 / 48.4, but K 4,096 22.8 / 23.1, 2,048 x 2,048
-        // (16 tiles) 11.4 / 13.7.  Not for a stored product: the sum of its parts costs more (768 tokens 3,072 x 2,048 17.7 / 27.7).
-        if (mode == kTcAccumulate) {
+        // (16 tiles) 11.4 / 13.7.  Not where the sums need a launch of their own (768 tokens 2,048 x 2,048 20.9 / 27.1, 3,072 x
+        // 3,072 27.0 / 35.2, 1,500 tokens 1,536 x 1,536 18.8 / 30.5; with K four times that 1,536 x 6,144 39.8 / 43.4).
+        if (mode == kTcAccumulate && folded) {
             const int k_blocks = (K + kBK - 1) / kBK;
             int splits = (int)(sm_count / 2 / pair_tiles);
             if (splits > 8) splits = 8;
@@ -1162,7 +1164,7 @@ int mdma_gemm_tc_runs(int mode, const void* x, int ldx, const void* w, const voi
         if (lo < 0 || m < 0) { rc = fail("gemm_tc_runs: run %d is not a run", r); break; }
         if (m == 0) continue;
         int bn = 0, splits = 0;
-        rc = mdma_gemm_tc_plan(mode, m, n_features, K, sm_count, &bn, &splits);
+        rc = mdma_gemm_tc_plan(mode, 0, m, n_features, K, sm_count, &bn, &splits);
         if (rc) break;
         if (splits > 1) splits = 1;          // no partial sums through the scratch: the runs side by side fill the device
         const char* xr = (const char*)x + (size_t)lo * ldx * 2;

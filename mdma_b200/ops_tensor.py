@@ -65,6 +65,7 @@ class TensorState:
         self.sk_flags = sk_flags if sk_flags is not None else zeros(max(512, 4 * self.sms), torch.int32)
         self.scratch = scratch if scratch is not None else zeros(max(scratch_floats, 1), torch.float32)
         self.pending: Optional[Pending] = None
+        self.folds = True          # whether the kernel behind a deferred product adds its partial sums up (`Runtime.unfolded`)
         self.growable = growable
 
     def need(self, floats: int, what: str) -> None:
@@ -108,10 +109,10 @@ def gemm_supported(n_features: int, k: int) -> bool:
 _plans: dict = {}
 
 
-def gemm_plan(mode: int, n_tokens: int, n_features: int, k: int, sms: int) -> tuple[int, int]:
+def gemm_plan(mode: int, n_tokens: int, n_features: int, k: int, sms: int, folded: bool = False) -> tuple[int, int]:
     """(token tile, K splits) the library chooses for a product of these sizes (kept: a step asks
-    for the same few products hundreds of times)."""
-    key = (mode, n_tokens, n_features, k, sms)
+    for the same few products hundreds of times).  `folded`: the kernel behind it adds partial sums up on its way."""
+    key = (mode, folded, n_tokens, n_features, k, sms)
     plan = _plans.get(key)
     if plan is None:
         if len(_plans) > 4096:
@@ -120,10 +121,10 @@ def gemm_plan(mode: int, n_tokens: int, n_features: int, k: int, sms: int) -> tu
     return plan
 
 
-def _gemm_plan(mode: int, n_tokens: int, n_features: int, k: int, sms: int) -> tuple[int, int]:
+def _gemm_plan(mode: int, folded: bool, n_tokens: int, n_features: int, k: int, sms: int) -> tuple[int, int]:
     lib = _build.load("tensor")
     bn, splits = ctypes.c_int(0), ctypes.c_int(0)
-    lib.mdma_gemm_tc_plan(_i(mode), _i(n_tokens), _i(n_features), _i(k), _i(sms),
+    lib.mdma_gemm_tc_plan(_i(mode), _i(int(folded)), _i(n_tokens), _i(n_features), _i(k), _i(sms),
                           ctypes.byref(bn), ctypes.byref(splits))
     return bn.value, splits.value
 
@@ -200,7 +201,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = ops.GE
     st = st or _device_state(a.device)
     flush_pending(a.device, st)
     if bn is None or splits is None:
-        pbn, psplits = gemm_plan(mode, M, N, K, st.sms)
+        pbn, psplits = gemm_plan(mode, M, N, K, st.sms, defer and mode == ops.GEMM_ACCUMULATE and st.folds)
         bn = bn or pbn
         splits = splits or psplits
     st.need(gemm_scratch_floats(bn, splits, M, N, st.sms), "a K-split product")

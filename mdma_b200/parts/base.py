@@ -36,6 +36,17 @@ class Runtime:
     tc: object = None                  # the engine's `ops_tensor.TensorState` (None: a shared default)
     alloc: object = None               # alloc(shape, dtype) for the device tensors a part derives at bind
 
+    def unfolded(self, run, *args):
+        """run(*args), a sublayer whose last product's partial sums take a launch of their own: no kernel behind it adds
+        them up on its way, so that product is planned to leave none where they cost more than they save."""
+        if self.tc is None:
+            return run(*args)
+        before, self.tc.folds = self.tc.folds, False
+        try:
+            return run(*args)
+        finally:
+            self.tc.folds = before
+
     def derived(self, host: torch.Tensor) -> torch.Tensor:
         """A device copy of a small tensor a part computed on the host (a table of frequencies):
         taken from the engine's arena when there is one (the part then names it in `device_tensors`)."""

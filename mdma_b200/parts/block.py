@@ -26,6 +26,8 @@ class PreNormBlock:
         self.mixer = MIXERS.get(spec.mixer.kind)(spec.mixer)
         self.ffn_norm = NORMS.get(spec.ffn_norm.kind)(spec.ffn_norm)
         self.ffn = FEED_FORWARDS.get(spec.ffn.kind)(spec.ffn)
+        # whether the norm behind each sublayer adds up what its product leaves (behind the feed-forward: the next layer's)
+        self.mixer_folds, self.ffn_folds = (getattr(n, "fuses_pending", False) for n in (self.ffn_norm, self.mixer_norm))
 
     handles_pending = True      # completes x itself where a product left partial sums (see _settle)
 
@@ -40,10 +42,16 @@ class PreNormBlock:
         h = ctx.buf("normed", x.shape[1])
         self._settle(ctx, x, self.mixer_norm)
         self.mixer_norm.forward(ctx, x, h)
-        self.mixer.forward(ctx, h, x, view, owns_cache)
+        if self.mixer_folds:
+            self.mixer.forward(ctx, h, x, view, owns_cache)
+        else:
+            ctx.rt.unfolded(self.mixer.forward, ctx, h, x, view, owns_cache)
         self._settle(ctx, x, self.ffn_norm)
         self.ffn_norm.forward(ctx, x, h)
-        self.ffn.forward(ctx, h, x)
+        if self.ffn_folds:
+            self.ffn.forward(ctx, h, x)
+        else:
+            ctx.rt.unfolded(self.ffn.forward, ctx, h, x)
 
     @staticmethod
     def _settle(ctx, x, norm):
@@ -135,7 +143,7 @@ class ShiftGatedBlock:
             part.produce(ctx, h, y, *more, defer=True)
             return
         y[:ctx.n_tokens].zero_()
-        part.forward(ctx, h, y, *more)
+        ctx.rt.unfolded(part.forward, ctx, h, y, *more)
         if ctx.rt.gemm == "tensor":
             from .. import ops_tensor
             ops_tensor.flush_pending(y.device, ctx.rt.tc)
@@ -155,6 +163,7 @@ class ParallelBlock:
         self.ffn = FEED_FORWARDS.get(spec.ffn.kind)(spec.ffn) if spec.ffn is not None else None
         if spec.ffn_norm is not None:
             raise ValueError("the parallel arrangement has one norm; its feed-forward reads the mixer's")
+        self.folds = getattr(self.mixer_norm, "fuses_pending", False)      # the next layer's norm
 
     def parts(self):
         return [p for p in (self.mixer_norm, self.mixer, self.ffn) if p is not None]
@@ -166,9 +175,17 @@ class ParallelBlock:
         h = ctx.buf("normed", x.shape[1])
         PreNormBlock._settle(ctx, x, self.mixer_norm)
         self.mixer_norm.forward(ctx, x, h)
-        self.mixer.forward(ctx, h, x, view, owns_cache)
-        if self.ffn is not None:
+        # (behind the mixer comes the feed-forward's first product, which reads no x)
+        if self.ffn is None and self.folds:
+            self.mixer.forward(ctx, h, x, view, owns_cache)
+        else:
+            ctx.rt.unfolded(self.mixer.forward, ctx, h, x, view, owns_cache)
+        if self.ffn is None:
+            return
+        if self.folds:
             self.ffn.forward(ctx, h, x)
+        else:
+            ctx.rt.unfolded(self.ffn.forward, ctx, h, x)
 
 
 @BLOCKS.register("sandwich")

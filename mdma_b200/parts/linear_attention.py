@@ -235,7 +235,7 @@ class SideBySide(Part):
         stores = folded and hasattr(first, "produce")
         if not stores:
             out[:ctx.n_tokens].zero_()
-        self.forward(ctx, h, out, view, owns_cache, stores)
+        ctx.rt.unfolded(self.forward, ctx, h, out, view, owns_cache, stores)
         if ctx.rt.gemm == "tensor":
             from .. import ops_tensor
             ops_tensor.flush_pending(out.device, ctx.rt.tc)
@@ -247,11 +247,15 @@ class SideBySide(Part):
             own = dataclasses.replace(view, state=view.state[:, at:at + floats] if floats else None)
             at += floats
             if folded:
-                (m.produce if first_stores and i == 0 else m.forward)(ctx, h, x, own, owns_cache)
+                run = m.produce if first_stores and i == 0 else m.forward
+                if i + 1 == len(self.members):
+                    run(ctx, h, x, own, owns_cache)
+                else:                                          # the next child's first product comes before any norm
+                    ctx.rt.unfolded(run, ctx, h, x, own, owns_cache)
                 continue
             tmp = ctx.buf("side_scratch", self.hidden, torch.float32)
             tmp[:ctx.n_tokens].zero_()
-            m.forward(ctx, h, tmp, own, owns_cache)
+            ctx.rt.unfolded(m.forward, ctx, h, tmp, own, owns_cache)
             if ctx.rt.gemm == "tensor":
                 from .. import ops_tensor
                 ops_tensor.flush_pending(tmp.device, ctx.rt.tc)

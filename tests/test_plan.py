@@ -43,6 +43,40 @@ def test_choices_that_the_measurements_rest_on():
     assert plan(STORE, 8, 128256, 4096) == (16, 1)           # the head: more tiles than SMs, no split
 
 
+def test_block_pairs_divide_k_only_where_a_norm_adds_the_parts_up():
+    plan = lambda m, n, k, folded: ops_tensor.gemm_plan(ACCUMULATE, m, n, k, 148, folded)  # noqa: E731
+    for m, n, k, splits in ((513, 2048, 2048, 3), (768, 2048, 8192, 3), (1024, 2048, 8192, 2), (768, 1024, 4096, 6), (2048, 1024, 4096, 2), (600, 1000, 1024, 4),
+                            (512, 4096, 4096, 2), (385, 4096, 4096, 2), (384, 4096, 14336, 2), (257, 4096, 14336, 2)):
+        assert plan(m, n, k, True) == (512, splits), (m, n, k)
+        bn, alone = plan(m, n, k, False)
+        assert (bn, alone) == (512, 1) if m > 512 else bn != 512, (m, n, k)
+    # ... nor of 257-512 tokens where the one-block kernel is faster, up to 256 tokens, or without idle pairs; never a stored product
+    for m, n, k in ((512, 2048, 2048), (384, 4096, 4096), (384, 2048, 2048), (256, 4096, 14336), (1500, 2048, 2048)):
+        assert plan(m, n, k, True) == plan(m, n, k, False) and (plan(m, n, k, True)[0] != 512 or plan(m, n, k, True)[1] == 1)
+    assert ops_tensor.gemm_plan(STORE, 768, 3072, 2048, 148) == (512, 1)
+    for m in range(257, 2049, 13):
+        for mode, n, k in SHAPES["1b"] + SHAPES["odd"]:
+            if mode == ACCUMULATE:
+                bn, splits = plan(m, n, k, True)
+                assert ops_tensor.gemm_scratch_floats(bn, splits, m, n, 148) <= ops_tensor.scratch_floats_bound(148, m, 1, ())
+
+
+def test_a_sublayer_says_whether_its_sums_are_added_up():
+    """Nested arrangements: one that does not add up holds for all that it contains, and the state is as before after an error."""
+    from types import SimpleNamespace
+    import torch
+    from mdma_b200.parts.base import Runtime
+    tc = SimpleNamespace(folds=True)
+    rt = Runtime(torch.bfloat16, torch.device("cpu"), "tensor", tc=tc)
+    seen = lambda: tc.folds  # noqa: E731
+    assert rt.unfolded(rt.unfolded, seen) is False and tc.folds is True
+    assert rt.unfolded(lambda: (rt.unfolded(seen), seen())) == (False, False) and tc.folds is True
+    with pytest.raises(KeyError):
+        rt.unfolded({}.__getitem__, 0)
+    assert tc.folds is True
+    assert Runtime(torch.float32, torch.device("cpu")).unfolded(lambda: 5) == 5
+
+
 def test_clusters_that_start_early_have_two_blocks():
     """A cluster is placed as ordinary blocks are up to two blocks; wider ones are launched in stream order and never planned."""
     from mdma_b200.csrc import build
