@@ -915,21 +915,23 @@ int mdma_gemm_tc_plan(int mode, int folded, int n_tokens, int n_features, int K,
         }
         if (mode != kTcSwiGLU && n_tokens <= 512 && pair_tiles * 10 < (long)(sm_count / 2) * 6) {
             // Token tiles of 128, or of 256 where that puts more blocks on the SMs at once (O and down of 384
-            // tokens: 64 tiles of 256 x 2 splits against 96 tiles of 128).  Not for a product that is stored
-            // (QKV): alone it gains (256 tokens: 20.7 against 24.7 us with 3 splits), but the kernel that
-            // rotates and stores then reads three float partial sums per value and the step loses more.
+            // tokens: 64 tiles of 256 x 2 splits against 96 tiles of 128).  A stored product only where a norm or a gate adds
+            // its parts up (product and norm in groups, us, 128 / 256: 4,096 x 16,384 160 tokens 48.1 / 40.6, 256 49.5 / 43.9;
+            // 2,048 x 8,192 130 tokens 18.8 / 17.0, 400 30.6 / 24.7; 4,096 x 4,096 300 tokens 28.7 / 24.7), not QKV: alone it gains
+            // (256 tokens: 20.7 against 24.7 us with 3 splits), but the kernel that rotates and stores then reads three float
+            // partial sums per value and the step loses more.
             const int k_blocks = (K + kBK - 1) / kBK;
             int best_bn = 128, best_splits = 1;
             long best_blocks = 0;
-            for (int bn = 128; bn <= (mode == kTcAccumulate ? 256 : 128); bn *= 2) {
+            for (int bn = 128; bn <= (mode == kTcAccumulate || folded ? 256 : 128); bn *= 2) {
                 const long tiles = (long)((n_features + kBM - 1) / kBM) * ((n_tokens + bn - 1) / bn);
                 int splits = (int)(sm_count / tiles);
                 if (splits > k_blocks / 4) splits = k_blocks / 4;
                 if (splits < 1) splits = 1;
                 // (as many blocks either way: one token tile of 256 with more splits for up to 192 tokens or a long K.
                 // 160 tokens: down 32.4 against 38.4 us, O 14.7 against 15.8 us; 256 tokens: down 37.1 against 38.8 us,
-                // but O 17.7 against 16.2 us)
-                const bool tie_for_wide = bn == 256 && tiles * splits == best_blocks && (n_tokens <= 192 || K >= 8192);
+                // but O 17.7 against 16.2 us; a stored one of up to 192 tokens 1,536 x 6,144 14.8 / 15.5 us)
+                const bool tie_for_wide = bn == 256 && tiles * splits == best_blocks && ((n_tokens <= 192 && mode == kTcAccumulate) || K >= 8192);
                 if ((tiles * splits > best_blocks || tie_for_wide) && tiles * splits <= sm_count) { best_blocks = tiles * splits; best_bn = bn; best_splits = splits; }
             }
             *bn_out = best_bn; *splits_out = best_splits; return 0;

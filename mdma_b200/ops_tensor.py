@@ -180,11 +180,12 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = ops.GE
          bn: Optional[int] = None, splits: Optional[int] = None, defer: bool = False,
          st: Optional[TensorState] = None, bias: Optional[torch.Tensor] = None,
          bias2: Optional[torch.Tensor] = None, act: int = ops.ACT_SILU, store_act: bool = False,
-         act_limit: float = 0.0, act_alpha: float = 1.0) -> None:
+         act_limit: float = 0.0, act_alpha: float = 1.0, rows: bool = False) -> None:
     """out[:m] (=, +=) a[:m] @ w.T (+ bias) on the tensor cores; the gated mode takes gate=w, up=w2 and
     gives act(gate) * up.
     `defer`: if the product is split over K, leave its partial sums for the next kernel
-    (a norm or the rotary write) to add up; see `take_pending`.  `st`: the engine's state.
+    (a norm or the rotary write) to add up; see `take_pending`.  `rows`: that kernel reads a stored product's rows
+    anyway, as the norm behind an added one does (the rotary write does not).  `st`: the engine's state.
     `store_act` (stored products only): out = act(a @ w.T + bias), applied where the sums are complete."""
     if store_act:
         assert mode == ops.GEMM_STORE and not defer
@@ -201,7 +202,7 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int = ops.GE
     st = st or _device_state(a.device)
     flush_pending(a.device, st)
     if bn is None or splits is None:
-        pbn, psplits = gemm_plan(mode, M, N, K, st.sms, defer and mode == ops.GEMM_ACCUMULATE and st.folds)
+        pbn, psplits = gemm_plan(mode, M, N, K, st.sms, defer and st.folds and (rows or mode == ops.GEMM_ACCUMULATE))
         bn = bn or pbn
         splits = splits or psplits
     st.need(gemm_scratch_floats(bn, splits, M, N, st.sms), "a K-split product")

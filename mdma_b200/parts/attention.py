@@ -212,7 +212,7 @@ class Attention(Part):
             ops.attention_distance(row, view.k, view.v, ctx, view.page_table, view.max_pages, view.page_size, None, gate,
                                    out, self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim, self.window, self.scale,
                                    tiled, sinks=self.sink_f32, gate_heads=True, out_scale=self.out_scale)
-        (self.o_proj.store if stores else self.o_proj.accumulate)(out, x, n, defer=defer)
+        (self.o_proj.produce if stores else self.o_proj.accumulate)(out, x, n, defer=defer)
 
     def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
         """The result as float rows; `defer`: the last product may leave K-split partial sums of `out` for the caller's next
@@ -220,7 +220,7 @@ class Attention(Part):
         if self.extended:
             self._forward_extended(ctx, h, out, view, owns_cache, True, defer)
         else:
-            self.o_proj.store(self._attend(ctx, h, view, owns_cache), out, ctx.n_tokens, defer=defer)
+            self.o_proj.produce(self._attend(ctx, h, view, owns_cache), out, ctx.n_tokens, defer)
 
     def forward(self, ctx, h, x, view, owns_cache=True):
         if self.extended:

@@ -183,7 +183,7 @@ class ChannelDelta(Part):
         self.o.accumulate(self._run(ctx, h, view), x, ctx.n_tokens, defer=False)
 
     def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
-        self.o.store(self._run(ctx, h, view), out, ctx.n_tokens, defer=defer)
+        self.o.produce(self._run(ctx, h, view), out, ctx.n_tokens, defer)
 
     def resident_tensors(self):
         return [self.proj.w, self.conv, self.a2.w, self.g2.w, self.o.w, self.a_log, self.dt_bias, self.norm]

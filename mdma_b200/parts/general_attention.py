@@ -226,7 +226,7 @@ class GeneralAttention(Part):
 
     def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
         """The result as float rows; `defer`: the last product may leave K-split partial sums of `out`."""
-        self.o.store(self._run(ctx, h, view, owns_cache), out, ctx.n_tokens, defer=defer)
+        self.o.produce(self._run(ctx, h, view, owns_cache), out, ctx.n_tokens, defer)
 
     def resident_tensors(self):
         return [t for t in (self.proj.w, self.o.w, self.q_weight, self.k_weight, self.sink_values, *self.l_vectors) if t is not None]

@@ -172,7 +172,7 @@ class LatentAttention(Part):
         if accumulate:
             self.o.accumulate(v, target, n, defer=False)
         else:
-            self.o.store(v, target, n, defer=defer)
+            self.o.produce(v, target, n, defer)
 
     def resident_tensors(self):
         return [self.q_dkv.w, self.o.w, self.latent_norm, self.sink, self.uk, self.expand.w]

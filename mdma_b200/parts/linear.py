@@ -30,12 +30,12 @@ class Linear:
             self._tensor_ok = ops_tensor.gemm_supported(self.out_features, self.in_features)
 
     def _run(self, mode: int, a: torch.Tensor, out: torch.Tensor, m: int, defer: bool = False,
-             store_act: bool = False) -> None:
+             store_act: bool = False, rows: bool = False) -> None:
         if self._tensor_ok:
             from .. import ops_tensor
             ops_tensor.gemm(a, self.w, out, mode, self.w2, m, defer=defer, st=self.rt.tc,
                             bias=self.bias, bias2=self.bias2, act=self.act, store_act=store_act,
-                            act_limit=self.act_limit, act_alpha=self.act_alpha)
+                            act_limit=self.act_limit, act_alpha=self.act_alpha, rows=rows)
         else:
             if self.rt.gemm == "tensor":
                 from .. import ops_tensor
@@ -47,6 +47,10 @@ class Linear:
         """out = a W^T.  `defer`: a K-split product may leave its partial sums for the
         next kernel to add up (the caller promises that kernel asks for them)."""
         self._run(ops.GEMM_STORE, a, out, m, defer)
+
+    def produce(self, a, out, m, defer: bool = False):
+        """out = a W^T, a sublayer's result.  `defer`: as in `store`, for a kernel that reads the rows anyway (a norm, a gate)."""
+        self._run(ops.GEMM_STORE, a, out, m, defer, rows=True)
 
     def accumulate(self, a, x, m, defer: bool = True):
         """x += a W^T.  Deferred by default: the norm that reads x next adds the partial sums."""

@@ -159,7 +159,7 @@ class LinearAttention(Part):
 
     def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
         """`defer`: the last product may leave K-split partial sums of `out` for the caller's next kernel."""
-        self.o.store(self._run(ctx, h, view), out, ctx.n_tokens, defer=defer)
+        self.o.produce(self._run(ctx, h, view), out, ctx.n_tokens, defer)
 
     def resident_tensors(self):
         return [t for t in (self.proj.w, self.norm, self.o.w) if t is not None]

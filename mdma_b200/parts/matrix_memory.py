@@ -135,7 +135,7 @@ class MatrixMemory(Part):
 
     def produce(self, ctx, h, out, view, owns_cache=True, defer=False):
         """The result as float rows; `defer`: the last product may leave K-split partial sums of `out`."""
-        self.o.store(self._run(ctx, h, view), out, ctx.n_tokens, defer=defer)
+        self.o.produce(self._run(ctx, h, view), out, ctx.n_tokens, defer)
 
     def resident_tensors(self):
         return [self.proj.w, self.o.w, self.norm, self.i_bias, self.f_bias]

@@ -59,7 +59,7 @@ class GatedMLP(Part):
         next kernel."""
         act = ctx.buf("act", self.inner)
         self.gate_up.gated(h, act, ctx.n_tokens)
-        self.down.store(act, out, ctx.n_tokens, defer=defer)
+        self.down.produce(act, out, ctx.n_tokens, defer)
 
     def resident_tensors(self):
         return [t for t in (self.gate_up.w, self.gate_up.w2, self.down.w, self.gate_up.bias, self.gate_up.bias2,
@@ -101,7 +101,7 @@ class DenseMLP(Part):
         """`defer`: the second product may leave K-split partial sums of `out` for the caller's next kernel."""
         act = ctx.buf(f"dense_act_{self.inner}", self.inner)
         self.up.store_act(h, act, ctx.n_tokens)
-        self.down.store(act, out, ctx.n_tokens, defer=defer)
+        self.down.produce(act, out, ctx.n_tokens, defer)
 
     def forward(self, ctx, h, x):
         act = ctx.buf(f"dense_act_{self.inner}", self.inner)

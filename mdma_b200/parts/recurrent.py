@@ -52,7 +52,7 @@ class _StatefulMixer(Part):
         if accumulate:
             proj.accumulate(a, target, n, defer=False)
         else:
-            proj.store(a, target, n, defer=defer)
+            proj.produce(a, target, n, defer)
 
 
 @MIXERS.register("mingru")

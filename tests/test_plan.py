@@ -61,6 +61,16 @@ def test_block_pairs_divide_k_only_where_a_norm_adds_the_parts_up():
                 assert ops_tensor.gemm_scratch_floats(bn, splits, m, n, 148) <= ops_tensor.scratch_floats_bound(148, m, 1, ())
 
 
+def test_a_stored_product_in_front_of_a_norm_takes_wide_token_tiles():
+    """... as an added one does; the products that the rotary write reads stay as they were."""
+    plan = lambda m, n, k, folded: ops_tensor.gemm_plan(STORE, m, n, k, 148, folded)  # noqa: E731
+    for m, n, k, want in ((160, 4096, 16384, (256, 4)), (256, 4096, 16384, (256, 4)), (512, 4096, 16384, (256, 2)), (130, 2048, 8192, (256, 9)),
+                          (400, 2048, 8192, (256, 4)), (300, 4096, 4096, (256, 2)), (160, 1536, 6144, (128, 6)), (160, 2048, 2048, (128, 4))):
+        assert plan(m, n, k, True) == want and plan(m, n, k, False)[0] == 128, (m, n, k)
+        assert ops_tensor.gemm_scratch_floats(*want, m, n, 148) <= ops_tensor.scratch_floats_bound(148, m, 1, ())
+    assert plan(256, 6144, 4096, False) == (128, 1)
+
+
 def test_a_sublayer_says_whether_its_sums_are_added_up():
     """Nested arrangements: one that does not add up holds for all that it contains, and the state is as before after an error."""
     from types import SimpleNamespace
