@@ -82,9 +82,8 @@ static void launch_mode(const void* A, int lda, const void* W, const void* W2, v
     const int feats = few ? few_rows_features(K, kDual) : kDual ? kTileFeats / 2 : kTileFeats;
     const int groups = (N + feats - 1) / feats;
     if constexpr (std::is_same<TW, float>::value) {
-        // from two groups a block on
         const int most = few_rows_stream_blocks();
-        if (passes == 1 && batch == 1 && groups >= 2 * most && few_rows_streams(W, W2, K)) {
+        if (passes == 1 && batch == 1 && few_rows_streams(W, W2, N, K, kDual, most)) {
             const auto kernel = gemm_nt_kernel<TA, TW, TO, MODE, kStream>;
             launch(kernel, kFewRows, most, few_rows_stream_smem(kernel, M, K));
             return;
@@ -110,6 +109,10 @@ static int launch_gemm(int mode, const void* A, int lda, const void* W, const vo
 }  // namespace mdma
 
 using namespace mdma;
+// Returns 1 if a product of up to 8 rows with a 16-byte aligned float matrix (`gated`: two of them) [N, K] streams it through
+// shared memory on a device of so many SMs.
+extern "C" int mdma_gemm_simt_streams(int N, int K, int gated, int sm_count) { return few_rows_streams(nullptr, nullptr, N, K, gated != 0, 2 * sm_count) ? 1 : 0; }
+
 extern "C" int mdma_gemm_simt(int mode, const void* A, int a_dtype, int lda, const void* W, const void* W2,
                               int w_dtype, void* out, int out_dtype, int ldo, int M, int N, int K,
                               const void* bias, const void* bias2, int bias_dtype, int act, float act_limit, float act_alpha,

@@ -148,9 +148,17 @@ __host__ __device__ inline int few_rows_stream_floats(int rows, int K) {
     const int chunk = few_rows_chunk(K);
     return 2 * kStreamStage + rows * chunk * kRun + 2 * (kRowsThreads / chunk) * (rows * (chunk + 1) + kFewRows) + 64;
 }
-// whether a product of float matrices takes this form: their rows lie on 16 bytes
-__host__ __device__ inline bool few_rows_streams(const void* W, const void* W2, int K) {
-    return K <= kStreamMaxK && K % 4 == 0 && (((uintptr_t)W | (uintptr_t)W2) & 15) == 0;
+// Whether a product of float matrices takes this form on so many blocks: their rows lie on 16 bytes, there are two groups a block,
+// and a block's two stages carry enough of W.  A stage is as long as a chunk of runs, whatever K leaves empty of it, so one matrix
+// streams from 2.75 full stages a block on, or where K fills the chunk; two matrices always (they are half of the groups).
+// us, a block a group / streamed, 1 and 5 rows: 14,000 x 128 6.9 / 9.1, 9.9 / 11.0, x 384 8.4 / 9.7, 11.3 / 11.5, x 512 9.7 / 9.7,
+// 12.8 / 11.7; 20,000 x 256 11.0 / 12.3, 15.4 / 14.3, x 384 13.4 / 12.7, 17.9 / 15.2; 32,000 x 64 14.3 / 14.6, 20.4 / 21.4, x 256
+// 17.3 / 14.7, 23.4 / 21.9; 4,736 x 768 5.6 / 6.1, 8.7 / 8.5, 4,800 x 1,024 7.3 / 7.2, 11.0 / 9.4; gated 9,472 x 64 9.2 / 8.2, 13.0 / 12.3.
+static inline bool few_rows_streams(const void* W, const void* W2, int N, int K, bool dual, int blocks) {
+    if (K > kStreamMaxK || K % 4 != 0 || (((uintptr_t)W | (uintptr_t)W2) & 15) != 0) return false;
+    const int feats = few_rows_features(K, dual);
+    if ((N + feats - 1) / feats < 2 * blocks) return false;
+    return dual || 32 * ((K + kRun - 1) / kRun) >= 31 * few_rows_chunk(K) || 4l * N * K >= 11l * blocks * kStreamStage;
 }
 
 // As few_rows_product for the groups of features `group`, `group` + `groups`, ..; the same sums in the same order.

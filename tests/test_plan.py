@@ -129,3 +129,14 @@ def test_contexts_of_one_tile_a_warp_are_not_divided():
     assert splits(384, 128) == {1} and splits(768, 64) == {1} and splits(100, 64) == {1}
     assert splits(385, 128) == {4} and splits(769, 64) == {4} and splits(1000, 128) == {4}
     assert ops_tensor.attention_splits(1, 1, 100, 32, 8, 148, 2) == 4
+
+def test_short_rows_of_one_matrix_are_not_streamed():
+    """A block's stages are as long as a chunk of runs: one matrix streams where K fills it, or where there is enough of W."""
+    from mdma_b200.csrc import build
+    streams = lambda n, k, gated=0: build.load("core").mdma_gemm_simt_streams(n, k, gated, 148)  # noqa: E731
+    for n, k in ((9472, 64), (9472, 128), (9472, 384), (14000, 384), (20000, 256), (32000, 64), (32000, 128), (4736, 520), (4736, 768), (7000, 640)):
+        assert streams(n, k) == 0, (n, k)
+    for n, k in ((32000, 1024), (32000, 512), (32000, 256), (20000, 384), (128256, 64), (4736, 1024), (4739, 1000), (9472, 512), (128256, 768)):
+        assert streams(n, k) == 1, (n, k)
+    assert streams(9472, 64, 1) == streams(4736, 520, 1) == streams(2368, 1024, 1) == 1
+    assert [streams(*c) for c in ((4728, 1024), (9456, 512), (2364, 1024, 1), (200000, 1028), (200000, 1022))] == [0] * 5

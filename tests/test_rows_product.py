@@ -101,7 +101,7 @@ def test_a_matrix_that_the_kernel_before_writes(batch):
 
 
 @pytest.mark.parametrize("M", [1, 3, 4, 5, 8])
-@pytest.mark.parametrize("N,K", [(4736, 1024), (4739, 1000), (9472, 512), (9473, 20), (11000, 516)])
+@pytest.mark.parametrize("N,K", [(4736, 1024), (4739, 1000), (9472, 512), (9473, 20), (11000, 516), (13500, 516), (333700, 20)])
 def test_matrices_larger_than_the_blocks_hold(M, N, K):
     """Blocks that walk over groups of features: the bits of a row among 40 others, which takes the tiles."""
     from mdma_b200 import ops
@@ -122,3 +122,46 @@ def test_matrices_larger_than_the_blocks_hold(M, N, K):
     ops.gemm_simt(a, w, gated, ops.GEMM_SWIGLU, w2)
     ops.gemm_simt(rows, w, many, ops.GEMM_SWIGLU, w2)
     assert torch.equal(many[:M], gated)
+
+
+@pytest.mark.parametrize("M", [1, 4, 5, 8])
+@pytest.mark.parametrize("gated", [False, True])
+def test_streamed_products_in_a_replayed_chain(M, gated):
+    """Kernels of this library write the rows that a streamed product reads, and read what it writes, several times over in one
+    graph: each replay gives the bits of the tiles on its own inputs."""
+    from mdma_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(M)
+    N, K, rounds = 9473, 1024, 3
+    draw = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    first, back = draw(K, K) * K ** -0.5, draw(K, N) * N ** -0.5
+    ws = [(draw(N, K) * K ** -0.5, draw(N, K)) for _ in range(rounds)]
+    rows, a, b = draw(M, K), torch.zeros(M, K, device=DEV), torch.zeros(M, K, device=DEV)
+    outs = [torch.zeros(M, N, device=DEV) for _ in range(rounds)]
+
+    def product(x, w, out):
+        ops.gemm_simt(x, w[0], out, ops.GEMM_SWIGLU if gated else ops.GEMM_STORE, w[1] if gated else None, w_fixed=True)
+
+    def chain():
+        ops.gemm_simt(rows, first, a, w_fixed=True)
+        for i in range(rounds):
+            product(a, ws[i], outs[i])
+            ops.gemm_simt(outs[i], back, b, w_fixed=True)
+            ops.gemm_simt(b, first, a, w_fixed=True)
+    chain()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain()
+    many = torch.empty(M + 40, N, device=DEV)
+    for _ in range(4):
+        rows.copy_(draw(M, K))
+        for _ in range(3):
+            graph.replay()
+        x = torch.zeros(M + 40, K, device=DEV)
+        ops.gemm_simt(torch.cat([rows, draw(40, K)]), first, x)
+        for i in range(rounds):
+            product(x, ws[i], many)
+            assert torch.equal(many[:M], outs[i])
+            y = torch.empty(M + 40, K, device=DEV)
+            ops.gemm_simt(many, back, y)
+            ops.gemm_simt(y, first, x)
