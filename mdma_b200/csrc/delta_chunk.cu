@@ -246,9 +246,8 @@ __device__ __forceinline__ void dw_copy16(void* dst_shared, const void* src) {
 static __host__ __device__ constexpr int dw_stage_floats(int dimP) { return kDc * (3 * dimP + 20 + 24) + dimP + kDc * 20; }
 static size_t dw_smem(int dimP) { return sizeof(float) * ((size_t)kDwStages * dw_stage_floats(dimP) + kDwWarps * 16 * 32); }
 
-// The sequence with the rank-th most rows (a whole warp asks); beyond 32 sequences, the rank-th as they stand.
+// The sequence with the rank-th most rows (a whole warp asks).
 __device__ __forceinline__ int dw_sequence(const int* seq_start, int n_seqs, int rank) {
-    if (n_seqs > 32) return rank;
     const int lane = threadIdx.x & 31, mine = lane < n_seqs ? seq_start[lane + 1] - seq_start[lane] : -1;
     int before = 0;
     for (int j = 0; j < n_seqs; ++j) {
@@ -258,20 +257,27 @@ __device__ __forceinline__ int dw_sequence(const int* seq_start, int n_seqs, int
     return __ffs(__ballot_sync(0xffffffffu, lane < n_seqs && before == rank)) - 1;
 }
 
-// Blocks by sequence, the longest first, then by head and columns: a block's time is its sequence's length, and as the prompts
-// stand long ones start late (four prompts of 100 to 801 rows, 16 heads of 128 x 128: 82 us, 119 as they stand).
+// Whether the sequences are walked longest first: a block's time is its sequence's length, and as the prompts stand long ones may
+// start late.  Finding the place costs a block up to a microsecond, so only where a walk is long and the lengths differ.  Both
+// kernels, 16 heads of 128 x 128, us, as they stand / longest first: four of 100 to 801 rows 213 / 196, 400 to 700 240 / 233, 15
+// of 40 and one of 400 145 / 129, 32 of 10 to 400 661 / 658; 32 of 30 127 / 134, 32 of 5 to 60 149 / 156, 8 of 17 to 38 35.1 / 36.1.
+static bool dw_longest_first(int n_rows, int n_seqs, int max_new) {
+    return n_seqs > 1 && n_seqs <= 32 && max_new >= 128 && 10l * n_rows <= 9l * n_seqs * max_new;
+}
+
+// Blocks by sequence (`longest_first`, or as they stand), then by head and columns.
 // NTD: tiles of eight key channels a warp has (dim up to 32 * NTD)
 template <int NTD>
 __global__ void __launch_bounds__(kDwWarps * 32)
 delta_chunk_walk_kernel(const float* __restrict__ scratch, const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
-                        float* __restrict__ state, size_t state_stride, float* __restrict__ out, int n_seqs, int heads, int dim, int vdim) {
+                        float* __restrict__ state, size_t state_stride, float* __restrict__ out, int n_seqs, int longest_first, int heads, int dim, int vdim) {
     chain_release();
     chain_wait();
     extern __shared__ __align__(16) float dw_sm[];
     constexpr int dimP = 32 * NTD, wp = dimP + 8, kp = dimP + 4, zp = 20, bp = 24, stage_floats = dw_stage_floats(dimP);
     constexpr int common = stage_floats - kDc * zp;
     const int slices = (vdim + kDcCols - 1) / kDcCols, slice = blockIdx.x % slices, h = blockIdx.x / slices % heads;
-    const int s = dw_sequence(seq_start, n_seqs, blockIdx.x / slices / heads), c0 = slice * kDcCols, cw = min(kDcCols, vdim - c0);
+    const int place = blockIdx.x / slices / heads, s = longest_first ? dw_sequence(seq_start, n_seqs, place) : place, c0 = slice * kDcCols, cw = min(kDcCols, vdim - c0);
     const int t0 = seq_start[s], t1 = seq_start[s + 1];
     if (t1 <= t0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
@@ -437,6 +443,9 @@ long mdma_delta_chunks_scratch(int n_rows, int n_seqs, int heads, int dim, int v
     return ((long)n_rows / kDc + n_seqs + 1) * heads * (long)DcLayout(dim, vdim).floats;
 }
 
+// Returns 1 if mdma_delta_chunks walks sequences of these sizes longest first.
+int mdma_delta_chunks_longest_first(int n_rows, int n_seqs, int max_new) { return dw_longest_first(n_rows, n_seqs, max_new) ? 1 : 0; }
+
 // proj rows [q | k | v | b | ..], raw [rows][heads * dim] the decays' inputs, out [rows][heads * vdim], all floats; the
 // convolutions' kept inputs are read, not brought up to date
 int mdma_delta_chunks(const float* proj, int proj_stride, const float* raw, const void* conv_w, int conv_dtype, int taps,
@@ -468,12 +477,13 @@ int mdma_delta_chunks(const float* proj, int proj_stride, const float* raw, cons
     const DcLayout lay(dim, vdim);
     MDMA_REQUIRE((long)n_seqs * heads * lay.slices <= 2147483647l, "delta_chunks: too many rows");
     dim3 grid((unsigned)((long)n_seqs * heads * lay.slices));
+    const int longest_first = dw_longest_first(n_rows, n_seqs, max_new) ? 1 : 0;
 #define MDMA_DW(NTD)                                                                                                     \
     do {                                                                                                                 \
         static bool up = false;                                                                                          \
         if (!up) { cudaFuncSetAttribute(delta_chunk_walk_kernel<NTD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dw_smem(32 * NTD)); up = true; } \
         launch_chained(delta_chunk_walk_kernel<NTD>, grid, dim3(kDwWarps * 32), dw_smem(32 * NTD), stream, (const float*)scratch, \
-                       seq_start, seq_slot, state, (size_t)state_stride, out, n_seqs, heads, dim, vdim);                 \
+                       seq_start, seq_slot, state, (size_t)state_stride, out, n_seqs, longest_first, heads, dim, vdim);                 \
     } while (0)
     if (lay.dimP == 32) MDMA_DW(1);
     else if (lay.dimP == 64) MDMA_DW(2);

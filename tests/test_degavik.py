@@ -843,9 +843,9 @@ def test_random_configurations(seed):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("lengths", [[5, 40, 40, 1, 0, 17], [3 + i % 7 for i in range(33)]])
+@pytest.mark.parametrize("lengths", [[5, 40, 40, 1, 0, 17], [5, 140, 140, 1, 0, 17], [3 + i % 7 for i in range(31)] + [130], [3 + i % 7 for i in range(32)] + [130]])
 def test_delta_chunks_of_a_sequence_are_the_same_among_others(lengths):
-    """Sequences are walked longest first (beyond 32 as they stand): each gives the bits that it gives alone."""
+    """Sequences are walked longest first (short or like ones and beyond 32 as they stand): each gives the bits that it gives alone."""
     from mdma_b200 import ops
     H, D, V, taps = 2, 32, 48, 4
     ch = 2 * H * D + H * V
@@ -871,3 +871,11 @@ def test_delta_chunks_of_a_sequence_are_the_same_among_others(lengths):
             alone, one = run([s], [s])
             assert torch.equal(alone, together[at:at + lengths[s]]) and torch.equal(one[s], state[s])
         at += lengths[s]
+
+
+def test_short_and_like_sequences_are_walked_as_they_stand():
+    from mdma_b200.csrc import build
+    longest_first = build.load("core").mdma_delta_chunks_longest_first
+    first = lambda lengths: longest_first(sum(lengths), len(lengths), max(lengths))  # noqa: E731
+    assert [first(n) for n in ([30] * 32, [5, 20, 60] * 10, [17, 38] * 4, [2000], [120, 125, 130, 130], [10, 130] * 17, [10, 127])] == [0] * 7
+    assert [first(n) for n in ([100, 333, 566, 801], [400, 500, 600, 700], [40] * 15 + [400], [10, 130] * 16, [10, 128], [5, 140, 140, 1, 0, 17])] == [1] * 6
