@@ -391,8 +391,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     const int n_seg = work.count();
 
     // This kernel takes no part in programmatic dependent launch: launched early next to the tail of
-    // another kernel it stalled now and then; it is used for many tokens, where a launch gap is
-    // nothing against its run time.
+    // another kernel it stalled now and then; it is used for many tokens or for experts' runs side by
+    // side, where a launch gap is nothing against its run time.
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { ptx::mbar_init(full_bar(s), 1); ptx::mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { ptx::mbar_init(acc_full(b), 1); ptx::mbar_init(acc_empty(b), 2 * tc2_epi_warps<MODE>()); }   // epilogue warps x 2 blocks
@@ -941,7 +941,10 @@ int mdma_gemm_tc_plan(int mode, int folded, int n_tokens, int n_features, int K,
     if (mode == kTcSwiGLU && n_tokens > 96) {
         // the gated product of 97-128 tokens: block pairs with one token tile (50.4 against 54.3 us at 128 tokens, 48.2
         // against 50.6 us at 96; below that one block per tile is faster); a decode step of 128 sequences: 6.41
-        // against 6.51 ms
+        // against 6.51 ms.  Of 33-64 tokens pairs are faster alone where one block a tile leaves half of the device idle (norm and
+        // product of 64 tokens 8,192 x 2,048 29.3 / 27.3), but they do not start early, and no decode step gains what some lose:
+        // one block / pairs, Llama-3.2-1B 33 sequences 1,122 / 1,148, 48 1,179 / 1,163, 64 1,206 / 1,203, Salipel of width 2,048
+        // 48 sequences 469 / 497, Degavik of 3,072 855 / 868, of 2,048 636 / 624.
         *bn_out = 512; *splits_out = 1; return 0;
     }
     int bn = 16;
@@ -949,11 +952,6 @@ int mdma_gemm_tc_plan(int mode, int folded, int n_tokens, int n_features, int K,
     const int k_blocks = (K + kBK - 1) / kBK;
     const long tiles = (long)((n_features + kBM - 1) / kBM) * ((n_tokens + bn - 1) / bn);
     int splits = 1;
-    if (mode == kTcSwiGLU && bn == 64 && 2 * tiles <= sm_count) {
-        // ... and of 33-64 tokens where one block a tile leaves half of the device idle: norm and product of 64 tokens, us, one
-        // block / pairs: 8,192 x 2,048 26.9 / 24.8, 5,632 x 2,048 26.4 / 23.6, 2,752 x 1,024 17.4 / 15.2 (14,336 x 4,096 52.3 / 52.3)
-        *bn_out = 512; *splits_out = 1; return 0;
-    }
     if (mode == kTcSwiGLU && bn <= 32 && tiles < sm_count && k_blocks >= 8) {
         // The SwiGLU ending needs complete sums, so its K split stays inside a cluster of two blocks
         // (measured at batch 8: 37.4 us against 41.8 us unsplit; larger clusters and cluster splits
@@ -1168,6 +1166,11 @@ int mdma_gemm_tc_runs(int mode, const void* x, int ldx, const void* w, const voi
         int bn = 0, splits = 0;
         rc = mdma_gemm_tc_plan(mode, 0, m, n_features, K, sm_count, &bn, &splits);
         if (rc) break;
+        // Gated runs of 33-64 rows whose tiles would leave half of the device idle go to block pairs: there is no chain to start
+        // early in (eight runs, us, one block / pairs: 40 rows 5,632 x 2,048 98 / 87, 2,816 x 2,048 57 / 56, 1,024 x 2,048 52 / 50; 9
+        // to 100 rows 110 / 94, 72 / 59, 56 / 50; one of 35 and seven of 2 72.3 / 73.4, 49.7 / 50.3, 38.5 / 37.0).  Not with a longer K
+        // (2,048 x 4,096: 9 to 100 rows 94 / 84, but 3 to 70 rows 92 / 93, 35 and 2 65 / 68; 7,168 x 4,096: 188 / 175, 172 / 178, 151 / 154).
+        if (mode == kTcSwiGLU && bn == 64 && K <= 2048 && 2 * ((n_features + kBM - 1) / kBM) <= sm_count) bn = 512;
         if (splits > 1) splits = 1;          // no partial sums through the scratch: the runs side by side fill the device
         const char* xr = (const char*)x + (size_t)lo * ldx * 2;
         const char* wr = (const char*)w + (size_t)r * w_stride * 2;

@@ -99,16 +99,37 @@ def test_pairs_that_divide_k(M, N, K, splits, mode, bias, act):
     assert bool(((got - want).abs() <= tol).all())
 
 
-@pytest.mark.parametrize("M,N,K,plan", [(1, 8192, 2048, (16, -2)), (8, 2752, 1024, (16, -2)), (16, 330, 1032, (16, -2)), (40, 8192, 2048, (512, 1)), (33, 300, 1024, (512, 1)), (64, 2750, 1032, (512, 1))])
+@pytest.mark.parametrize("M,N,K,plan", [(1, 8192, 2048, (16, -2)), (8, 2752, 1024, (16, -2)), (16, 330, 1032, (16, -2)), (40, 8192, 2048, (64, 1)), (33, 300, 1024, (64, 1)), (64, 2750, 1032, (64, 1))])
 def test_gated_products_of_few_tiles(M, N, K, plan):
     from mdma_b200 import ops, ops_tensor
     assert ops_tensor.gemm_plan(2, M, N, K, 148) == plan
     torch.manual_seed(M + N)
     a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
     w, w2 = ((torch.randn(N, K, device=DEV) * K ** -0.5).bfloat16() for _ in range(2))
-    out = torch.full((M + 1, N), 9.0, device=DEV, dtype=torch.bfloat16)
-    ops_tensor.gemm(a, w, out, ops.GEMM_SWIGLU, w2, M)
-    ops_tensor.check_status(torch.device(DEV))
     ref = a.double() @ w.double().t()
     ref = ref / (1 + torch.exp(-ref)) * (a.double() @ w2.double().t())
-    assert bool((out[M:] == 9.0).all()) and bool(((out[:M].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all())
+    for forced in ({}, dict(bn=512, splits=1)):                  # as planned, and on block pairs (experts' runs of 33-64 rows)
+        out = torch.full((M + 1, N), 9.0, device=DEV, dtype=torch.bfloat16)
+        ops_tensor.gemm(a, w, out, ops.GEMM_SWIGLU, w2, M, **forced)
+        ops_tensor.check_status(torch.device(DEV))
+        assert bool((out[M:] == 9.0).all()) and bool(((out[:M].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all())
+
+
+@pytest.mark.parametrize("N,K", [(5632, 2048), (300, 1032)])
+def test_gated_runs_of_33_to_64_rows(N, K):
+    """Experts side by side, some on block pairs: each gives what it gives alone."""
+    from mdma_b200 import ops, ops_tensor
+    torch.manual_seed(N)
+    first = [0, 40, 43, 43, 107, 140, 152, 217]
+    runs = len(first) - 1
+    a = (torch.randn(first[-1], K, device=DEV) * 0.5).bfloat16()
+    w, w2 = ((torch.randn(runs * N, K, device=DEV) * K ** -0.5).bfloat16() for _ in range(2))
+    out = torch.full((first[-1] + 1, N), 9.0, device=DEV, dtype=torch.bfloat16)
+    ops_tensor.gemm_runs(a, w, out, first, N, ops.GEMM_SWIGLU, w2)
+    ops_tensor.check_status(torch.device(DEV))
+    assert bool((out[first[-1]:] == 9.0).all())
+    for r in range(runs):
+        x = a[first[r]:first[r + 1]].double()
+        ref = x @ w[r * N:(r + 1) * N].double().t()
+        ref = ref / (1 + torch.exp(-ref)) * (x @ w2[r * N:(r + 1) * N].double().t())
+        assert bool(((out[first[r]:first[r + 1]].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()), r

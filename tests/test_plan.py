@@ -36,6 +36,7 @@ def test_choices_that_the_measurements_rest_on():
     assert plan(ACCUMULATE, 8, 4096, 4096) == (16, 9)        # O: two blocks per SM
     assert plan(GATED, 8, 14336, 4096) == (16, -2)           # gate+up: K split inside a cluster of two
     assert plan(GATED, 64, 14336, 4096) == (64, 1)
+    assert [plan(GATED, m, 5632, 2048) for m in (33, 48, 64)] == [(64, 1)] * 3        # in a decode step pairs, which do not start early, lose
     assert plan(GATED, 128, 14336, 4096)[0] == 512           # block pairs from 97 tokens
     assert plan(ACCUMULATE, 256, 4096, 14336) == (256, 4)    # down of 256 tokens: one wide token tile, four splits
     assert plan(STORE, 256, 6144, 4096) == (128, 1)          # QKV stays unsplit there (its partial sums cost the rotary kernel more)
