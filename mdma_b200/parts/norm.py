@@ -30,9 +30,10 @@ class RMSNorm(Part):
             raise ValueError(f"a row of {self.width} numbers does not split into {self.groups} equal parts")
         if self.groups > 1:
             self.fuses_pending = False      # the grouped kernel reads complete rows of x
-        # `add_normed(.., stored=True)` completes a stored product's partial sums itself; of the two, only the plain norm
-        # leaves a copy of the stream
-        self.adds_stored, self.completes_stored = self.groups == 1, True
+        # `adds_stored`: `add_normed` takes a stored result, whole rows and a copy of the stream alike.  `completes_stored`: it takes
+        # one without leaving a copy; in groups that is this class's own, a derived norm's in its place may not know `stored`.
+        self.adds_stored = self.groups == 1
+        self.completes_stored = type(self).add_normed is RMSNorm.add_normed
 
     def tensor_specs(self):
         return {"weight": TensorSpec((self.width,), "vector")}
