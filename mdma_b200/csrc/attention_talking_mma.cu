@@ -120,8 +120,8 @@ talking_attention_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfl
     const int row_lo = lane >> 2, row_hi = row_lo + 8;
     const uint32_t sx_addr = (uint32_t)__cvta_generic_to_shared(sxw);
 
-    // a chunk's key rows and value rows, asked for 16 bytes at a time (a warp takes whole rows: one look at the page
-    // table per row); rows no key owns: zero.  Two blocks share an SM: while one waits for its copies the other multiplies.
+    // a chunk's key rows and value rows, asked for 16 bytes at a time, whole rows a warp; rows no key owns: zero.  Two blocks
+    // share an SM: while one waits for its copies the other multiplies.
     const int k_cols = kd / 8, v_cols = v_dim / 8;
     // with `splits` > 1 this block takes a run of the tile's chunks and leaves unnormalised sums for the merge kernel
     const int n_chunks = (last + 1 - first + kTmChunk - 1) / kTmChunk, per_split = (n_chunks + splits - 1) / splits;

@@ -49,7 +49,7 @@ __device__ __forceinline__ void add_splits(float4& v, const float* pp, int split
 
 // Blocks of groups * slices warps (or fewer warps that walk the groups when there are more than 16 groups).
 template <typename TW, typename TO, bool ADD>
-__global__ void __launch_bounds__(kGroupNormMaxWarps * 32, 2)       // 64 registers: the block starts beside those of the product in front
+__global__ void __launch_bounds__(kGroupNormMaxWarps * 32, 2)       // 64 registers (ADD spills 4 to 16 bytes): the block starts beside those of the product in front
 group_rmsnorm_kernel(const float* src, float* y_complete, const float* __restrict__ partial,
                      int splits, size_t split_stride, int only, const int* __restrict__ rows, const TW* __restrict__ w,
                      TO* __restrict__ out, float* __restrict__ x_add, int width, int groups, int slices, int fours, float eps) {

@@ -161,7 +161,9 @@ static inline bool few_rows_streams(const void* W, const void* W2, int N, int K,
     return dual || 32 * ((K + kRun - 1) / kRun) >= 31 * few_rows_chunk(K) || 4l * N * K >= 11l * blocks * kStreamStage;
 }
 
-// As few_rows_product for the groups of features `group`, `group` + `groups`, ..; the same sums in the same order.
+// As few_rows_product for the groups of features `group`, `group` + `groups`, ..; the same sums in the same order.  Where the rows of
+// A, the sums and the totals lie in `smem` depends on `rows`: a barrier belongs between two calls in one block, and W is asked
+// for before `arrived()`, so its address may not depend on anything that the kernel in front writes.
 template <typename TA, bool DUAL, class RowOf, class Arrived, class Store>
 __device__ __forceinline__ void few_rows_stream(int rows, RowOf row_of, const float* __restrict__ W, const float* __restrict__ W2,
                                                 int group, int groups, int N, int K, bool vec_a, float* smem, Arrived arrived, Store store) {
@@ -350,7 +352,7 @@ __device__ __forceinline__ void tile_product(int rows, RowOf row_of, const TW* _
     }
 }
 
-// Blocks of few_rows_stream that the device holds: two an SM (one with more than four rows of A).
+// Blocks of few_rows_stream that the device holds: two an SM (115,456 bytes each at most, with eight rows of A and 1,024 of K).
 static inline int few_rows_stream_blocks() {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

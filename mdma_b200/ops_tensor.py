@@ -18,7 +18,9 @@ EVEN_SPLIT = os.environ.get("MDMA_EVEN_SPLIT", "1") != "0"
 
 FORCED_ATTENTION = os.environ.get("MDMA_ATTN")        # "tc" or "mma": one attention kernel for every step (comparisons)
 
-PAIR_TOKENS = 96         # steps of more tokens than this may run a product on the block-pair kernel (the gated one from 97)
+# Steps of more tokens than this may run a product on the block-pair kernel with partial tiles (the gated one from 97; experts' runs
+# of 33-64 rows run there as whole tiles, which need no scratch).
+PAIR_TOKENS = 96
 
 
 def pair_scratch_floats(sms: int) -> int:
@@ -30,7 +32,8 @@ def scratch_floats_bound(sms: int, max_tokens: int, max_seqs: int, attention_sha
     """An upper bound of the scratch any step of up to `max_tokens` tokens in up to `max_seqs`
     sequences needs, from sizes alone (an engine reserves this much once and never grows it).
     K-split products keep splits x tokens x features floats with splits x tiles <= 2 x SMs, tiles of
-    128 features x up to 64 tokens (one per SM for 128 tokens); attention keeps tokens x heads x
+    128 features x up to 64 tokens (one per SM for 128 tokens); block pairs that divide K keep splits x
+    tiles <= SMs / 2 of 256 x 256, half of what their partial tiles reserve; attention keeps tokens x heads x
     splits x (head_dim + 2) floats.  `attention_shapes`: (heads, kv heads, head_dim) of each mixer."""
     del max_seqs          # the bounds below hold for any number of sequences
     need = 2 * sms * 128 * 64

@@ -72,7 +72,7 @@ def test_gates_far_from_zero(bn):
 
 
 def _product(M, N, K, mode, bias, act, **forced):
-    """(result, reference, bound) of a product through the planner or as `forced`; partial sums are added up at once."""
+    """(result, reference, bound) of a product as `forced`; partial sums are added up at once."""
     from mdma_b200 import ops, ops_tensor
     torch.manual_seed(M + N + K)
     a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
@@ -133,3 +133,36 @@ def test_gated_runs_of_33_to_64_rows(N, K):
         ref = x @ w[r * N:(r + 1) * N].double().t()
         ref = ref / (1 + torch.exp(-ref)) * (x @ w2[r * N:(r + 1) * N].double().t())
         assert bool(((out[first[r]:first[r + 1]].double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5).all()), r
+
+
+@pytest.mark.parametrize("M,N,K,plan", [(600, 1000, 1024, (512, 4)), (768, 2048, 8192, (512, 3)), (257, 4096, 14336, (512, 2)), (513, 1024, 520, (512, 2))])
+@pytest.mark.parametrize("groups", [1, 4])
+@pytest.mark.parametrize("bias", [False, True])
+def test_a_norm_adds_up_what_pairs_leave(M, N, K, plan, groups, bias):
+    """As planned: the pairs' parts go to the norm behind the product, added to the residual stream or onto a sublayer's result."""
+    from mdma_b200 import ops, ops_tensor
+    assert ops_tensor.gemm_plan(ops.GEMM_ACCUMULATE, M, N, K, 148, True) == plan
+    torch.manual_seed(M + N + groups)
+    a = (torch.randn(M, K, device=DEV) * 0.5).bfloat16()
+    w = (torch.randn(N, K, device=DEV) * K ** -0.5).bfloat16()
+    b = torch.randn(N, device=DEV).bfloat16() if bias else None
+    x, y, nw = torch.randn(M, N, device=DEV), torch.randn(M, N, device=DEV), 1 + 0.3 * torch.randn(N, device=DEV)
+    want_y = y.double() + a.double() @ w.double().t() + (b.double() if bias else 0.0)
+    part = want_y.view(M, groups, -1)
+    normed = (part / torch.sqrt((part * part).mean(-1, keepdim=True) + 1e-5)).reshape(M, N) * nw.double()
+    ops_tensor.gemm(a, w, y, ops.GEMM_ACCUMULATE, None, M, bias=b, defer=True)
+    pend = ops_tensor.take_pending(y, ops.GEMM_ACCUMULATE, M)
+    assert pend is not None and pend[1] == plan[1] and pend[2] == M * N
+    if groups == 1:
+        h = torch.empty(M, N, device=DEV)
+        ops.rmsnorm(y, nw, 1e-5, h, None, M, *pend)
+        got, want = h.double(), normed
+    else:
+        want = x.double() + normed
+        ops.group_rmsnorm_add(x, y, nw, 1e-5, groups, M, *pend)
+        got = x.double()
+    ops_tensor.check_status(torch.device(DEV))
+    # a part is K / splits products, 16 to an addition whose sum is cut to a float (2 ** -23 of sums below 2); then the parts and the rest
+    tol = 1e-5 + K / plan[1] / 16 * 2.0 ** -22
+    assert bool(((y.double() - want_y).abs() <= tol * (1 + want_y.abs())).all())
+    assert bool(((got - want).abs() <= 4 * tol * (1 + want.abs())).all())               # the same, over the row's deviation and times w
